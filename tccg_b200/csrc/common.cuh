@@ -254,6 +254,18 @@ __device__ __forceinline__ uint64_t umma_desc_k128(uint32_t smem_addr) {
   return d;
 }
 
+// The same for the 64-byte swizzle (rows of 64 B, 8-row atoms of 512 B):
+// SBO = 512 B, layout type 4 (SWIZZLE_64B).
+__device__ __forceinline__ uint64_t umma_desc_k64(uint32_t smem_addr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((smem_addr & 0x3FFFFu) >> 4);
+  d |= (uint64_t)1 << 16;
+  d |= (uint64_t)(512 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)4 << 61;
+  return d;
+}
+
 // Instruction descriptor of kind::f16 with BF16 A/B, FP32 D, both K-major.
 __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
   return (1u << 4)                          // D format: F32
@@ -274,6 +286,61 @@ __device__ __forceinline__ void split_bf16x2(float x0, float x1, uint32_t& hi, u
   const __nv_bfloat162 l = __floats2bfloat162_rn(x0 - __low2float(h), x1 - __high2float(h));
   hi = *reinterpret_cast<const uint32_t*>(&h);
   lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
+// ---- three-way split of FP32 ---------------------------------------------------
+// x = hi + mid + lo exactly: hi = bf16_rn(x), mid = bf16_rn(x - hi), lo =
+// x - hi - mid (|x - hi| <= 2^-8 |x| and |x - hi - mid| <= 2^-17 |x|, so at
+// most 7 of x's 24 significant bits are left for lo). Exact for every x that
+// f32_split_exact() accepts.
+__device__ __forceinline__ void split3_bf16x2(float x0, float x1, uint32_t& hi, uint32_t& mid,
+                                              uint32_t& lo) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(x0, x1);
+  const float r0 = x0 - __low2float(h), r1 = x1 - __high2float(h);
+  const __nv_bfloat162 m = __floats2bfloat162_rn(r0, r1);
+  const __nv_bfloat162 l = __floats2bfloat162_rn(r0 - __low2float(m), r1 - __high2float(m));
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  mid = *reinterpret_cast<const uint32_t*>(&m);
+  lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
+// Magnitude range of one operand, kept by the packing pass as two words that
+// shrink by atomicMin from 0xffffffff: w[0] = ~(largest |x|'s bits), w[1] =
+// (smallest nonzero |x|'s bits) - 1. NaN and infinity count as the largest.
+struct AbsRange {
+  uint32_t not_max = 0xffffffffu, min_less1 = 0xffffffffu;
+  __device__ __forceinline__ void add(float x) {
+    const uint32_t b = __float_as_uint(x) & 0x7fffffffu;
+    not_max = min(not_max, ~b);
+    min_less1 = min(min_less1, b - 1u);  // zero wraps to 0xffffffff
+  }
+  // one warp's values into w (all lanes take part); the words are read first,
+  // so that few warps need an atomic
+  __device__ __forceinline__ void flush(uint32_t* w) {
+    const uint32_t a = __reduce_min_sync(0xffffffffu, not_max);
+    const uint32_t b = __reduce_min_sync(0xffffffffu, min_less1);
+    if ((threadIdx.x & 31) == 0) {
+      if (a < *reinterpret_cast<volatile uint32_t*>(w)) atomicMin(w, a);
+      if (b < *reinterpret_cast<volatile uint32_t*>(w + 1)) atomicMin(w + 1, b);
+    }
+  }
+};
+
+// Whether FP32 products of two operands with ranges w[0..1] and w[2..3] over
+// K terms may run as products of their three-way splits: every value finite
+// and below 2^127 (the split's rounding cannot overflow), no sum of products
+// near overflow, nonzero values at least 2^-100 (every part of the split is a
+// normal bf16 or exact) and nonzero products at least 2^-100 (the dropped and
+// the smallest kept terms stay clear of FP32's subnormals).
+__device__ __forceinline__ bool f32_split_exact(const uint32_t* w, int K) {
+  const uint4 r = *reinterpret_cast<const uint4*>(w);
+  const int ea = (int)(~r.x >> 23), eb = (int)(~r.z >> 23);  // biased exponents
+  if (ea >= 254 || eb >= 254) return false;
+  if (r.y == 0xffffffffu || r.w == 0xffffffffu) return true;  // an operand of zeros
+  const int logk = 32 - __clz(K);
+  if (ea - 127 + eb - 127 + 2 + logk >= 126) return false;
+  const int ma = (int)((r.y + 1u) >> 23) - 127, mb = (int)((r.w + 1u) >> 23) - 127;
+  return ma >= -100 && mb >= -100 && ma + mb >= -100;
 }
 
 // ---- cp.async (SIMT kernels) ------------------------------------------------

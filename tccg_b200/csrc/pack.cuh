@@ -19,7 +19,12 @@ enum PackLayout : int {
   PACK_K_BF16 = 1,    // dst[r * ld + k], bf16, k < Kcover (zeros beyond K)
   PACK_K_BF16X3 = 2,  // dst[r * ld + (k/32)*64 + k%32] = hi, +32 = lo (bf16)
   PACK_MN_BF16 = 3,   // as PACK_MN, each value rounded to bf16 (BF16 semantics on CUDA cores)
+  PACK_K_F32X6 = 4,   // dst[r * ld + (k/32)*96 + k%32] = hi, +32 = mid, +64 = lo (bf16): the
+                      // exact three-way split of FP32, with the operand's magnitude range
 };
+__host__ __device__ constexpr bool pack_k_major(int layout) {
+  return layout == PACK_K_BF16 || layout == PACK_K_BF16X3 || layout == PACK_K_F32X6;
+}
 
 struct PackOperand {
   const void* src;
@@ -52,6 +57,25 @@ struct PackOperand {
   int32_t kstream;
   // tile grid of this operand: tiles along k and in total (set by the host)
   int64_t ktiles, tiles;
+  // PACK_K_F32X6: the operand's two range words (AbsRange), 0xffffffff before
+  // the pass
+  uint32_t* range;
+};
+
+// The values a thread packs, for PACK_K_F32X6's range words (else nothing).
+template <int LAYOUT>
+struct PackRange {
+  __device__ __forceinline__ void add(const float (&)[4]) {}
+  __device__ __forceinline__ void flush(uint32_t*) {}
+};
+template <>
+struct PackRange<PACK_K_F32X6> {
+  AbsRange r;
+  __device__ __forceinline__ void add(const float (&x)[4]) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) r.add(x[j]);
+  }
+  __device__ __forceinline__ void flush(uint32_t* w) { r.flush(w); }
 };
 
 struct PackArgs {
@@ -77,11 +101,21 @@ __device__ __forceinline__ float load_as_acc<__nv_bfloat16>(const __nv_bfloat16*
 }
 
 // Writes 4 consecutive k (k .. k+3, k % 4 == 0) of destination row `base`
-// in a K-major layout: bf16, or [hi x32 | lo x32] per 32-wide k block.
+// in a K-major layout: bf16, or [hi x32 | lo x32] per 32-wide k block, or
+// [hi x32 | mid x32 | lo x32].
 template <int LAYOUT>
 __device__ __forceinline__ void store_k4(__nv_bfloat16* base, int64_t k, int64_t kcover,
-                                         int64_t ld, const float (&x)[4]) {
-  if constexpr (LAYOUT == PACK_K_BF16) {
+                                         int64_t ld, const float (&x)[4], PackRange<LAYOUT>& rng) {
+  rng.add(x);
+  if constexpr (LAYOUT == PACK_K_F32X6) {  // kcover is a multiple of 32
+    __nv_bfloat16* row = base + (k / 32) * 96;  // 64-byte aligned: ld % 96 == 0
+    uint2 uh, um, ul;
+    split3_bf16x2(x[0], x[1], uh.x, um.x, ul.x);
+    split3_bf16x2(x[2], x[3], uh.y, um.y, ul.y);
+    *reinterpret_cast<uint2*>(row + k % 32) = uh;
+    *reinterpret_cast<uint2*>(row + 32 + k % 32) = um;
+    *reinterpret_cast<uint2*>(row + 64 + k % 32) = ul;
+  } else if constexpr (LAYOUT == PACK_K_BF16) {
     if (k + 3 < kcover && (ld & 3) == 0) {
       __nv_bfloat162 p0 = __floats2bfloat162_rn(x[0], x[1]);
       __nv_bfloat162 p1 = __floats2bfloat162_rn(x[2], x[3]);
@@ -119,7 +153,8 @@ __host__ __device__ constexpr int pack_k_tile() {
 
 template <typename Tin, typename Tout, int LAYOUT>
 __device__ __forceinline__ void pack_tile_wide(const PackOperand& o, int64_t kt, int64_t rt,
-                                               typename AccOf<Tin>::type (&tile)[PACK_KT_WIDE][33]) {
+                                               typename AccOf<Tin>::type (&tile)[PACK_KT_WIDE][33],
+                                               PackRange<LAYOUT>& rng) {
   using Acc = typename AccOf<Tin>::type;
   constexpr int KT = PACK_KT_WIDE, SB = KT / 32;
   const int64_t k0 = kt * KT, r0 = rt * 32;
@@ -195,7 +230,7 @@ __device__ __forceinline__ void pack_tile_wide(const PackOperand& o, int64_t kt,
     if (k >= o.Kcover) break;
     const float x[4] = {(float)tile[kl][rl], (float)tile[kl + 1][rl], (float)tile[kl + 2][rl],
                         (float)tile[kl + 3][rl]};
-    store_k4<LAYOUT>(base, k, o.Kcover, o.ld, x);
+    store_k4<LAYOUT>(base, k, o.Kcover, o.ld, x, rng);
   }
 }
 
@@ -232,7 +267,7 @@ struct KbWalk {
 // issues all its copies (R T / 256 <= 16) before it waits. FP32 sources only.
 template <typename Tin, int LAYOUT>
 __device__ __forceinline__ void pack_kblock(const PackOperand& o, int64_t kt, int64_t rt,
-                                            float* tile) {
+                                            float* tile, PackRange<LAYOUT>& rng) {
   constexpr int NV = PACK_KB_ELEMS / 256;
   const int lo = o.kb_lo, run = o.kb_run, T = lo * run, R = o.kb_rows, TP = T + T / 32;
   const int64_t k0 = kt * T, r0 = rt * R;
@@ -276,7 +311,7 @@ __device__ __forceinline__ void pack_kblock(const PackOperand& o, int64_t kt, in
     if (row >= o.Rcover || k >= o.Kcover) continue;
     const float* t = tile + r * TP + kq + kq / 32;  // kq % 4 == 0: the quad shares one 32-group
     const float x[4] = {t[0], t[1], t[2], t[3]};
-    store_k4<LAYOUT>(static_cast<__nv_bfloat16*>(o.dst) + row * o.ld, k, o.Kcover, o.ld, x);
+    store_k4<LAYOUT>(static_cast<__nv_bfloat16*>(o.dst) + row * o.ld, k, o.Kcover, o.ld, x, rng);
   }
 }
 
@@ -287,7 +322,7 @@ __device__ __forceinline__ void pack_kblock(const PackOperand& o, int64_t kt, in
 // Quads past K or the last row are read element by element (or zero).
 template <int LAYOUT>
 __device__ __forceinline__ void pack_kblock_quad(const PackOperand& o, int64_t kt, int64_t rt,
-                                                 float* tile) {
+                                                 float* tile, PackRange<LAYOUT>& rng) {
   constexpr int NQ = PACK_KB_ELEMS / 4 / 256;  // 16-byte copies per thread at most
   const int lo = o.kb_lo, run = o.kb_run, T = lo * run, R = o.kb_rows;
   const int nch = run / 4;  // 16-byte chunks per (r, l) row
@@ -331,7 +366,7 @@ __device__ __forceinline__ void pack_kblock_quad(const PackOperand& o, int64_t k
     float x[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) x[j] = chunk(r, l + j, u >> 2)[u & 3];
-    store_k4<LAYOUT>(static_cast<__nv_bfloat16*>(o.dst) + row * o.ld, k, o.Kcover, o.ld, x);
+    store_k4<LAYOUT>(static_cast<__nv_bfloat16*>(o.dst) + row * o.ld, k, o.Kcover, o.ld, x, rng);
   }
 }
 
@@ -346,7 +381,8 @@ __device__ __forceinline__ void pack_kblock_quad(const PackOperand& o, int64_t k
 constexpr int PACK_KS_Q = 4;
 
 template <typename Tin, int LAYOUT>
-__device__ __forceinline__ void pack_kstream(const PackOperand& o, int64_t blk, float* smem) {
+__device__ __forceinline__ void pack_kstream(const PackOperand& o, int64_t blk, float* smem,
+                                             PackRange<LAYOUT>& rng) {
   static_assert(sizeof(Tin) == 4 || sizeof(Tin) == 2, "float or bf16 sources");
   const int64_t qr = o.Kcover / 4;  // quads per row
   const int tid = threadIdx.x + 32 * threadIdx.y;
@@ -387,7 +423,7 @@ __device__ __forceinline__ void pack_kstream(const PackOperand& o, int64_t blk, 
       float x[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) x[j] = load_as_acc<Tin>(d + j);
-      store_k4<LAYOUT>(static_cast<__nv_bfloat16*>(o.dst) + row * o.ld, kq * 4, o.Kcover, o.ld, x);
+      store_k4<LAYOUT>(static_cast<__nv_bfloat16*>(o.dst) + row * o.ld, kq * 4, o.Kcover, o.ld, x, rng);
     }
     kq += dkq;
     row += drow;
@@ -407,29 +443,38 @@ enum PackRead : int {
 };
 
 template <typename Tin, typename Tout, int LAYOUT, int READ>
-__device__ __forceinline__ void pack_any(const PackOperand& o, int64_t kt, int64_t rt) {
+__device__ __forceinline__ void pack_tiles(const PackOperand& o, int64_t kt, int64_t rt,
+                                           PackRange<LAYOUT>& rng) {
   using Acc = typename AccOf<Tin>::type;
   __shared__ __align__(16) Acc tile[PACK_KT_WIDE][33];
   static_assert(PACK_KB_ELEMS + PACK_KB_ELEMS / 32 <= PACK_KT_WIDE * 33, "k-block tile fits");
   static_assert(PACK_KS_Q * 256 * 4 <= PACK_KT_WIDE * 33, "streaming buffer fits");
-  constexpr bool KMAJOR = LAYOUT == PACK_K_BF16 || LAYOUT == PACK_K_BF16X3;
+  constexpr bool KMAJOR = pack_k_major(LAYOUT);
   if constexpr (KMAJOR && (READ == PACK_READ_STREAM || READ == PACK_READ_ANY)) {
     if (READ == PACK_READ_STREAM || o.kstream) {
-      pack_kstream<Tin, LAYOUT>(o, rt, &tile[0][0]);  // one tile along k
+      pack_kstream<Tin, LAYOUT>(o, rt, &tile[0][0], rng);  // one tile along k
       return;
     }
   }
   if constexpr (KMAJOR && sizeof(Tin) == 4 && (READ == PACK_READ_KBLOCK || READ == PACK_READ_ANY)) {
     if (READ == PACK_READ_KBLOCK || o.kb_lo > 0) {
       if (o.kb_quad)
-        pack_kblock_quad<LAYOUT>(o, kt, rt, &tile[0][0]);
+        pack_kblock_quad<LAYOUT>(o, kt, rt, &tile[0][0], rng);
       else
-        pack_kblock<Tin, LAYOUT>(o, kt, rt, &tile[0][0]);
+        pack_kblock<Tin, LAYOUT>(o, kt, rt, &tile[0][0], rng);
       return;
     }
   }
   if constexpr (!KMAJOR || READ == PACK_READ_WIDE || READ == PACK_READ_ANY)
-    pack_tile_wide<Tin, Tout, LAYOUT>(o, kt, rt, tile);
+    pack_tile_wide<Tin, Tout, LAYOUT>(o, kt, rt, tile, rng);
+}
+
+template <typename Tin, typename Tout, int LAYOUT, int READ>
+__device__ __forceinline__ void pack_any(const PackOperand& o, int64_t kt, int64_t rt) {
+  PackRange<LAYOUT> rng;
+  pack_tiles<Tin, Tout, LAYOUT, READ>(o, kt, rt, rng);
+  if constexpr (LAYOUT == PACK_K_F32X6) __syncwarp();
+  rng.flush(o.range);
 }
 
 // grid = (max tiles of the two operands, 1, 2), block = (32, 8); CTA x covers

@@ -41,7 +41,23 @@
 
 namespace tccg {
 
-enum TcMode : int { TC_BF16 = 0, TC_BF16X3 = 1 };
+// TC_F32X6: FP32 results. Operands packed as their exact three-way bf16 split
+// [hi 32 k | mid 32 k | lo 32 k]; per k-step of 16 six MMAs -- hi*hi into the
+// chunk accumulator, and lo*hi, hi*lo, mid*mid, mid*hi, hi*mid into a third
+// one. mid*lo, lo*mid and lo*lo, at most 2^-24 of the product together, are
+// dropped (below the rounding of an FP32 product and sum). Bound: the tensor
+// pipe at 6 MMAs per product, 1/6 of the BF16 rate; FFMA gives 54 TFLOP/s.
+//   Accumulation: every MMA truncates its sum to the accumulator's 24 bits,
+//   so hi*hi runs in chunks of 128 k (8 truncations, chunk sums added RN in
+//   registers) and the five small products, 2^-8 of the sum, stay in the
+//   third accumulator for up to 4096 k, where their truncations count 2^-8.
+//   Tile: 128 x 160 -- three accumulators of 160 columns in 480 of the 512
+//   TMEM columns, and four 54 KB stages beside the epilogue staging.
+//   Values that the split does not represent (infinity, NaN, magnitudes near
+//   either end of the range): the packing pass keeps the operands' ranges,
+//   every role skips the tiles of such a contraction (f32_split_exact), and a
+//   CUDA-core launch behind computes it from the caller's tensors.
+enum TcMode : int { TC_BF16 = 0, TC_BF16X3 = 1, TC_F32X6 = 2 };
 
 // How the operand stages are filled.
 //   TC_LOAD_TMA   : one thread issues 2-D TMA loads of operands packed K-major
@@ -74,23 +90,29 @@ enum GatherRead : int {
 template <int MODE, int LOAD = TC_LOAD_TMA, int BNV = 0>
 struct TcCfgT {
   static constexpr bool GATHER = LOAD == TC_LOAD_GATHER;
+  static constexpr bool X6 = MODE == TC_F32X6;
+  static_assert(!X6 || (!GATHER && BNV == 0), "FP32 split: packed operands, one tile width");
   static_assert(!GATHER || MODE == TC_BF16X3, "the gather loader serves split-BF16x3");
   static_assert(!GATHER || BNV == 0 || BNV == 128, "the gather loader has 128-column tiles");
   static_assert(BNV == 0 || BNV == 128 || BNV == 192 || (BNV == 256 && MODE == TC_BF16),
                 "tile widths: 128, 192 (and 256 for BF16)");
   static constexpr int BM = 128;
-  static constexpr int BN = BNV ? BNV : GATHER ? 128 : (MODE == TC_BF16X3) ? 192 : 256;
-  static constexpr int ROW_BYTES = 128;  // one swizzle row per operand row per stage
+  static constexpr int BN = BNV ? BNV : GATHER ? 128 : X6 ? 160 : (MODE == TC_BF16X3) ? 192 : 256;
+  // one 128-byte swizzle row per operand row per stage; X6: plus the lo part
+  // in a 64-byte swizzle row (after the operand's BM / BN 128-byte rows)
+  static constexpr int ROW_BYTES = X6 ? 192 : 128;
   static constexpr int A_STAGE = BM * ROW_BYTES;   // 16 KB
   static constexpr int B_STAGE = BN * ROW_BYTES;   // 16 / 24 / 32 KB
   static constexpr int STAGE_BYTES = A_STAGE + B_STAGE;
   // default shapes keep their measured ring depths (BF16X3 5 x 40 KB, BF16
   // 4 x 48 KB); other widths take what fits next to the epilogue staging
   static constexpr int STAGES = GATHER ? 2
-                                : BNV == 0 ? ((MODE == TC_BF16X3) ? 5 : 4)
+                                : BNV == 0 ? ((MODE == TC_BF16X3) ? 5 : 4)  // X6 4 x 54 KB
                                 : (200 * 1024 / STAGE_BYTES > 6 ? 6 : 200 * 1024 / STAGE_BYTES);
-  static constexpr int ACC_STRIDE = BN <= 128 ? 128 : 256;  // accumulator b starts at column ACC_STRIDE*b
-  static constexpr int TMEM_COLS = 2 * ACC_STRIDE;       // two accumulators of BN columns
+  static constexpr int ACC_STRIDE = X6 ? BN : BN <= 128 ? 128 : 256;  // accumulator b starts at column ACC_STRIDE*b
+  static constexpr int TMEM_COLS = X6 ? 512 : 2 * ACC_STRIDE;  // two accumulators of BN columns (X6 three)
+  // X6: k-blocks of the small products' accumulator before it is added up
+  static constexpr int SMALL_KB = 128;
   static constexpr int PRODUCER_WARPS = GATHER ? 4 : 1;
   static constexpr int MMA_WARP = PRODUCER_WARPS;
   static constexpr int EPI_WARP0 = PRODUCER_WARPS + 1;
@@ -106,9 +128,10 @@ struct TcCfgT {
   static constexpr int STG_SLOTS = GATHER ? 3 : 0;
   static constexpr int STG_SLOT_BYTES = (BM + BN) * STG_LD * 4;
   static constexpr int ROWCACHE_BYTES = GATHER ? (BM + BN) * 8 : 0;
-  // staged C stores (TcArgs::crun): 32 rows x 16 columns per epilogue warp
+  // staged C stores (TcArgs::crun): 32 rows x EPI_NC columns per epilogue warp
   static constexpr int EPI_LD = 33;
-  static constexpr int EPI_STG_BYTES = EPI_WARPS * 16 * EPI_LD * 4;
+  static constexpr int EPI_NC = X6 ? 8 : 16;
+  static constexpr int EPI_STG_BYTES = EPI_WARPS * EPI_NC * EPI_LD * 4;
   static constexpr size_t SMEM_BYTES = 1024 + (size_t)STAGES * STAGE_BYTES +
                                        (size_t)STG_SLOTS * STG_SLOT_BYTES + ROWCACHE_BYTES +
                                        EPI_STG_BYTES + 256;
@@ -164,6 +187,8 @@ struct TcArgs {
   // C by the first N mode: stores go through shared memory in runs of e0 m
   // by 32 / e0 columns, which are consecutive addresses of C
   int32_t crun;
+  // TC_F32X6: the operands' range words (AbsRange, GA's two then GB's)
+  const uint32_t* range;
 };
 
 // Grouped launch: one entry per contraction, in device memory. The tensor maps
@@ -171,6 +196,8 @@ struct TcArgs {
 struct __align__(64) TcGroupItem {
   CUtensorMap tmA;
   CUtensorMap tmB;
+  CUtensorMap tmAl;  // TC_F32X6: the lo parts
+  CUtensorMap tmBl;
   TcArgs args;
   int64_t tile_begin;  // first global tile of this item
 };
@@ -216,6 +243,8 @@ struct TileRef {
   const TcArgs* a;
   const CUtensorMap* tA;
   const CUtensorMap* tB;
+  const CUtensorMap* tAl;  // TC_F32X6: the lo parts
+  const CUtensorMap* tBl;
   int tm, tn;
   int z, kb_begin, kb_end;
   int tail;  // index among the tail tiles (a slice of it), or -1
@@ -242,18 +271,24 @@ __device__ __forceinline__ void split_coords(int local, const TcArgs& a, TileRef
 template <bool GROUPED>
 __device__ __forceinline__ TileRef resolve_tile(int tile, const CUtensorMap* tmA,
                                                 const CUtensorMap* tmB, const TcArgs* a1,
-                                                const TcGroup& g) {
+                                                const TcGroup& g,
+                                                const CUtensorMap* tmAl = nullptr,
+                                                const CUtensorMap* tmBl = nullptr) {
   TileRef r;
   if constexpr (GROUPED) {
     const TcGroupItem& it = g.items[find_segment(g.tile_begin, g.n_items, tile)];
     r.a = &it.args;
     r.tA = &it.tmA;
     r.tB = &it.tmB;
+    r.tAl = &it.tmAl;
+    r.tBl = &it.tmBl;
     split_coords(tile - (int)it.tile_begin, it.args, r);
   } else {
     r.a = a1;
     r.tA = tmA;
     r.tB = tmB;
+    r.tAl = tmAl;
+    r.tBl = tmBl;
     split_coords(tile, *a1, r);
   }
   return r;
@@ -562,15 +597,25 @@ __device__ __forceinline__ void gather_producer(const TcArgs* a1, const TcGroup&
   cp_async_wait<0>();  // no copy in flight when the producers leave
 }
 
+// TC_F32X6: chunks of `chunk_kb` k-blocks (at most 4) per fill of the small
+// products' accumulator.
+template <int SMALL_KB>
+__device__ __forceinline__ int small_chunks(int chunk_kb) {
+  return chunk_kb < SMALL_KB ? SMALL_KB / chunk_kb : 1;
+}
+
 template <int MODE, int LOAD, int BNV, bool GROUPED>
 __device__ __forceinline__ void gett_tc_body(const CUtensorMap* tmA, const CUtensorMap* tmB,
                                              const TcArgs* a1, const TcGroup& g,
-                                             int32_t* status) {
+                                             int32_t* status, const CUtensorMap* tmAl = nullptr,
+                                             const CUtensorMap* tmBl = nullptr) {
   using Cfg = TcCfgT<MODE, LOAD, BNV>;
+  constexpr bool X6 = Cfg::X6;
+  constexpr int A_LO = Cfg::BM * 128, B_LO = Cfg::BN * 128;  // X6: lo rows inside a stage
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + (((raw_addr + 1023u) & ~1023u) - raw_addr);
-  uint8_t* sA = smem;                                   // STAGES x 16 KB
+  uint8_t* sA = smem;                                   // STAGES x A_STAGE
   uint8_t* sB = smem + Cfg::STAGES * Cfg::A_STAGE;      // STAGES x B_STAGE
   // gather: FP32 staging slots and the row-offset cache after the stages
   float* stg = reinterpret_cast<float*>(smem + Cfg::STAGES * Cfg::STAGE_BYTES);
@@ -587,7 +632,9 @@ __device__ __forceinline__ void gett_tc_body(const CUtensorMap* tmA, const CUten
   uint64_t* accf = bars + 2 * Cfg::STAGES; // [2] accumulator ready
   uint64_t* acce = accf + 2;               // [2] accumulator drained
   uint64_t* drain = acce + 2;              // MMA completion on the abort path
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
+  uint64_t* smf = drain + 1;               // X6: small products' accumulator ready
+  uint64_t* sme = smf + 1;                 //     and drained
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sme + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_tiles =
@@ -615,10 +662,18 @@ __device__ __forceinline__ void gett_tc_body(const CUtensorMap* tmA, const CUten
       mbar_init(&acce[b], Cfg::EPI_WARPS);
     }
     mbar_init(drain, 1);
+    if (X6) {
+      mbar_init(smf, 1);
+      mbar_init(sme, Cfg::EPI_WARPS);
+    }
     fence_mbar_init();
     if (!GROUPED && !Cfg::GATHER) {
       tma_prefetch_desc(tmA);
       tma_prefetch_desc(tmB);
+      if (X6) {
+        tma_prefetch_desc(tmAl);
+        tma_prefetch_desc(tmBl);
+      }
     }
   }
   if (warp == Cfg::MMA_WARP) tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
@@ -643,7 +698,8 @@ __device__ __forceinline__ void gett_tc_body(const CUtensorMap* tmA, const CUten
     for (int s = 0; s < Cfg::STAGES; ++s) issued_phase[s] = -1;
     bool ok = true;
     for (int tile = cta; tile < num_tiles && ok; tile += gridDim.x) {
-      const TileRef t = resolve_tile<GROUPED>(tile, tmA, tmB, a1, g);
+      const TileRef t = resolve_tile<GROUPED>(tile, tmA, tmB, a1, g, tmAl, tmBl);
+      if (X6 && !f32_split_exact(t.a->range, t.a->K)) continue;
       for (int kb = t.kb_begin; kb < t.kb_end; ++kb) {
         if (!mbar_wait(&empty[stage], phase ^ 1, wait_ns)) {
           record_error(status, 1);
@@ -652,8 +708,15 @@ __device__ __forceinline__ void gett_tc_body(const CUtensorMap* tmA, const CUten
         }
         if (tile + 1 != skip_tile1 || kb != t.kb_begin) {
           mbar_arrive_expect_tx(&full[stage], Cfg::STAGE_BYTES);
-          tma_load_2d(sA + stage * Cfg::A_STAGE, t.tA, kb * 64, t.tm * Cfg::BM, &full[stage]);
-          tma_load_2d(sB + stage * Cfg::B_STAGE, t.tB, kb * 64, t.tn * Cfg::BN, &full[stage]);
+          constexpr int KB_COLS = X6 ? 96 : 64;  // packed columns of a k-block
+          tma_load_2d(sA + stage * Cfg::A_STAGE, t.tA, kb * KB_COLS, t.tm * Cfg::BM, &full[stage]);
+          tma_load_2d(sB + stage * Cfg::B_STAGE, t.tB, kb * KB_COLS, t.tn * Cfg::BN, &full[stage]);
+          if constexpr (X6) {
+            tma_load_2d(sA + stage * Cfg::A_STAGE + A_LO, t.tAl, kb * KB_COLS + 64, t.tm * Cfg::BM,
+                        &full[stage]);
+            tma_load_2d(sB + stage * Cfg::B_STAGE + B_LO, t.tBl, kb * KB_COLS + 64, t.tn * Cfg::BN,
+                        &full[stage]);
+          }
           issued_phase[stage] = (int)phase;
         }
         if (++stage == Cfg::STAGES) {
@@ -673,9 +736,14 @@ __device__ __forceinline__ void gett_tc_body(const CUtensorMap* tmA, const CUten
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true, issued_any = false;
+    uint32_t sm_phase = 0;  // X6: fills of the small products' accumulator
     for (int tile = cta; tile < num_tiles && ok; tile += gridDim.x) {
       const TileRef t = resolve_tile<GROUPED>(tile, tmA, tmB, a1, g);
+      if (X6 && !f32_split_exact(t.a->range, t.a->K)) continue;
       const int nkb = t.kb_end, K = t.a->K, ckb = t.a->chunk_kb;
+      const int seg = small_chunks<Cfg::SMALL_KB>(ckb);  // X6: chunks per fill
+      int seg_ch = 0;
+      uint32_t sm_acc = 0;
       // the MMAs stop at the tile's last column of C, rounded up to 32 (the
       // epilogue reads no further): a narrow C, or the last column tile,
       // costs only the tensor work its columns need
@@ -687,6 +755,16 @@ __device__ __forceinline__ void gett_tc_body(const CUtensorMap* tmA, const CUten
           record_error(status, 2);
           ok = false;
           break;
+        }
+        if constexpr (X6) {
+          if (seg_ch == 0) {
+            if (!mbar_wait(sme, sm_phase ^ 1, wait_ns)) {
+              record_error(status, 2);
+              ok = false;
+              break;
+            }
+            sm_acc = 0;
+          }
         }
         tc_fence_after();
         const uint32_t d_tmem = tbase + (uint32_t)(acc * Cfg::ACC_STRIDE);
@@ -707,6 +785,25 @@ __device__ __forceinline__ void gett_tc_body(const CUtensorMap* tmA, const CUten
               if (kb * 64 + ks * 16 < K) {
                 tc_mma_f16(d_tmem, ad + 2 * ks, bd + 2 * ks, idesc, accumulate);
                 accumulate = 1;
+              }
+            }
+          } else if constexpr (X6) {
+            const uint32_t d_small = tbase + (uint32_t)(2 * Cfg::ACC_STRIDE);
+            const uint64_t al = umma_desc_k64(smem_u32(sA + stage * Cfg::A_STAGE + A_LO));
+            const uint64_t bl = umma_desc_k64(smem_u32(sB + stage * Cfg::B_STAGE + B_LO));
+#pragma unroll
+            for (int ks = 0; ks < 2; ++ks) {
+              if (kb * 32 + ks * 16 < K) {
+                // +4 = 64 B: the mid half of the 128-byte row
+                const uint64_t ah = ad + 2 * ks, bh = bd + 2 * ks;
+                tc_mma_f16(d_small, al + 2 * ks, bh, idesc, sm_acc);
+                tc_mma_f16(d_small, ah, bl + 2 * ks, idesc, 1);
+                tc_mma_f16(d_small, ah + 4, bh + 4, idesc, 1);
+                tc_mma_f16(d_small, ah + 4, bh, idesc, 1);
+                tc_mma_f16(d_small, ah, bh + 4, idesc, 1);
+                tc_mma_f16(d_tmem, ah, bh, idesc, accumulate);
+                accumulate = 1;
+                sm_acc = 1;
               }
             }
           } else {
@@ -731,6 +828,13 @@ __device__ __forceinline__ void gett_tc_body(const CUtensorMap* tmA, const CUten
         }
         if (!ok) break;
         tc_commit(&accf[acc]);  // chunk sum ready for the epilogue
+        if constexpr (X6) {
+          if (++seg_ch == seg || kend == nkb) {
+            tc_commit(smf);
+            sm_phase ^= 1;
+            seg_ch = 0;
+          }
+        }
         if (++acc == 2) {
           acc = 0;
           acc_phase ^= 1;
@@ -746,13 +850,14 @@ __device__ __forceinline__ void gett_tc_body(const CUtensorMap* tmA, const CUten
     const int q = warp & 3;             // TMEM lanes [32q, 32q+32) are accessible to this warp
     const int h = (warp - Cfg::EPI_WARP0) >> 2;  // column half of the tile
     constexpr int HC = Cfg::BN / 2;     // columns per epilogue warp
-    float* wstg = epi_stg + (warp - Cfg::EPI_WARP0) * 16 * Cfg::EPI_LD;  // staged C stores
+    float* wstg = epi_stg + (warp - Cfg::EPI_WARP0) * Cfg::EPI_NC * Cfg::EPI_LD;  // staged C stores
     int acc = 0;
-    uint32_t acc_phase = 0;
+    uint32_t acc_phase = 0, sm_phase = 0;
     bool ok = true;
     for (int tile = cta; tile < num_tiles && ok; tile += gridDim.x) {
       const TileRef t = resolve_tile<GROUPED>(tile, tmA, tmB, a1, g);
       const TcArgs& a = *t.a;
+      if (X6 && !f32_split_exact(a.range, a.K)) continue;
       const int64_t m = (int64_t)t.tm * Cfg::BM + q * 32 + lane;
       const bool m_ok = m < a.M;
       const int64_t cmo = m_ok ? a.c_m_off[m] : 0;
@@ -852,11 +957,14 @@ __device__ __forceinline__ void gett_tc_body(const CUtensorMap* tmA, const CUten
         // C's offsets of this warp's columns, column 32 i + lane in lane's
         // cn[i] (loaded while the MMAs run; passed around by shuffles when
         // storing, so no store waits on a table load)
-        int64_t cn[HC / 32];
+        constexpr int CG = (HC + 31) / 32;
+        int64_t cn[CG];
 #pragma unroll
-        for (int i = 0; i < HC / 32; ++i)
+        for (int i = 0; i < CG; ++i)
           cn[i] = 32 * i + lane < nlim ? __ldg(cno + 32 * i + lane) : 0;
         float sum[HC];
+        const int seg = small_chunks<Cfg::SMALL_KB>(a.chunk_kb);
+        int seg_ch = 0;
         for (int ch = 0; ch < nchunks; ++ch) {
           if (!mbar_wait(&accf[acc], acc_phase, wait_ns)) {
             record_error(status, 3);
@@ -884,6 +992,34 @@ __device__ __forceinline__ void gett_tc_body(const CUtensorMap* tmA, const CUten
             acc = 0;
             acc_phase ^= 1;
           }
+          if constexpr (X6) {  // the five small products of the last `seg` chunks
+            if (++seg_ch == seg || ch + 1 == nchunks) {
+              seg_ch = 0;
+              if (!mbar_wait(smf, sm_phase, wait_ns)) {
+                record_error(status, 3);
+                ok = false;
+                break;
+              }
+              sm_phase ^= 1;
+              tc_fence_after();
+              const uint32_t ssrc =
+                  tbase + ((uint32_t)(q * 32) << 16) + (uint32_t)(2 * Cfg::ACC_STRIDE + h * HC);
+#pragma unroll
+              for (int cc = 0; cc < HC; cc += 16) {
+                if (cc < nlim) {
+                  uint32_t r[16];
+                  tmem_ld_32x32b_x16(ssrc + (uint32_t)cc, r);
+                  tmem_ld_wait();
+#pragma unroll
+                  for (int j = 0; j < 16; ++j)
+                    sum[cc + j] = __fadd_rn(sum[cc + j], __uint_as_float(r[j]));
+                }
+              }
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(sme);
+            }
+          }
         }
         if (!ok) break;
         if (part) {  // warp-uniform, like the branches below
@@ -893,17 +1029,18 @@ __device__ __forceinline__ void gett_tc_body(const CUtensorMap* tmA, const CUten
               if (j < nlim) part[(size_t)(pc0 + j) * pld] = sum[j];
           }
         } else if (a.crun > 0) {
+          constexpr int NC = Cfg::EPI_NC;
 #pragma unroll
-          for (int cc = 0; cc < HC; cc += 16) {
+          for (int cc = 0; cc < HC; cc += NC) {
             if (cc < nlim) {  // warp-uniform
               __syncwarp();
 #pragma unroll
-              for (int j = 0; j < 16; ++j) wstg[j * Cfg::EPI_LD + lane] = sum[cc + j];
+              for (int j = 0; j < NC; ++j) wstg[j * Cfg::EPI_LD + lane] = sum[cc + j];
               __syncwarp();
               const int64_t left = nlim - cc;
               const int64_t cn_lane =
-                  lane < 16 && cc + lane < nlim ? __ldg(cno + cc + lane) : 0;
-              store_runs(wstg, a, (int64_t)t.tm * Cfg::BM + q * 32, left < 16 ? (int)left : 16,
+                  lane < NC && cc + lane < nlim ? __ldg(cno + cc + lane) : 0;
+              store_runs(wstg, a, (int64_t)t.tm * Cfg::BM + q * 32, left < NC ? (int)left : NC,
                          a.crun, alpha, beta, lane, cmo, cn_lane);
             }
           }
@@ -957,6 +1094,19 @@ __global__ void __launch_bounds__(TcCfgT<MODE, LOAD, BNV>::NUM_THREADS, 1)
   gett_tc_body<MODE, LOAD, BNV, true>(nullptr, nullptr, nullptr, g, status);
 }
 
+// FP32 results (TC_F32X6): the hi | mid parts through tmA / tmB, the lo parts
+// through tmAl / tmBl, all on the packed operands.
+template <int MODE, int LOAD = TC_LOAD_TMA, int BNV = 0>
+__global__ void __launch_bounds__(TcCfgT<MODE, LOAD, BNV>::NUM_THREADS, 1)
+    gett_tc_f32_kernel(const __grid_constant__ CUtensorMap tmA,
+                       const __grid_constant__ CUtensorMap tmB,
+                       const __grid_constant__ CUtensorMap tmAl,
+                       const __grid_constant__ CUtensorMap tmBl, const TcArgs a) {
+  static_assert(MODE == TC_F32X6, "FP32 split");
+  TcGroup g{nullptr, nullptr, 0, 0};
+  gett_tc_body<MODE, LOAD, BNV, false>(&tmA, &tmB, &a, g, a.status, &tmAl, &tmBl);
+}
+
 // Tail split: C = alpha * (slice 0 + slice 1 + ...) + beta * C over the tail
 // tiles (RN adds in slice order). grid = (tail tiles, BM * BN / 256), block
 // 256: thread e of a tile takes element (m_local = e % BM, n_local = e / BM).
@@ -964,6 +1114,7 @@ template <int MODE, int LOAD = TC_LOAD_TMA, int BNV = 0>
 __global__ void __launch_bounds__(256) tc_tail_reduce_kernel(const TcArgs a) {
   using Cfg = TcCfgT<MODE, LOAD, BNV>;
   grid_dep_wait();  // partial sums written by the GETT kernel before
+  if (MODE == TC_F32X6 && !f32_split_exact(a.range, a.K)) return;
   const int tail = a.tiles_m * a.tiles_n - a.full_tiles;
   const int tl = blockIdx.x;
   const int e = blockIdx.y * 256 + threadIdx.x;

@@ -112,6 +112,10 @@ struct tccg_plan {
   // TcArgs::crun), or 0
   int32_t crun = 0;
   int32_t tcv = 0;  // TcVariant of a tensor-core plan
+  // FP32 on the tensor cores (TC_F32X6): operands as exact three-way bf16
+  // splits, their range words at off_range
+  bool f32x6 = false;
+  size_t off_range = 0;
   // skinny kernel (skinny_gett.cuh): geometry and tables in sk (operand, C
   // and slice pointers are filled in per run); s_is_n: the narrow side is N
   bool skinny = false, sk_s_is_n = false, sk_p_vec = false;
@@ -142,6 +146,7 @@ enum TcVariant : int {
   TCV_BF16,           // BF16, packing pass + TMA, 128 x 256
   TCV_BF16_N192,      // BF16, packing pass + TMA, 128 x 192
   TCV_BF16_N128,      // BF16, packing pass + TMA, 128 x 128
+  TCV_F32X6,          // FP32 as six bf16 products, packing pass + TMA, 128 x 160
   TCV_COUNT
 };
 
@@ -149,7 +154,12 @@ template <int MODE, int LOAD, int BNV>
 struct TcKernels {
   using Cfg = TcCfgT<MODE, LOAD, BNV>;
   static constexpr bool GATHER = LOAD == TC_LOAD_GATHER;
-  static constexpr auto single = &gett_tc_kernel<MODE, LOAD, BNV>;
+  static constexpr auto single = [] {
+    if constexpr (MODE == TC_F32X6)
+      return &gett_tc_f32_kernel<MODE, LOAD, BNV>;
+    else
+      return &gett_tc_kernel<MODE, LOAD, BNV>;
+  }();
   static constexpr auto group = &gett_tc_group_kernel<MODE, LOAD, BNV>;
   static constexpr auto tail = &tc_tail_reduce_kernel<MODE, LOAD, BNV>;
 };
@@ -163,6 +173,7 @@ static void with_tc_variant(int v, F&& f) {
     case TCV_X3_GATHER: f(TcKernels<TC_BF16X3, TC_LOAD_GATHER, 0>{}); break;
     case TCV_BF16: f(TcKernels<TC_BF16, TC_LOAD_TMA, 0>{}); break;
     case TCV_BF16_N192: f(TcKernels<TC_BF16, TC_LOAD_TMA, 192>{}); break;
+    case TCV_F32X6: f(TcKernels<TC_F32X6, TC_LOAD_TMA, 0>{}); break;
     default: f(TcKernels<TC_BF16, TC_LOAD_TMA, 128>{}); break;
   }
 }
@@ -286,8 +297,42 @@ static double simt_time(const tccg_plan* p) {
   return std::max(2.0 * simt_work * K / 35e12, (cb + simt_passes * op) / 4.5e12);
 }
 
+// FP32 as six bf16 products on the tensor cores (TC_F32X6). Its normwise error
+// against FP64 on N(0, 1) values is below FFMA's at every K measured (K = 64:
+// 0.7e-7 against 1.4e-7, 256: 1.2e-7 / 2.9e-7, 1024: 1.3e-7 / 5.7e-7, 4096:
+// 1.6e-7 / 1.15e-6; the same order for uniform and for wide-ranged values),
+// so time decides: tiles of 128 x 160 at 0.72 us per 32 k and round of the
+// persistent grid (half rounds where the tail split applies), the pack's 4 + 6
+// and the loads' 6 bytes per element at 4.5 TB/s and 20 us of launches,
+// against FFMA at 45 TFLOP/s on padded tiles. 2048 x 2080 x K, us: K = 128
+// 31.8 against 35.6 (both near the launch floor; the rule keeps FFMA), 256: 38
+// / 59, 512: 54 / 106, 4096: 228 / 773. Half a round of tiles at least (no
+// k-split here). A tuning that names a CUDA-core form (variant < 0, direct,
+// shortk, simt_tile, an explicit k-split) keeps the CUDA cores; variant > 0
+// asks for this path.
+static constexpr int64_t F32X6_MIN_K = 128;  // an accumulation chunk
+static constexpr int F32X6_BM = TcCfgT<TC_F32X6>::BM, F32X6_BN = TcCfgT<TC_F32X6>::BN;
+static bool choose_f32x6(const tccg_plan* p) {
+  const tccg_tuning& t = p->tune;
+  if (p->prec != TCCG_PREC_FP32 || p->dtype != TCCG_F32 || t.method != TCCG_METHOD_GETT || t.pair ||
+      t.variant < 0 || t.ksplit > 1 || t.direct > 0 || t.shortk > 0 || t.simt_tile != 0)
+    return false;
+  const int64_t lim = int64_t(1) << 30;
+  if (p->M >= lim || p->N >= lim || p->K >= lim) return false;
+  if (t.variant > 0) return true;
+  const int64_t tiles = cdiv(p->M, F32X6_BM) * cdiv(p->N, F32X6_BN);
+  if (p->K < F32X6_MIN_K || 2 * tiles < p->num_sms) return false;
+  const double rounds = std::max(1.0, 0.5 * (double)cdiv(2 * tiles, p->num_sms));
+  const double K = (double)p->K;
+  const double t_tc = rounds * (K / 32) * 0.72e-6 +
+                      (double)(p->M + p->N) * K * 16.0 / 4.5e12 + 20e-6;
+  const double t_ffma = 2.0 * (double)round_up(p->M, 128) * (double)round_up(p->N, 128) * K / 45e12;
+  return t_tc < t_ffma;
+}
+
 static bool choose_simt(const tccg_plan* p) {
-  if (p->prec == TCCG_PREC_FP32 || p->prec == TCCG_PREC_FP64) return true;
+  if (p->prec == TCCG_PREC_FP32) return !choose_f32x6(p);
+  if (p->prec == TCCG_PREC_FP64) return true;
   if (p->tune.pair || p->tune.variant > 0 || p->tune.load > 0) return false;
   if (p->tune.variant < 0) return true;
   // against the tensor-core model (tc_time, with the loader the tuning asks for)
@@ -1009,6 +1054,7 @@ extern "C" int tccg_plan_create(const tccg_desc* desc, int32_t dtype, int32_t pr
     }
   }
   p->simt = !p->skinny && choose_simt(p);
+  p->f32x6 = !p->skinny && !p->simt && p->prec == TCCG_PREC_FP32;
   p->read_k_fast_a = pick_read_k_fast(d.nm, d.m_ext, d.a_m_stride, d.nk, d.k_ext, d.a_k_stride);
   p->read_k_fast_b = pick_read_k_fast(d.nn, d.n_ext, d.b_n_stride, d.nk, d.k_ext, d.b_k_stride);
   if (!p->skinny && !simt_path(p) && p->tune.load == 2 && p->prec == TCCG_PREC_BF16X3 && p->dtype == TCCG_F32 &&
@@ -1154,17 +1200,19 @@ static int plan_layout(tccg_plan* p) {
              p->direct ? (int)p->gather_k_a : p->read_k_fast_a,
              p->direct ? (int)p->gather_k_b : p->read_k_fast_b);
   } else {
-    const bool x3 = p->prec == TCCG_PREC_BF16X3;
-    if (x3) {
-      p->Kc = 2 * round_up(p->K, 32);
+    const bool x3 = p->prec == TCCG_PREC_BF16X3, x6 = p->f32x6;
+    if (x3 || x6) {
+      p->Kc = (x6 ? 3 : 2) * round_up(p->K, 32);
       p->num_kb = (int32_t)cdiv(p->K, 32);
     } else {
       p->Kc = round_up(p->K, 8);
       p->num_kb = (int32_t)cdiv(p->K, 64);
     }
     // BF16X3 accumulates 512 k per TMEM accumulator (tuning.variant overrides,
-    // in k-blocks of 32); BF16 one chunk per tile
-    p->chunk_kb = x3 ? (p->tune.variant > 0 ? p->tune.variant : 16) : p->num_kb;
+    // in k-blocks of 32), FP32 at most 128 (its error bound needs short
+    // chunks: 6400 k in one gave 6e-6); BF16 one chunk per tile
+    p->chunk_kb = x3 || x6 ? (p->tune.variant > 0 ? p->tune.variant : x6 ? 4 : 16) : p->num_kb;
+    if (x6) p->chunk_kb = std::min(p->chunk_kb, 4);
     if (p->chunk_kb < 1) p->chunk_kb = 1;
     const bool pair = p->tune.pair != 0;
     int stages = 0;
@@ -1172,7 +1220,7 @@ static int plan_layout(tccg_plan* p) {
       p->bn = x3 ? Tc2Cfg<TC_BF16X3>::BN : Tc2Cfg<TC_BF16>::BN;
       stages = x3 ? Tc2Cfg<TC_BF16X3>::STAGES : Tc2Cfg<TC_BF16>::STAGES;
     } else {
-      p->tcv = tc_variant(x3, p->gather, p->tune.tile_n);
+      p->tcv = x6 ? TCV_F32X6 : tc_variant(x3, p->gather, p->tune.tile_n);
       if (p->tcv < 0)
         return fail(TCCG_ERR_UNSUPPORTED, "tile width %d is not built for %s%s", p->tune.tile_n,
                     x3 ? "BF16X3" : "BF16", p->gather ? " with the gather loader" : "");
@@ -1190,7 +1238,7 @@ static int plan_layout(tccg_plan* p) {
     int ctas = p->tune.max_ctas > 0 ? std::min(p->tune.max_ctas, p->num_sms) : p->num_sms;
     // one CTA per SM; a slice is at least one accumulation chunk (BF16X3) or
     // 512 k (BF16). The CTA-pair kernel does not split.
-    p->kb_per_split = (int32_t)choose_ksplit(pair ? 1 : p->tune.ksplit, tiles, p->num_kb, ctas,
+    p->kb_per_split = (int32_t)choose_ksplit(pair || x6 ? 1 : p->tune.ksplit, tiles, p->num_kb, ctas,
                                              x3 ? p->chunk_kb : 8, &p->ksplit);
     tiles *= p->ksplit;
     // Tail split: whole rounds of the persistent grid plus a short tail (at
@@ -1198,8 +1246,8 @@ static int plan_layout(tccg_plan* p) {
     // last round while the full tiles keep all of K. It saves (1 - 1/slices)
     // of a tile's time and costs the slices' partial sums (written, read back,
     // C written) and a launch, so it is taken only for long tiles: a tile at
-    // about 0.52 us per k-block (BF16X3, 128 x 192) or 0.47 us (BF16,
-    // 128 x 256), the partial sums at 6.5 TB/s, 5 us fixed. Automatic k-split
+    // about 0.52 us per k-block (BF16X3, 128 x 192), 0.47 us (BF16, 128 x 256)
+    // or 0.72 us (FP32, 128 x 160), the partial sums at 6.5 TB/s, 5 us fixed. Automatic k-split
     // only (not with an explicit ksplit, nor for the CTA-pair kernel).
     const int64_t mn = (int64_t)p->tiles_m * p->tiles_n;
     p->full_tiles = 0;
@@ -1207,12 +1255,12 @@ static int plan_layout(tccg_plan* p) {
     p->tail_kb = 0;
     if (!pair && p->ksplit == 1 && p->tune.ksplit == 0 && p->tune.tail_split >= 0 && mn > ctas) {
       const int64_t full = mn / ctas * ctas, tail = mn - full;
-      const int64_t min_kb = x3 ? p->chunk_kb : 8;
+      const int64_t min_kb = x3 ? p->chunk_kb : x6 ? 16 : 8;
       const int64_t want = tail > 0 ? std::min<int64_t>(ctas / tail, p->num_kb / min_kb) : 0;
       if (tail > 0 && 2 * tail <= ctas && want >= 2) {
         const int64_t per = cdiv(p->num_kb, want);  // no empty slice
         const int64_t splits = cdiv(p->num_kb, per);
-        const double t_tile = p->num_kb * (x3 ? 0.52e-6 : 0.47e-6);
+        const double t_tile = p->num_kb * (x6 ? 0.72e-6 : x3 ? 0.52e-6 : 0.47e-6);
         const double t_sum =
             5e-6 + (double)tail * 128 * p->bn * 4 * (2.0 * splits + 2.0) / 6.5e12;
         if ((1.0 - 1.0 / splits) * t_tile > t_sum) {
@@ -1238,6 +1286,10 @@ static int plan_layout(tccg_plan* p) {
       p->off_b = ws;
       ws = align_up(ws + (size_t)(p->N * p->Kc) * 2, 256);
     }
+    if (x6) {  // the operands' range words
+      p->off_range = ws;
+      ws += 256;
+    }
     if (p->ksplit > 1) {  // FP32 slices [split][N][M]
       p->off_part = ws;
       ws = align_up(ws + (size_t)p->ksplit * p->N * p->M * 4, 256);
@@ -1261,11 +1313,12 @@ static int plan_layout(tccg_plan* p) {
              "method=%s prec=%s kernel=gett_tc%s<%s> tile=%dx%d stages=%d M=%lld N=%lld K=%lld "
              "kblocks=%d chunk=%d ksplit=%d tail=%dx%d grid=%d raster=%d pack=K-major bf16%s(read_k_fast a=%d b=%d "
              "visit a=%d b=%d kblock a=%dx%dx%d%s b=%dx%dx%d%s kstream a=%d b=%d)",
-             ttgt ? "TTGT" : "GETT", x3 ? "bf16x3" : "bf16", pair ? "2" : "", x3 ? "BF16X3" : "BF16",
+             ttgt ? "TTGT" : "GETT", x6 ? "fp32" : x3 ? "bf16x3" : "bf16", pair ? "2" : "",
+             x6 ? "F32X6" : x3 ? "BF16X3" : "BF16",
              pair ? 256 : 128, p->bn, stages,
              (long long)p->M, (long long)p->N, (long long)p->K, p->num_kb, p->chunk_kb, p->ksplit,
              p->tail_split > 1 ? (int)((int64_t)p->tiles_m * p->tiles_n - p->full_tiles) : 0,
-             p->tail_split, p->grid, p->raster, x3 ? " hi|lo " : " ", p->read_k_fast_a, p->read_k_fast_b,
+             p->tail_split, p->grid, p->raster, x6 ? " hi|mid|lo " : x3 ? " hi|lo " : " ", p->read_k_fast_a, p->read_k_fast_b,
              p->t_a_vsrc ? 1 : 0, p->t_b_vsrc ? 1 : 0, p->kb_a[0], p->kb_a[1], p->kb_a[2],
              p->kb_a[0] && p->kbq_a ? " x16B" : "", p->kb_b[0], p->kb_b[1], p->kb_b[2],
              p->kb_b[0] && p->kbq_b ? " x16B" : "", p->ks_a ? 1 : 0, p->ks_b ? 1 : 0);
@@ -1308,18 +1361,27 @@ extern "C" int tccg_plan_workspace(const tccg_plan* p, size_t* bytes) {
 // is the cost. Default: on for the CUDA-core kernels (independent CTAs) and
 // for tcgen05 grids of at most 4 rounds (little reuse across rounds to
 // lose); TCCG_B200_PDL=1 / =0 in the environment forces it on / off.
-static bool pdl_auto(const tccg_plan* p) {
-  if (p->simt || p->skinny) return true;
+// FP32 plans on the tensor cores have a third kernel (f32_fallback_kernel),
+// always dependent; their tcgen05 grid follows the same rounds rule
+// (tc_dependent).
+static bool few_rounds(const tccg_plan* p) {
   const int64_t mn = (int64_t)p->tiles_m * p->tiles_n;
   const int64_t tiles = p->tail_split > 1 ? p->full_tiles + (mn - p->full_tiles) * p->tail_split
                                           : mn * p->ksplit;
   return tiles <= 4 * (int64_t)std::max(p->grid, 1);
+}
+static bool pdl_auto(const tccg_plan* p) {
+  return p->simt || p->skinny || p->f32x6 || few_rounds(p);
 }
 static int pdl_forced() {  // 1 on, 0 off, -1 the size rule
   const char* e = std::getenv("TCCG_B200_PDL");
   if (e && e[0] == '0') return 0;
   if (e && e[0] == '1') return 1;
   return -1;
+}
+// Whether the tcgen05 kernel itself may start while the packing pass drains.
+static bool tc_dependent(const tccg_plan* p) {
+  return !p->f32x6 || pdl_forced() == 1 || few_rounds(p);
 }
 // Whether tccg_plan_run launches this plan's kernels with programmatic
 // dependent launch; tccg_plan_run_timed never does (an event sits between
@@ -1384,6 +1446,10 @@ static cudaError_t set_attrs() {
                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SimtShortKCfg<double>::SMEM_BYTES));
   chk(cudaFuncSetAttribute(simt_shortk_kernel<double, false>,
                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SimtShortKCfg<double>::SMEM_BYTES));
+  chk(cudaFuncSetAttribute(f32_fallback_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)simt_smem_bytes<float>()));
+  chk(cudaFuncSetAttribute(f32_fallback_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)simt_smem_bytes<float>()));
   for (int v = 0; v < TCV_COUNT; ++v)
     with_tc_variant(v, [&](auto k) {
       using K = decltype(k);
@@ -1473,20 +1539,21 @@ static int get_encode() {
   return TCCG_OK;
 }
 
-// 2-D bf16 K-major operand [rows][cols], box {64, box_rows}, 128-byte swizzle.
+// 2-D bf16 K-major operand [rows][cols], box {64, box_rows} with the 128-byte
+// swizzle, or {32, box_rows} with the 64-byte one.
 static int encode_kmajor(CUtensorMap* tm, const void* base, int64_t rows, int64_t cols,
-                         int box_rows) {
+                         int box_rows, int box_cols = 64) {
   int rc = get_encode();
   if (rc) return rc;
   if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0 || (cols * 2) % 16 != 0)
     return fail(TCCG_ERR_ALIGNMENT, "TMA operand not 16-byte aligned");
   cuuint64_t gdim[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
   cuuint64_t gstride[1] = {(cuuint64_t)(cols * 2)};
-  cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
+  cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = g_encode(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), gdim,
                         gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        box_cols == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(TCCG_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
   return TCCG_OK;
@@ -1593,6 +1660,7 @@ static PackOperand pack_op(const void* src, const int64_t* roff, const int64_t* 
   o.kb_lo = o.kb_run = o.kb_rows = o.kb_ext = o.kb_step = o.kb_quad = 0;
   o.kstream = 0;
   o.ktiles = o.tiles = 0;
+  o.range = nullptr;
   return o;
 }
 
@@ -1663,7 +1731,7 @@ static int launch_pack(PackArgs pa, cudaStream_t s, bool* launched = nullptr) {
   if (ctas == 0) return TCCG_OK;
   if (launched) *launched = true;
   const dim3 grid((unsigned)ctas, 1, 2), block(32, 8);
-  constexpr bool KMAJOR = LAYOUT == PACK_K_BF16 || LAYOUT == PACK_K_BF16X3;
+  constexpr bool KMAJOR = pack_k_major(LAYOUT);
   mark(0, 0, s);
   if (!KMAJOR || read == PACK_READ_WIDE)
     pack_kernel<Tin, Tout, LAYOUT, PACK_READ_WIDE><<<grid, block, 0, s>>>(pa);
@@ -1823,7 +1891,45 @@ static TcArgs tc_args(const tccg_plan* p, float* Cout, const int64_t* c_m, const
   a.tail_partial = p->tail_split > 1 ? reinterpret_cast<float*>(ws + p->off_tail) : nullptr;
   a.crun = c_m == p->t_c_m ? p->crun : 0;  // not for TTGT's contiguous C'
   a.sm_order = sm_order_enabled() ? 1 : 0;
+  a.range = p->f32x6 ? reinterpret_cast<uint32_t*>(ws + p->off_range) : nullptr;
   return a;
+}
+
+// The four tensor maps of an FP32 plan's packed operands: hi | mid (64
+// columns of a k-block, 128-byte swizzle) and lo (32 columns, 64-byte
+// swizzle).
+static int encode_f32x6(const tccg_plan* p, void* Ap, void* Bp, CUtensorMap* tmA, CUtensorMap* tmB,
+                        CUtensorMap* tmAl, CUtensorMap* tmBl) {
+  int rc = encode_kmajor(tmA, Ap, p->M, p->Kc, F32X6_BM);
+  if (!rc) rc = encode_kmajor(tmB, Bp, p->N, p->Kc, F32X6_BN);
+  if (!rc) rc = encode_kmajor(tmAl, Ap, p->M, p->Kc, F32X6_BM, 32);
+  if (!rc) rc = encode_kmajor(tmBl, Bp, p->N, p->Kc, F32X6_BN, 32);
+  return rc;
+}
+
+// The CUDA-core form of an FP32 plan on the tensor cores, for values its
+// operand splits do not represent.
+static F32FallbackItem f32_fallback_item(const tccg_plan* p, const void* GA, const void* GB,
+                                         float* C, const uint32_t* range, float alpha, float beta) {
+  F32FallbackItem it{};
+  SimtArgs<float>& a = it.args;
+  a.M = p->M;
+  a.N = p->N;
+  a.ktiles = a.ktiles_per_split = (int32_t)cdiv(p->K, SimtCfg<float>::BK);
+  a.C = C;
+  a.c_m_off = p->t_c_m;
+  a.c_n_off = p->t_c_n;
+  a.alpha = alpha;
+  a.beta = beta;
+  set_direct(a, p, GA, GB);
+  a.direct = 1;
+  a.status = p->d_status;
+  a.crun = p->crun;
+  it.range = range;
+  it.K = (int32_t)p->K;
+  it.tiles_m = (int32_t)cdiv(p->M, SimtCfg<float>::BM);
+  it.tiles = (int64_t)it.tiles_m * cdiv(p->N, SimtCfg<float>::BN);
+  return it;
 }
 
 // Gather loader: the kernel reads GA and GB through the plan's offset tables.
@@ -1868,9 +1974,9 @@ static int tc_reduce(const tccg_plan* p, const TcArgs& a, float* Cout, const int
 static int run_tc(const tccg_plan* p, const void* GA, const void* GB, float* Cout,
                   const int64_t* c_m, const int64_t* c_n, float alpha, float beta, char* ws,
                   cudaStream_t s) {
-  const bool x3 = p->prec == TCCG_PREC_BF16X3;
+  const bool x3 = p->prec == TCCG_PREC_BF16X3, x6 = p->f32x6;
   TcArgs a = tc_args(p, Cout, c_m, c_n, alpha, beta, ws);
-  CUtensorMap tmA, tmB;
+  CUtensorMap tmA, tmB, tmAl, tmBl;
   int rc;
   bool packed = false;  // the packing kernel is the last launch on s
   const bool pair = p->tune.pair != 0;
@@ -1883,7 +1989,7 @@ static int run_tc(const tccg_plan* p, const void* GA, const void* GB, float* Cou
     void* Ap = ws + p->off_a;
     void* Bp = ws + p->off_b;
     PackArgs pa;
-    const int64_t kcover = x3 ? round_up(p->K, 32) : p->Kc;
+    const int64_t kcover = x3 || x6 ? round_up(p->K, 32) : p->Kc;
     const size_t es = p->dtype == TCCG_BF16 ? 2 : 4;
     pa.op[0] = with_kread(with_visit(pack_op(GA, p->t_a_m, p->t_a_k, p->M, p->K, p->M, kcover, Ap,
                                              p->Kc, p->read_k_fast_a), p->t_a_vsrc, p->t_a_vdst),
@@ -1891,16 +1997,25 @@ static int run_tc(const tccg_plan* p, const void* GA, const void* GB, float* Cou
     pa.op[1] = with_kread(with_visit(pack_op(GB, p->t_b_n, p->t_b_k, p->N, p->K, p->N, kcover, Bp,
                                              p->Kc, p->read_k_fast_b), p->t_b_vsrc, p->t_b_vdst),
                           p->ks_b, p->kb_b, p->kbq_b, es);
-    if (x3)
+    if (x6) {
+      uint32_t* range = reinterpret_cast<uint32_t*>(ws + p->off_range);
+      CUDA_TRY(cudaMemsetAsync(range, 0xff, 4 * sizeof(uint32_t), s));
+      pa.op[0].range = range;
+      pa.op[1].range = range + 2;
+      rc = launch_pack<float, __nv_bfloat16, PACK_K_F32X6>(pa, s, &packed);
+    } else if (x3)
       rc = launch_pack<float, __nv_bfloat16, PACK_K_BF16X3>(pa, s, &packed);
     else if (p->dtype == TCCG_BF16)
       rc = launch_pack<__nv_bfloat16, __nv_bfloat16, PACK_K_BF16>(pa, s, &packed);
     else
       rc = launch_pack<float, __nv_bfloat16, PACK_K_BF16>(pa, s, &packed);
     if (rc) return rc;
-    rc = encode_kmajor(&tmA, Ap, p->M, p->Kc, 128);
-    if (rc) return rc;
-    rc = encode_kmajor(&tmB, Bp, p->N, p->Kc, pair ? p->bn / 2 : p->bn);
+    if (x6) {
+      rc = encode_f32x6(p, Ap, Bp, &tmA, &tmB, &tmAl, &tmBl);
+    } else {
+      rc = encode_kmajor(&tmA, Ap, p->M, p->Kc, 128);
+      if (!rc) rc = encode_kmajor(&tmB, Bp, p->N, p->Kc, pair ? p->bn / 2 : p->bn);
+    }
     if (rc) return rc;
   }
   mark(1, 0, s);
@@ -1914,14 +2029,23 @@ static int run_tc(const tccg_plan* p, const void* GA, const void* GB, float* Cou
     take_injection(a);
     with_tc_variant(p->tcv, [&](auto k) {
       using K = decltype(k);
-      launch_after(packed, p, K::single, dim3((unsigned)p->grid), dim3(K::Cfg::NUM_THREADS),
-                   K::Cfg::SMEM_BYTES, s, tmA, tmB, a);
+      const bool after = packed && tc_dependent(p);
+      const dim3 grid((unsigned)p->grid), block(K::Cfg::NUM_THREADS);
+      if constexpr (K::Cfg::X6)
+        launch_after(after, p, K::single, grid, block, K::Cfg::SMEM_BYTES, s, tmA, tmB, tmAl, tmBl, a);
+      else
+        launch_after(after, p, K::single, grid, block, K::Cfg::SMEM_BYTES, s, tmA, tmB, a);
     });
   }
   mark(1, 1, s);
   rc = launch_check(p->gather ? "gett_tc (gather)" : "gett_tc");
   if (rc) return rc;
-  return tc_reduce(p, a, Cout, c_m, c_n, alpha, beta, s);
+  rc = tc_reduce(p, a, Cout, c_m, c_n, alpha, beta, s);
+  if (rc || !x6) return rc;
+  const F32FallbackItem it = f32_fallback_item(p, GA, GB, Cout, a.range, alpha, beta);
+  launch_after(true, p, f32_fallback_kernel, dim3((unsigned)std::min<int64_t>(it.tiles, 2 * p->num_sms)),
+               dim3(256), simt_smem_bytes<float>(), s, it);
+  return launch_check("f32_fallback");
 }
 
 // Kernel arguments of a skinny plan for one call (P / Q by the narrow side).
@@ -2292,6 +2416,11 @@ struct tccg_group {
   int32_t n_tc = 0;
   PackJob* d_tc_jobs = nullptr;
   int32_t* tc_status = nullptr;
+  // FP32 items on the tensor cores: their CUDA-core forms (one per item of
+  // the TCV_F32X6 lanes, wave after wave) and range words (four per item)
+  F32FallbackItem* d_fb = nullptr;
+  uint32_t* d_range = nullptr;
+  int32_t n_x6 = 0;
   // k-split reductions: ReduceJob<T>[] (same T as the CUDA-core lane)
   void* d_reduce = nullptr;
   // skinny lane (FP32 operands): the items' contractions and the k-split
@@ -2327,6 +2456,7 @@ struct tccg_group {
     int64_t lane_tiles[TCV_COUNT] = {};
     int32_t tcj0 = 0, ntcj = 0;  // pack jobs of the packed-operand lanes (two per item)
     int64_t simt_tiles = 0, simt_pack_ctas = 0, tc_pack_ctas = 0, red_ctas = 0;
+    int32_t fb0 = 0;  // the TCV_F32X6 lane's items are [fb0, fb0 + nlane) of d_fb / d_range
     // skinny lanes, one per rows-per-thread class (rs / 4 - 1: 4, 8, 12): items
     // [sk0[c], sk0[c] + nsk[c]) of d_sk with sk_jobs[c] jobs; reductions
     int32_t sk0[3] = {}, nsk[3] = {}, skr0 = 0, nskr = 0;
@@ -2353,7 +2483,7 @@ static constexpr size_t kGroupWaveBytes = size_t(TCCG_GROUP_WAVE_MB) << 20;
 static void group_free(tccg_group* g) {
   if (!g) return;
   void* ps[] = {g->d_simt, g->d_simt_jobs, g->d_tc, g->d_tc_jobs, g->d_reduce, g->d_begin,
-                g->d_sk, g->d_skr, g->d_sktc};
+                g->d_sk, g->d_skr, g->d_sktc, g->d_fb, g->d_range};
   for (void* q : ps)
     if (q) cudaFree(q);
   for (cudaStream_t q : g->side)
@@ -2396,6 +2526,7 @@ extern "C" int tccg_group_create(const tccg_plan* const* plans, int32_t count, t
     } else {
       if (!g->tc_status) g->tc_status = p->d_status;
       ++g->n_tc;
+      g->n_x6 += p->f32x6;
     }
   }
   // waves, largest workspaces first (next fit under kGroupWaveBytes)
@@ -2444,6 +2575,10 @@ extern "C" int tccg_group_create(const tccg_plan* const* plans, int32_t count, t
   const int32_t n_tcj = 2 * g->n_tc + g->n_sktc;
   if (e == cudaSuccess && n_tcj) e = cudaMalloc((void**)&g->d_tc_jobs, sizeof(PackJob) * n_tcj);
   if (e == cudaSuccess && g->n_tc) e = cudaMalloc((void**)&g->d_tc, sizeof(TcGroupItem) * g->n_tc);
+  if (e == cudaSuccess && g->n_x6) {
+    e = cudaMalloc((void**)&g->d_fb, sizeof(F32FallbackItem) * g->n_x6);
+    if (e == cudaSuccess) e = cudaMalloc((void**)&g->d_range, 4 * sizeof(uint32_t) * g->n_x6);
+  }
   if (e == cudaSuccess && g->n_sk) e = cudaMalloc((void**)&g->d_sk, sizeof(SkinnyItem) * g->n_sk);
   if (e == cudaSuccess && g->n_sktc)
     e = cudaMalloc((void**)&g->d_sktc, sizeof(SkinnyTcItem) * g->n_sktc);
@@ -2619,9 +2754,11 @@ static int bind_simt(tccg_group* g, tccg_group::Wave& wv, const void* const* A,
 static int bind_tc(tccg_group* g, tccg_group::Wave& wv, const void* const* A, const void* const* B,
                    void* const* C, const double* alpha, const double* beta, char* ws,
                    std::vector<TcGroupItem>& items, std::vector<PackJob>& jobs,
-                   std::vector<ReduceJob<float>>& red, int64_t& rctas) {
+                   std::vector<ReduceJob<float>>& red, int64_t& rctas,
+                   std::vector<F32FallbackItem>& fallback) {
   int64_t pctas = 0;
   wv.tcj0 = (int32_t)jobs.size();
+  wv.fb0 = (int32_t)fallback.size();
   for (int lane = 0; lane < TCV_COUNT; ++lane) {  // one lane per kernel variant
     const bool gather = lane == TCV_X3_GATHER;
     wv.lane0[lane] = (int32_t)items.size();
@@ -2643,7 +2780,8 @@ static int bind_tc(tccg_group* g, tccg_group::Wave& wv, const void* const* A, co
       if (gather) {
         set_gather(it.args, p, GA, GB);
       } else {
-        const int64_t kcover = p->prec == TCCG_PREC_BF16X3 ? round_up(p->K, 32) : p->Kc;
+        const int64_t kcover =
+            p->prec == TCCG_PREC_BF16X3 || p->f32x6 ? round_up(p->K, 32) : p->Kc;
         const size_t es = p->dtype == TCCG_BF16 ? 2 : 4;
         add_pack_jobs(jobs, pctas,
                       with_kread(with_visit(pack_op(GA, p->t_a_m, p->t_a_k, p->M, p->K, p->M, kcover,
@@ -2653,8 +2791,19 @@ static int bind_tc(tccg_group* g, tccg_group::Wave& wv, const void* const* A, co
                                                     w + p->off_b, p->Kc, p->read_k_fast_b),
                                             p->t_b_vsrc, p->t_b_vdst), p->ks_b, p->kb_b, p->kbq_b, es),
                       pack_k_tile<PACK_K_BF16>(), true);
-        int rc = encode_kmajor(&it.tmA, w + p->off_a, p->M, p->Kc, 128);
-        if (!rc) rc = encode_kmajor(&it.tmB, w + p->off_b, p->N, p->Kc, p->bn);
+        int rc;
+        if (p->f32x6) {
+          uint32_t* range = g->d_range + 4 * fallback.size();
+          it.args.range = range;
+          jobs[jobs.size() - 2].op.range = range;
+          jobs[jobs.size() - 1].op.range = range + 2;
+          fallback.push_back(f32_fallback_item(p, GA, GB, static_cast<float*>(C[i]), range,
+                                               (float)alpha[i], (float)beta[i]));
+          rc = encode_f32x6(p, w + p->off_a, w + p->off_b, &it.tmA, &it.tmB, &it.tmAl, &it.tmBl);
+        } else {
+          rc = encode_kmajor(&it.tmA, w + p->off_a, p->M, p->Kc, 128);
+          if (!rc) rc = encode_kmajor(&it.tmB, w + p->off_b, p->N, p->Kc, p->bn);
+        }
         if (rc) return rc;
       }
       it.tile_begin = tile;
@@ -2800,6 +2949,7 @@ extern "C" int tccg_group_bind(tccg_group* g, const void* const* A, const void* 
     std::vector<TcGroupItem> titems;
     std::vector<SkinnyItem> kitems, kred;
     std::vector<SkinnyTcItem> ktc;
+    std::vector<F32FallbackItem> fitems;
     int r = TCCG_OK;
     for (tccg_group::Wave& wv : g->waves) {
       int64_t rctas = 0;
@@ -2807,7 +2957,7 @@ extern "C" int tccg_group_bind(tccg_group* g, const void* const* A, const void* 
       r = bind_simt<T>(g, wv, A, B, C, alpha, beta, w, simt_items, sjobs, red, rctas);
       if (r) return r;
       if constexpr (sizeof(T) == 4) {
-        r = bind_tc(g, wv, A, B, C, alpha, beta, w, titems, tjobs, red, rctas);
+        r = bind_tc(g, wv, A, B, C, alpha, beta, w, titems, tjobs, red, rctas, fitems);
         if (r) return r;
         bind_skinny(g, wv, A, B, C, alpha, beta, w, kitems, kred);
         r = bind_sktc(g, wv, A, B, C, alpha, beta, w, ktc, tjobs, kred);
@@ -2825,6 +2975,9 @@ extern "C" int tccg_group_bind(tccg_group* g, const void* const* A, const void* 
     }
     if (!titems.empty())
       CUDA_TRY(cudaMemcpy(g->d_tc, titems.data(), sizeof(TcGroupItem) * titems.size(),
+                          cudaMemcpyHostToDevice));
+    if (!fitems.empty())
+      CUDA_TRY(cudaMemcpy(g->d_fb, fitems.data(), sizeof(F32FallbackItem) * fitems.size(),
                           cudaMemcpyHostToDevice));
     if (!tjobs.empty())
       CUDA_TRY(cudaMemcpy(g->d_tc_jobs, tjobs.data(), sizeof(PackJob) * tjobs.size(),
@@ -2938,9 +3091,14 @@ static int run_wave(const tccg_group* g, const tccg_group::Wave& wv, cudaStream_
   const bool x3 = g->prec == TCCG_PREC_BF16X3;
   const PackJob* tjobs = g->d_tc_jobs + wv.tcj0;
   const int64_t* tb = g->b_tc_jobs + wv.tcj0;
+  const int n_x6 = wv.nlane[TCV_F32X6];
+  if (n_x6 > 0)
+    CUDA_TRY(cudaMemsetAsync(g->d_range + 4 * wv.fb0, 0xff, 4 * sizeof(uint32_t) * n_x6, s));
   if (wv.tc_pack_ctas > 0) {
     const dim3 pg((unsigned)wv.tc_pack_ctas);
-    if (x3)
+    if (g->prec == TCCG_PREC_FP32)
+      pack_group_kernel<float, __nv_bfloat16, PACK_K_F32X6><<<pg, blk, 0, s>>>(tjobs, tb, tj);
+    else if (x3)
       pack_group_kernel<float, __nv_bfloat16, PACK_K_BF16X3><<<pg, blk, 0, s>>>(tjobs, tb, tj);
     else if (g->dtype == TCCG_BF16)
       pack_group_kernel<__nv_bfloat16, __nv_bfloat16, PACK_K_BF16><<<pg, blk, 0, s>>>(tjobs, tb, tj);
@@ -2961,6 +3119,11 @@ static int run_wave(const tccg_group* g, const tccg_group::Wave& wv, cudaStream_
       K::group<<<grid, K::Cfg::NUM_THREADS, K::Cfg::SMEM_BYTES, s>>>(tg, g->tc_status);
     });
     if ((rc = launch_check("gett_tc_group"))) return rc;
+  }
+  if (n_x6 > 0) {
+    f32_fallback_group_kernel<<<2 * (unsigned)g->num_sms, 256, simt_smem_bytes<float>(), s>>>(
+        g->d_fb + wv.fb0, n_x6);
+    if ((rc = launch_check("f32_fallback_group"))) return rc;
   }
   if constexpr (sizeof(T) == 4) {
     if (wv.nsktc > 0) {
