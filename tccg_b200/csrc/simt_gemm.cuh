@@ -71,16 +71,20 @@ struct SimtCfg<float, SIMT_NARROW_M> {
   static constexpr int LDA = BM + 4, LDB = BN + 4;
 };
 
+// FP64: mma.sync m16n8k8 (simt_fma_ktile), warp tiles of 32 x 32. The stage
+// rows are padded by 32 bytes: a fragment load's 4 k x 4 (half warp) rows
+// then cover all banks. Epilogue rows padded by 64 bytes: the 16-byte
+// accumulator pairs of 2 columns x 4 lanes do.
 template <>
 struct SimtCfg<double, SIMT_SQUARE> {
   static constexpr int BM = 128, BN = 64, BK = 8;
-  static constexpr int WARPS_M = 2, WARPS_N = 4;
-  static constexpr int TMG = 2, TNG = 1;
+  static constexpr int WARPS_M = 4, WARPS_N = 2;
+  static constexpr int TMG = 2, TNG = 1;  // 8 m x 4 n per thread
   static constexpr int STAGES = 4;
   static constexpr int EPN = 64;
-  static constexpr int PAD = 2;
+  static constexpr int PAD = 8;
   static constexpr int MIN_BLOCKS = 2;
-  static constexpr int LDA = BM, LDB = BN;
+  static constexpr int LDA = BM + 4, LDB = BN + 4;
 };
 
 template <typename T>
@@ -147,64 +151,126 @@ __device__ __forceinline__ Vec4<T> lds4(const T* p) {
   return r;
 }
 
-// Thread fragment geometry of the 256-thread CUDA-core tiles: warps WARPS_M x
-// WARPS_N, lanes 8 (m) x 4 (n), each thread TMG groups of 4 m and TNG groups of
-// 4 n. A fragment: per group g of 32 m, a thread owns 4 m. FP32: m = 4 lm + i,
-// one 16-byte load. FP64: two 16-byte loads at m = 2 lm + {0,1} and
-// 16 + 2 lm + {0,1}, so the 8 lane groups of each load read 128 contiguous
-// bytes (4 consecutive doubles per lane would put lanes lm and lm + 4 on
-// the same banks: a 2-way conflict on every A load).
-template <typename T, int S = SIMT_SQUARE>
+// Thread fragment geometry of the 256-thread tiles.
+// FMA fragments (FP32, and FP64 in the short-K kernel): lanes 8 (m) x 4 (n),
+// a thread has groups of 4 m of every 32 and groups of 4 n of every 16. FP32:
+// warps WARPS_M x WARPS_N, m = 4 lm + i, one 16-byte load. FP64: warps 2 x 4,
+// two 16-byte loads at m = 2 lm + {0, 1} and 16 + 2 lm + {0, 1}, so the 8 lane
+// groups of each load read 128 contiguous bytes (4 consecutive doubles per
+// lane would put lanes lm and lm + 4 on the same banks).
+// MMA fragments (FP64): warp tiles of 32 x 32, computed as (n x k) (k x m)
+// products of mma m16n8k8: a thread holds, per 16 n and 8 m, n = lane / 4 +
+// {0, 8} and the pair m = 2 (lane % 4) + {0, 1} (consecutive in C's staged
+// columns).
+template <typename T, int S = SIMT_SQUARE, bool MMA = sizeof(T) == 8>
 struct SimtFrag {
   using Cfg = SimtCfg<T, S>;
   static constexpr int TM = Cfg::TMG * 4, TN = Cfg::TNG * 4;
   static constexpr bool PAIRS = sizeof(T) == 8;
-  int a_off, b_off;
+  // panel row strides: the FP64 FMA fragments read dense panels
+  static constexpr int LDA = PAIRS && !MMA ? Cfg::BM : Cfg::LDA, LDB = PAIRS && !MMA ? Cfg::BN : Cfg::LDB;
+  int a_off, b_off;  // this thread's first element of the A and B panels
+  int m0, n0;        // its first m and n
   __device__ __forceinline__ explicit SimtFrag(int tid) {
     const int warp = tid >> 5, lane = tid & 31;
-    const int wm = warp % Cfg::WARPS_M, wn = warp / Cfg::WARPS_M;
-    a_off = wm * (Cfg::TMG * 32) + (lane & 7) * (PAIRS ? 2 : 4);
-    b_off = wn * (Cfg::TNG * 16) + (lane >> 3) * 4;
+    if constexpr (MMA) {
+      static_assert(Cfg::WARPS_M * 32 == Cfg::BM && Cfg::WARPS_N * 32 == Cfg::BN, "32 x 32 per warp");
+      const int wm = warp % Cfg::WARPS_M, wn = warp / Cfg::WARPS_M;
+      a_off = (lane & 3) * LDA + wm * 32 + (lane >> 2);
+      b_off = (lane & 3) * LDB + wn * 32 + (lane >> 2);
+      m0 = wm * 32 + 2 * (lane & 3);
+      n0 = wn * 32 + (lane >> 2);
+    } else {
+      constexpr int WARPS_M = PAIRS ? 2 : Cfg::WARPS_M, WARPS_N = PAIRS ? 4 : Cfg::WARPS_N;
+      static_assert(WARPS_M * Cfg::TMG * 32 == Cfg::BM && WARPS_N * Cfg::TNG * 16 == Cfg::BN,
+                    "warps cover the tile");
+      const int wm = warp % WARPS_M, wn = warp / WARPS_M;
+      a_off = m0 = wm * (Cfg::TMG * 32) + (lane & 7) * (PAIRS ? 2 : 4);
+      b_off = n0 = wn * (Cfg::TNG * 16) + (lane >> 3) * 4;
+    }
   }
   // tile-local m of accumulator row i and n of accumulator column j
   __device__ __forceinline__ int m(int i) const {
-    return PAIRS ? a_off + (i / 4) * 32 + ((i % 4) / 2) * 16 + (i % 2) : a_off + (i / 4) * 32 + (i % 4);
+    return MMA     ? m0 + (i / 2) * 8 + (i % 2)
+           : PAIRS ? m0 + (i / 4) * 32 + ((i % 4) / 2) * 16 + (i % 2)
+                   : m0 + (i / 4) * 32 + (i % 4);
   }
-  __device__ __forceinline__ int n(int j) const { return b_off + (j / 4) * 16 + (j % 4); }
+  __device__ __forceinline__ int n(int j) const {
+    return MMA ? n0 + (j / 2) * 16 + (j % 2) * 8 : n0 + (j / 4) * 16 + (j % 4);
+  }
 };
+
+// D (16 x 8) += A (16 x 8) B (8 x 8) in FP64. Lane l holds A(l / 4 + {0, 8},
+// l % 4 + {0, 4}) as a0 a1 (k), a2 a3 (k + 4); B(l % 4 + {0, 4}, l / 4); D rows
+// l / 4 (c0 c1) and l / 4 + 8 (c2 c3), columns 2 (l % 4) + {0, 1}.
+__device__ __forceinline__ void mma_f64(double& c0, double& c1, double& c2, double& c3, double a0,
+                                        double a1, double a2, double a3, double b0, double b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%0,%1,%2,%3};"
+      : "+d"(c0), "+d"(c1), "+d"(c2), "+d"(c3)
+      : "d"(a0), "d"(a1), "d"(a2), "d"(a3), "d"(b0), "d"(b1));
+}
 
 // One k-tile: acc += A[k][m] * B[k][n] over the BK rows of the stage's
 // A [BK][LDA] and B [BK][LDB] panels, k in increasing order.
-template <typename T, int S = SIMT_SQUARE>
-__device__ __forceinline__ void simt_fma_ktile(const T* as, const T* bs, int a_off, int b_off,
-                                               T (&acc)[SimtFrag<T, S>::TM][SimtFrag<T, S>::TN]) {
+// FP64 bound: the fp64 pipe. Fragments of DFMA (8 x 4 per thread) read 12
+// doubles of shared memory per 32 FMAs -- 79 % of the shared-memory wavefronts
+// at 64 % of the pipe; the mma fragments read 16 per 256 FMAs of a lane:
+// 3825 x 4056 x 3080 in 3.04 ms against 4.25 (31.4 and 22.5 TFLOP/s). A K
+// that ends after two steps is bound by C and keeps DFMA, whose short phases
+// cost less (96^4 x 16 in the short-K kernel: 217 us, 238 with mma).
+template <typename T, int S = SIMT_SQUARE, bool MMA = sizeof(T) == 8>
+__device__ __forceinline__ void simt_fma_ktile(
+    const T* as, const T* bs, int a_off, int b_off,
+    T (&acc)[SimtFrag<T, S, MMA>::TM][SimtFrag<T, S, MMA>::TN]) {
   using Cfg = SimtCfg<T, S>;
+  using Frag = SimtFrag<T, S, MMA>;
   constexpr int BK = Cfg::BK;
-  constexpr int TM = SimtFrag<T, S>::TM, TN = SimtFrag<T, S>::TN;
+  constexpr int TM = Frag::TM, TN = Frag::TN;
+  if constexpr (MMA) {
+    static_assert(BK == 8 && TM == 8 && TN == 4, "one mma k step per tile");
+    double a[4][2], b[2][4];  // [8 m][k, k + 4], [16 n][(n, k), (n + 8, k), (n, k + 4), (n + 8, k + 4)]
 #pragma unroll
-  for (int k = 0; k < BK; ++k) {
-    T av[TM], bv[TN];
+    for (int mt = 0; mt < 4; ++mt)
 #pragma unroll
-    for (int g = 0; g < Cfg::TMG; ++g) {
-      Vec4<T> x;
-      if constexpr (SimtFrag<T, S>::PAIRS) {
-        const double2 lo = *reinterpret_cast<const double2*>(as + k * Cfg::LDA + a_off + g * 32);
-        const double2 hi = *reinterpret_cast<const double2*>(as + k * Cfg::LDA + a_off + g * 32 + 16);
-        x.v[0] = lo.x; x.v[1] = lo.y; x.v[2] = hi.x; x.v[3] = hi.y;
-      } else {
-        x = lds4<T>(as + k * Cfg::LDA + a_off + g * 32);
+      for (int h = 0; h < 2; ++h) a[mt][h] = as[a_off + 4 * h * Cfg::LDA + 8 * mt];
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int h = 0; h < 4; ++h) b[nt][h] = bs[b_off + 4 * (h / 2) * Cfg::LDB + 16 * nt + 8 * (h % 2)];
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int mt = 0; mt < 4; ++mt)
+        mma_f64(acc[2 * mt][2 * nt], acc[2 * mt + 1][2 * nt], acc[2 * mt][2 * nt + 1],
+                acc[2 * mt + 1][2 * nt + 1], b[nt][0], b[nt][1], b[nt][2], b[nt][3], a[mt][0], a[mt][1]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < BK; ++k) {
+      T av[TM], bv[TN];
+#pragma unroll
+      for (int g = 0; g < Cfg::TMG; ++g) {
+        Vec4<T> x;
+        if constexpr (Frag::PAIRS) {
+          const double2 lo = *reinterpret_cast<const double2*>(as + k * Frag::LDA + a_off + g * 32);
+          const double2 hi = *reinterpret_cast<const double2*>(as + k * Frag::LDA + a_off + g * 32 + 16);
+          x.v[0] = lo.x; x.v[1] = lo.y; x.v[2] = hi.x; x.v[3] = hi.y;
+        } else {
+          x = lds4<T>(as + k * Frag::LDA + a_off + g * 32);
+        }
+        av[g * 4 + 0] = x.v[0]; av[g * 4 + 1] = x.v[1]; av[g * 4 + 2] = x.v[2]; av[g * 4 + 3] = x.v[3];
       }
-      av[g * 4 + 0] = x.v[0]; av[g * 4 + 1] = x.v[1]; av[g * 4 + 2] = x.v[2]; av[g * 4 + 3] = x.v[3];
+#pragma unroll
+      for (int g = 0; g < Cfg::TNG; ++g) {
+        const Vec4<T> x = lds4<T>(bs + k * Frag::LDB + b_off + g * 16);
+        bv[g * 4 + 0] = x.v[0]; bv[g * 4 + 1] = x.v[1]; bv[g * 4 + 2] = x.v[2]; bv[g * 4 + 3] = x.v[3];
+      }
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = fma(av[i], bv[j], acc[i][j]);
     }
-#pragma unroll
-    for (int g = 0; g < Cfg::TNG; ++g) {
-      Vec4<T> x = lds4<T>(bs + k * Cfg::LDB + b_off + g * 16);
-      bv[g * 4 + 0] = x.v[0]; bv[g * 4 + 1] = x.v[1]; bv[g * 4 + 2] = x.v[2]; bv[g * 4 + 3] = x.v[3];
-    }
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-      for (int j = 0; j < TN; ++j) acc[i][j] = fma(av[i], bv[j], acc[i][j]);
   }
 }
 
@@ -224,8 +290,6 @@ __device__ __forceinline__ void simt_gett_tile(const SimtArgs<T>& a, int bx, int
   constexpr int VEC = 16 / sizeof(T);                 // elements per 16-byte chunk
   constexpr int A_CHUNKS = BK * BM / VEC, B_CHUNKS = BK * BN / VEC;
   constexpr int A_ROW_CHUNKS = BM / VEC, B_ROW_CHUNKS = BN / VEC;
-  static_assert(Cfg::WARPS_M * Cfg::TMG * 32 == BM, "tile M");
-  static_assert(Cfg::WARPS_N * Cfg::TNG * 16 == BN, "tile N");
 
   extern __shared__ __align__(16) uint8_t smem_raw[];
   T* As = reinterpret_cast<T*>(smem_raw);              // [STAGES][BK][LDA]
@@ -445,8 +509,14 @@ __device__ __forceinline__ void simt_gett_tile(const SimtArgs<T>& a, int bx, int
     for (int j = 0; j < TN; ++j) {
       const int nl = nloc(j) - p * EPN;
       if (nl >= 0 && nl < EPN) {
+        if constexpr (sizeof(T) == 8) {
 #pragma unroll
-        for (int i = 0; i < TM; ++i) Cs[nl * LDC + mloc(i)] = acc[i][j];
+          for (int i = 0; i < TM; i += 2)
+            *reinterpret_cast<double2*>(Cs + nl * LDC + mloc(i)) = make_double2(acc[i][j], acc[i + 1][j]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < TM; ++i) Cs[nl * LDC + mloc(i)] = acc[i][j];
+        }
       }
     }
     if (tid < EPN) {
@@ -625,7 +695,8 @@ __global__ void __launch_bounds__(256, 2)
   constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK;
   constexpr int VEC = 16 / sizeof(T);  // elements per 16-byte access
   constexpr int QPC = BM / 4, CPI = 256 / QPC, ITER = BN / CPI;
-  constexpr int TM = SimtFrag<T>::TM, TN = SimtFrag<T>::TN;
+  using Frag = SimtFrag<T, SIMT_SQUARE, false>;
+  constexpr int TM = Frag::TM, TN = Frag::TN;
   constexpr int64_t NONE = INT64_MIN;  // offsets may be negative (negative strides)
   static_assert(BN <= 256, "one column offset per thread");
   extern __shared__ __align__(16) uint8_t smem_raw[];
@@ -637,7 +708,7 @@ __global__ void __launch_bounds__(256, 2)
   T* Bs = As + (size_t)SC::KP * BM;                                    // [KP][BN]
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + SC::USED - 16);
   const int tid = threadIdx.x;
-  const SimtFrag<T> frag(tid);
+  const Frag frag(tid);
   const int64_t m0 = (int64_t)blockIdx.x * BM, n0 = (int64_t)blockIdx.y * BN;
   const int kp = a.ktiles * BK;
   const T alpha = a.alpha, beta = a.beta;
@@ -711,7 +782,8 @@ __global__ void __launch_bounds__(256, 2)
 #pragma unroll
     for (int j = 0; j < TN; ++j) acc[i][j] = T(0);
   for (int kt = 0; kt < a.ktiles; ++kt)
-    simt_fma_ktile<T>(As + kt * BK * BM, Bs + kt * BK * BN, frag.a_off, frag.b_off, acc);
+    simt_fma_ktile<T, SIMT_SQUARE, false>(As + kt * BK * BM, Bs + kt * BK * BN, frag.a_off,
+                                          frag.b_off, acc);
   if constexpr (TMA) {
     if (read_c && !mbar_wait(bar, 0)) {
       record_error(a.status, 4);
