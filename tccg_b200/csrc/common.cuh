@@ -105,6 +105,16 @@ __device__ __forceinline__ void tma_store_2d(const void* tmap, const void* smem_
                "r"(smem_u32(smem_src)), "r"(c0), "r"(c1)
                : "memory");
 }
+// 1-D bulk copy global -> shared, completing on `bar`; both addresses 16-byte
+// aligned, bytes a multiple of 16
+__device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gsrc, uint32_t bytes,
+                                             uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+          smem_u32(smem_dst)),
+      "l"(reinterpret_cast<uint64_t>(gsrc)), "r"(bytes), "r"(smem_u32(bar))
+      : "memory");
+}
 // 1-D bulk copy shared -> global (bulk-group completion); both addresses
 // 16-byte aligned, bytes a multiple of 16
 __device__ __forceinline__ void bulk_store_1d(void* gdst, const void* smem_src, uint32_t bytes) {
@@ -273,6 +283,24 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
          | (1u << 10)                       // B format: BF16
          | ((uint32_t)(N >> 3) << 17)       // N / 8
          | ((uint32_t)(M >> 4) << 24);      // M / 16
+}
+
+// ---- packed FP32 pairs -------------------------------------------------------
+// Two FP32 values in one 64-bit register pair: x = low, y = high word.
+// fma_x2 is fma.rn.f32x2: both lanes rounded as fmaf rounds one, in one
+// instruction.
+__device__ __forceinline__ uint64_t f32x2(float x, float y) {
+  uint64_t v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(x), "f"(y));
+  return v;
+}
+__device__ __forceinline__ float f32x2_lo(uint64_t v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float f32x2_hi(uint64_t v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ uint64_t f32x2_swap(uint64_t v) { return f32x2(f32x2_hi(v), f32x2_lo(v)); }
+__device__ __forceinline__ uint64_t fma_x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
 }
 
 // ---- split-BF16x3 representation ---------------------------------------------

@@ -117,8 +117,14 @@ struct SimtArgs {
   // C layout (as TcArgs::crun): e0 in [2, 31] = C's stride-one index is the
   // first M mode, of extent e0, directly followed in C by the first N mode;
   // the epilogue then stores runs of e0 m by 32 / e0 columns per warp
-  // instruction (consecutive addresses); 0 = quads along m
+  // instruction (consecutive addresses); 0 = quads along m, or lanes along m
   int32_t crun;
+  // every quad m % 4 == 0 .. + 3 of C is 4 consecutive, aligned elements in
+  // every column: the epilogue moves 4 m per thread as a vector. Otherwise
+  // its lanes run along m, one element each: a quad of scattered alignment
+  // would write each 32-byte sector of C in 4 instructions of 4 bytes a lane
+  int32_t c_vec;
+  int64_t ldc;  // > 0: C(m, n) = C[m + ldc n] (short-K kernel, SHORTK_BULK)
 };
 
 template <typename T, int S = SIMT_SQUARE>
@@ -212,6 +218,39 @@ __device__ __forceinline__ void mma_f64(double& c0, double& c1, double& c2, doub
       : "d"(a0), "d"(a1), "d"(a2), "d"(a3), "d"(b0), "d"(b1));
 }
 
+// A thread's TM x TN sums.
+// FP32: pairs for fma.rn.f32x2. A pair of m times a pair of n gives the two
+// "diagonal" sums, times the swapped pair of n the other two, so no operand
+// has to be duplicated: v[ip][j] = (sum of (2 ip, j), sum of (2 ip + 1, j ^ 1)).
+// The FMA pipe takes a pair in two cycles: half the issue slots of the loop
+// are left for its shared-memory loads and the swaps.
+template <typename T, int S = SIMT_SQUARE, bool MMA = sizeof(T) == 8>
+struct SimtAcc {
+  static constexpr int TM = SimtFrag<T, S, MMA>::TM, TN = SimtFrag<T, S, MMA>::TN;
+  T v[TM][TN];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) v[i][j] = T(0);
+  }
+  __device__ __forceinline__ T get(int i, int j) const { return v[i][j]; }
+};
+template <int S>
+struct SimtAcc<float, S, false> {
+  static constexpr int TM = SimtFrag<float, S, false>::TM, TN = SimtFrag<float, S, false>::TN;
+  uint64_t v[TM / 2][TN];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int i = 0; i < TM / 2; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) v[i][j] = 0;
+  }
+  __device__ __forceinline__ float get(int i, int j) const {
+    return i % 2 == 0 ? f32x2_lo(v[i / 2][j]) : f32x2_hi(v[i / 2][j ^ 1]);
+  }
+};
+
 // One k-tile: acc += A[k][m] * B[k][n] over the BK rows of the stage's
 // A [BK][LDA] and B [BK][LDB] panels, k in increasing order.
 // FP64 bound: the fp64 pipe. Fragments of DFMA (8 x 4 per thread) read 12
@@ -220,15 +259,40 @@ __device__ __forceinline__ void mma_f64(double& c0, double& c1, double& c2, doub
 // 3825 x 4056 x 3080 in 3.04 ms against 4.25 (31.4 and 22.5 TFLOP/s). A K
 // that ends after two steps is bound by C and keeps DFMA, whose short phases
 // cost less (96^4 x 16 in the short-K kernel: 217 us, 238 with mma).
-template <typename T, int S = SIMT_SQUARE, bool MMA = sizeof(T) == 8>
+template <typename T, int S = SIMT_SQUARE, bool MMA = sizeof(T) == 8, int BK = SimtCfg<T, S>::BK>
 __device__ __forceinline__ void simt_fma_ktile(
-    const T* as, const T* bs, int a_off, int b_off,
-    T (&acc)[SimtFrag<T, S, MMA>::TM][SimtFrag<T, S, MMA>::TN]) {
+    const T* as, const T* bs, int a_off, int b_off, SimtAcc<T, S, MMA>& acc_) {
   using Cfg = SimtCfg<T, S>;
   using Frag = SimtFrag<T, S, MMA>;
-  constexpr int BK = Cfg::BK;
   constexpr int TM = Frag::TM, TN = Frag::TN;
-  if constexpr (MMA) {
+  auto& acc = acc_.v;
+  if constexpr (sizeof(T) == 4) {
+#pragma unroll
+    for (int k = 0; k < BK; ++k) {
+      uint64_t av[TM / 2], bv[TN / 2];  // pairs of m, pairs of n
+#pragma unroll
+      for (int g = 0; g < Cfg::TMG; ++g) {
+        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(as + k * Frag::LDA + a_off + g * 32);
+        av[2 * g] = x.x;
+        av[2 * g + 1] = x.y;
+      }
+#pragma unroll
+      for (int g = 0; g < Cfg::TNG; ++g) {
+        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(bs + k * Frag::LDB + b_off + g * 16);
+        bv[2 * g] = x.x;
+        bv[2 * g + 1] = x.y;
+      }
+#pragma unroll
+      for (int j = 0; j < TN / 2; ++j) {
+        const uint64_t sw = f32x2_swap(bv[j]);
+#pragma unroll
+        for (int i = 0; i < TM / 2; ++i) {
+          acc[i][2 * j] = fma_x2(av[i], bv[j], acc[i][2 * j]);
+          acc[i][2 * j + 1] = fma_x2(av[i], sw, acc[i][2 * j + 1]);
+        }
+      }
+    }
+  } else if constexpr (MMA) {
     static_assert(BK == 8 && TM == 8 && TN == 4, "one mma k step per tile");
     double a[4][2], b[2][4];  // [8 m][k, k + 4], [16 n][(n, k), (n + 8, k), (n, k + 4), (n + 8, k + 4)]
 #pragma unroll
@@ -251,15 +315,9 @@ __device__ __forceinline__ void simt_fma_ktile(
       T av[TM], bv[TN];
 #pragma unroll
       for (int g = 0; g < Cfg::TMG; ++g) {
-        Vec4<T> x;
-        if constexpr (Frag::PAIRS) {
-          const double2 lo = *reinterpret_cast<const double2*>(as + k * Frag::LDA + a_off + g * 32);
-          const double2 hi = *reinterpret_cast<const double2*>(as + k * Frag::LDA + a_off + g * 32 + 16);
-          x.v[0] = lo.x; x.v[1] = lo.y; x.v[2] = hi.x; x.v[3] = hi.y;
-        } else {
-          x = lds4<T>(as + k * Frag::LDA + a_off + g * 32);
-        }
-        av[g * 4 + 0] = x.v[0]; av[g * 4 + 1] = x.v[1]; av[g * 4 + 2] = x.v[2]; av[g * 4 + 3] = x.v[3];
+        const double2 lo = *reinterpret_cast<const double2*>(as + k * Frag::LDA + a_off + g * 32);
+        const double2 hi = *reinterpret_cast<const double2*>(as + k * Frag::LDA + a_off + g * 32 + 16);
+        av[g * 4 + 0] = lo.x; av[g * 4 + 1] = lo.y; av[g * 4 + 2] = hi.x; av[g * 4 + 3] = hi.y;
       }
 #pragma unroll
       for (int g = 0; g < Cfg::TNG; ++g) {
@@ -432,11 +490,8 @@ __device__ __forceinline__ void simt_gett_tile(const SimtArgs<T>& a, int bx, int
     }
   };
 
-  T acc[TM][TN];
-#pragma unroll
-  for (int i = 0; i < TM; ++i)
-#pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = T(0);
+  SimtAcc<T, S> acc;
+  acc.zero();
 
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {
@@ -471,7 +526,7 @@ __device__ __forceinline__ void simt_gett_tile(const SimtArgs<T>& a, int bx, int
     for (int j = 0; j < TN; ++j) {
       const int64_t n = n0 + nloc(j);
 #pragma unroll
-      for (int i = 0; i < TM; ++i) P[n * a.Mp + m0 + mloc(i)] = acc[i][j];
+      for (int i = 0; i < TM; ++i) P[n * a.Mp + m0 + mloc(i)] = acc.get(i, j);
     }
     return;
   }
@@ -512,10 +567,10 @@ __device__ __forceinline__ void simt_gett_tile(const SimtArgs<T>& a, int bx, int
         if constexpr (sizeof(T) == 8) {
 #pragma unroll
           for (int i = 0; i < TM; i += 2)
-            *reinterpret_cast<double2*>(Cs + nl * LDC + mloc(i)) = make_double2(acc[i][j], acc[i + 1][j]);
+            *reinterpret_cast<double2*>(Cs + nl * LDC + mloc(i)) = make_double2(acc.get(i, j), acc.get(i + 1, j));
         } else {
 #pragma unroll
-          for (int i = 0; i < TM; ++i) Cs[nl * LDC + mloc(i)] = acc[i][j];
+          for (int i = 0; i < TM; ++i) Cs[nl * LDC + mloc(i)] = acc.get(i, j);
         }
       }
     }
@@ -561,6 +616,41 @@ __device__ __forceinline__ void simt_gett_tile(const SimtArgs<T>& a, int bx, int
           if (i >= L) {
             i -= L;
             ++j;
+          }
+        }
+      }
+    } else if (!a.c_vec) {
+      // lanes along m, one element per thread and column
+      constexpr int CS = 256 / BM, CH = 8;  // columns per step, steps whose C loads are in flight
+      const int ml = tid % BM, c0 = tid / BM;
+      const int64_t nleft = a.N - (n0 + p * EPN);
+      const int ncols = nleft < EPN ? (int)nleft : EPN;
+      if (m0 + ml < a.M) {
+        T* const Cb = a.C + a.c_m_off[m0 + ml];
+#pragma unroll 1
+        for (int c1 = c0; c1 < ncols; c1 += CS * CH) {
+          // shared memory is read before the stores (which may alias it as
+          // far as the compiler knows): one wait per CH columns
+          int64_t no[CH];
+          T v[CH], old[CH];
+#pragma unroll
+          for (int u = 0; u < CH; ++u) {
+            const int c = c1 + u * CS;
+            no[u] = c < ncols ? Cn[c] : 0;
+            v[u] = c < ncols ? Cs[c * LDC + ml] : T(0);
+          }
+          if (beta != T(0)) {
+#pragma unroll
+            for (int u = 0; u < CH; ++u)
+              old[u] = c1 + u * CS < ncols ? Cb[no[u]] : T(0);
+          }
+#pragma unroll
+          for (int u = 0; u < CH; ++u) {
+            if (c1 + u * CS < ncols) {
+              v[u] = alpha * v[u];
+              if (beta != T(0)) v[u] = fma(beta, old[u], v[u]);
+              Cb[no[u]] = v[u];
+            }
           }
         }
       }
@@ -664,20 +754,33 @@ __global__ void __launch_bounds__(256, 2)
 // the read runs under the FMA phase; the epilogue combines in shared memory
 // (alpha * acc + beta * C, 16-byte accesses at the fragment positions) and
 // the block leaves as one bulk store.
-//   TMA = true  (C is a 2-D matrix in the GETT view: unit M stride, one N
-//               stride): the C block comes in and goes out by TMA -- one
-//               instruction each, the store draining while the next CTA on
-//               the SM computes.
-//   TMA = false (any layout): cp.async per thread through the offset tables,
-//               stores from the threads (16-byte vectors where 4 consecutive
-//               m are contiguous and aligned in C).
+//   SHORTK_TMA  (C is a 2-D matrix in the GETT view: unit M stride, one N
+//               stride of 16-byte multiple): the C block comes in and goes
+//               out by TMA -- one instruction each, the store draining while
+//               the next CTA on the SM computes.
+//   SHORTK_BULK (FP32, a 2-D C whose columns start off 16-byte boundaries):
+//               one bulk copy per column each way. A column lies in shared
+//               memory at its global offset modulo 16 bytes; it comes in as
+//               the 16-byte-aligned range around it (where that is inside
+//               C) and leaves as the aligned range inside it, its up to 3 + 3
+//               edge elements by plain stores. In the combine step the 4 lanes
+//               that share a bank group take their 4 m in rotated order.
+//   SHORTK_ANY  (any layout): each thread has one m and every other column,
+//               cp.async in and stores out with lanes along m.
+// 6930 x 8585 x 19, FP32, beta = 1: 119 us; SHORTK_ANY 156 (bound by its
+// per-element instructions), the tile kernel with 4-element quads per thread
+// 181. HBM time of C in and out: 73 us; the FMA phase (its shared-memory loads
+// at 60 TFLOP/s) and the C traffic share the shared-memory path and add up.
+// The FMA loop stops at K rounded up to 4, not at the packed panel's end.
 // Two CTAs per SM. Same k order and epilogue arithmetic as simt_gett_tile:
 // the results are bitwise equal.
 template <typename T>
 struct SimtShortKCfg {
   using Cfg = SimtCfg<T>;
   static constexpr int KP = sizeof(T) == 4 ? 32 : 16;  // longest padded K it takes
-  static constexpr size_t C_BYTES = (size_t)Cfg::BN * Cfg::BM * sizeof(T);  // [BN][BM], dense
+  static constexpr int LDCB = Cfg::BM + 4;  // SHORTK_BULK: column pitch
+  // [BN][BM], dense; FP32 also [BN][LDCB]
+  static constexpr size_t C_BYTES = (size_t)Cfg::BN * (sizeof(T) == 4 ? LDCB : Cfg::BM) * sizeof(T);
   static constexpr size_t N_BYTES = (size_t)Cfg::BN * sizeof(int64_t);
   static constexpr size_t A_BYTES = (size_t)KP * Cfg::BM * sizeof(T);
   static constexpr size_t B_BYTES = (size_t)KP * Cfg::BN * sizeof(T);
@@ -687,14 +790,39 @@ struct SimtShortKCfg {
   static_assert(2 * (SMEM_BYTES + 1024) <= 228 * 1024, "two CTAs per SM");
 };
 
-template <typename T, bool TMA>
+enum ShortKC : int { SHORTK_ANY = 0, SHORTK_TMA = 1, SHORTK_BULK = 2 };
+
+// One column of a SHORTK_BULK block: g = its first element (len of them), at
+// element `shift` of its shared-memory column; [lo, hi) = the aligned range
+// around it, [in0, in1) the one inside it (empty when in1 <= in0).
+struct ShortKCol {
+  const char *g, *end, *lo, *hi, *in0, *in1;
+  int shift;
+  __device__ __forceinline__ ShortKCol(const float* first, int len) {
+    g = reinterpret_cast<const char*>(first);
+    end = g + 4 * (int64_t)len;
+    const uintptr_t u = reinterpret_cast<uintptr_t>(g), e = reinterpret_cast<uintptr_t>(end);
+    lo = g - (u & 15);
+    hi = end + (-e & 15);
+    in0 = g + (-u & 15);
+    in1 = end - (e & 15);
+    shift = (int)(u & 15) / 4;
+  }
+  // offset of p in the column's shared memory (bytes)
+  __device__ __forceinline__ int at(const char* p) const { return (int)(p - lo); }
+};
+
+template <typename T, int MODE>
 __global__ void __launch_bounds__(256, 2)
     simt_shortk_kernel(const SimtArgs<T> a, const __grid_constant__ CUtensorMap tmC) {
+  constexpr bool TMA = MODE == SHORTK_TMA, BULK = MODE == SHORTK_BULK;
+  static_assert(!BULK || sizeof(T) == 4, "bulk columns: FP32");
   using Cfg = SimtCfg<T>;
   using SC = SimtShortKCfg<T>;
   constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK;
   constexpr int VEC = 16 / sizeof(T);  // elements per 16-byte access
-  constexpr int QPC = BM / 4, CPI = 256 / QPC, ITER = BN / CPI;
+  constexpr int CPI = 256 / BM, CH = 16;  // element path: columns per step, steps at once
+  static_assert(BN % (CPI * CH) == 0, "whole steps");
   using Frag = SimtFrag<T, SIMT_SQUARE, false>;
   constexpr int TM = Frag::TM, TN = Frag::TN;
   constexpr int64_t NONE = INT64_MIN;  // offsets may be negative (negative strides)
@@ -714,7 +842,37 @@ __global__ void __launch_bounds__(256, 2)
   const T alpha = a.alpha, beta = a.beta;
   const bool read_c = beta != T(0);
 
-  if constexpr (TMA) {
+  if constexpr (BULK) {
+    if (tid == 0) {
+      mbar_init(bar, BN);
+      fence_mbar_init();
+    }
+    __syncthreads();
+    if (read_c && tid < BN) {  // column tid; the packing kernel does not write C
+      uint32_t bytes = 0;
+      if (n0 + tid < a.N) {
+        const float* first = a.C + m0 + a.ldc * (n0 + tid);
+        const ShortKCol c(first, (int)(a.M - m0 < BM ? a.M - m0 : BM));
+        char* dst = reinterpret_cast<char*>(Cs + tid * SC::LDCB);
+        const char *b0 = c.lo, *b1 = c.hi;
+        if (c.lo < reinterpret_cast<const char*>(a.C) ||
+            c.hi > reinterpret_cast<const char*>(a.C + a.M + a.ldc * (a.N - 1))) {
+          // an end of C: the aligned range inside the column, edges one by one
+          b0 = c.in0;
+          b1 = c.in1 > c.in0 ? c.in1 : c.in0;
+          for (const char* p = c.g; p < c.end; p += 4)
+            if (p < b0 || p >= b1)
+              *reinterpret_cast<float*>(dst + c.at(p)) = *reinterpret_cast<const float*>(p);
+        }
+        bytes = (uint32_t)(b1 - b0);
+        if (bytes) {
+          mbar_arrive_expect_tx(bar, bytes);
+          bulk_load_1d(dst + c.at(b0), b0, bytes, bar);
+        }
+      }
+      if (!bytes) mbar_arrive(bar);
+    }
+  } else if constexpr (TMA) {
     if (tid == 0) {
       mbar_init(bar, 1);
       fence_mbar_init();
@@ -723,7 +881,7 @@ __global__ void __launch_bounds__(256, 2)
     // the packing kernel before this one does not write C: the block comes
     // in while that kernel may still run
     if (read_c && tid == 0) {
-      mbar_arrive_expect_tx(bar, (uint32_t)SC::C_BYTES);
+      mbar_arrive_expect_tx(bar, (uint32_t)(BN * BM * sizeof(T)));
       tma_load_2d(Cs, &tmC, (int32_t)m0, (int32_t)n0, bar);
     }
   }
@@ -738,53 +896,34 @@ __global__ void __launch_bounds__(256, 2)
     cp_async_16(Bs + row * BN + col, a.Bp + (int64_t)row * a.Np + n0 + col);
   }
   cp_async_commit();
-  // element path: the thread's 4 m (quad q) of columns cl + u * CPI
-  const int q = tid % QPC, cl = tid / QPC;
-  int64_t cmo[4] = {NONE, NONE, NONE, NONE};
-  bool vq = false;
-  if constexpr (!TMA) {
+  // element path: the thread's m and its columns cl + u * CPI
+  const int ml = tid % BM, cl = tid / BM;
+  int64_t cmo = NONE;
+  if constexpr (MODE == SHORTK_ANY) {
     if (tid < BN) Cn[tid] = n0 + tid < a.N ? __ldg(a.c_n_off + n0 + tid) : NONE;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int64_t m = m0 + 4 * q + i;
-      cmo[i] = m < a.M ? __ldg(a.c_m_off + m) : NONE;
-    }
-    vq = cmo[3] != NONE && cmo[1] == cmo[0] + 1 && cmo[2] == cmo[0] + 2 && cmo[3] == cmo[0] + 3;
-  }
-  auto aligned16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-  if constexpr (!TMA) {
+    if (m0 + ml < a.M) cmo = __ldg(a.c_m_off + m0 + ml);
     __syncthreads();  // Cn staged
-    if (read_c && cmo[0] != NONE) {
+    if (read_c && cmo != NONE) {
+      T* const Cb = a.C + cmo;
+#pragma unroll 1
+      for (int c1 = cl; c1 < BN; c1 += CPI * CH) {
+        int64_t no[CH];  // read before the copies (each clobbers memory)
 #pragma unroll
-      for (int u = 0; u < ITER; ++u) {
-        const int col = u * CPI + cl;
-        const int64_t no = Cn[col];
-        if (no == NONE) continue;
-        T* dst = Cs + col * BM + 4 * q;
-        const T* src = a.C + cmo[0] + no;
-        if (vq && aligned16(src)) {
-          cp_async_16(dst, src);
-          if constexpr (sizeof(T) == 8) cp_async_16(dst + 2, src + 2);
-        } else {
+        for (int u = 0; u < CH; ++u) no[u] = Cn[c1 + u * CPI];
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            if (cmo[i] != NONE) cp_async_elem<sizeof(T)>(dst + i, a.C + cmo[i] + no);
-        }
+        for (int u = 0; u < CH; ++u)
+          if (no[u] != NONE) cp_async_elem<sizeof(T)>(Cs + (c1 + u * CPI) * BM + ml, Cb + no[u]);
       }
     }
   }
   cp_async_commit();
   cp_async_wait<1>();  // operand panels in place; the C block may still be in flight
   __syncthreads();
-  T acc[TM][TN];
-#pragma unroll
-  for (int i = 0; i < TM; ++i)
-#pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = T(0);
-  for (int kt = 0; kt < a.ktiles; ++kt)
-    simt_fma_ktile<T, SIMT_SQUARE, false>(As + kt * BK * BM, Bs + kt * BK * BN, frag.a_off,
-                                          frag.b_off, acc);
-  if constexpr (TMA) {
+  SimtAcc<T, SIMT_SQUARE, false> acc;
+  acc.zero();
+  for (int k = 0; k < (int)a.K; k += 4)  // the panels are padded with zeros past K
+    simt_fma_ktile<T, SIMT_SQUARE, false, 4>(As + k * BM, Bs + k * BN, frag.a_off, frag.b_off, acc);
+  if constexpr (TMA || BULK) {
     if (read_c && !mbar_wait(bar, 0)) {
       record_error(a.status, 4);
       return;  // nothing stored; the block's load never completed
@@ -792,6 +931,59 @@ __global__ void __launch_bounds__(256, 2)
   } else {
     cp_async_wait<0>();
     __syncthreads();
+  }
+  if constexpr (BULK) {
+    // element (n, m) at Cs[n LDCB + shift(n) + m]; a thread's 4 columns n, n +
+    // 1, .. of a group are 4 lanes' worth apart (same shift, banks 16 apart):
+    // lane group ln takes m = 4 lm + (i + ln) % 4
+    const int ln = (tid & 31) >> 3;
+    const uint32_t s0 = (uint32_t)(reinterpret_cast<uintptr_t>(a.C) / 4) + (uint32_t)m0 +
+                        (uint32_t)a.ldc * (uint32_t)n0;
+#pragma unroll
+    for (int j = 0; j < TN; ++j) {
+      const int n = frag.n(j);
+      float* c = Cs + n * SC::LDCB + (int)((s0 + (uint32_t)n * (uint32_t)a.ldc) & 3u) + frag.m0;
+#pragma unroll
+      for (int g = 0; g < TM; g += 4) {
+        float w[4], v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = alpha * acc.get(g + i, j);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[i] = ln & 1 ? v[(i + 1) & 3] : v[i];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = ln & 2 ? w[(i + 2) & 3] : w[i];
+        float* cg = c + 8 * g;  // group g / 4: 32 m further
+        if (read_c) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) v[i] = fma(beta, cg[(i + ln) & 3], v[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) cg[(i + ln) & 3] = v[i];
+      }
+    }
+    fence_proxy_async_smem();
+    __syncthreads();
+    const int col = tid % BN;
+    if (n0 + col >= a.N) return;
+    const ShortKCol c(a.C + m0 + a.ldc * (n0 + col), (int)(a.M - m0 < BM ? a.M - m0 : BM));
+    const char* src = reinterpret_cast<const char*>(Cs + col * SC::LDCB);
+    if (tid < BN) {  // the aligned range inside the column
+      if (c.in1 > c.in0) {
+        bulk_store_1d(const_cast<char*>(c.in0), src + c.at(c.in0), (uint32_t)(c.in1 - c.in0));
+        bulk_commit();
+        bulk_wait_read_all();  // shared memory stays valid until the store has read it
+      }
+    } else {  // its edges: before in0, and from in1 on
+      const char* e0 = c.in0 < c.end ? c.in0 : c.end;
+      const char* e1 = c.in1 > e0 ? c.in1 : e0;
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        const char *p = c.g + 4 * i, *q = e1 + 4 * i;
+        if (p < e0) *reinterpret_cast<float*>(const_cast<char*>(p)) = *reinterpret_cast<const float*>(src + c.at(p));
+        if (q < c.end) *reinterpret_cast<float*>(const_cast<char*>(q)) = *reinterpret_cast<const float*>(src + c.at(q));
+      }
+    }
+    return;
   }
   // combine at the fragment positions: runs of VEC consecutive m (16 bytes)
 #pragma unroll
@@ -801,7 +993,7 @@ __global__ void __launch_bounds__(256, 2)
       T* c = Cs + frag.n(j) * BM + frag.m(i0);
       T v[VEC];
 #pragma unroll
-      for (int e = 0; e < VEC; ++e) v[e] = alpha * acc[i0 + e][j];
+      for (int e = 0; e < VEC; ++e) v[e] = alpha * acc.get(i0 + e, j);
       if (read_c) {
         if constexpr (sizeof(T) == 4) {
           const float4 o = *reinterpret_cast<const float4*>(c);
@@ -828,26 +1020,20 @@ __global__ void __launch_bounds__(256, 2)
     return;
   }
   __syncthreads();
-  if (cmo[0] == NONE) return;
+  if (cmo == NONE) return;
+  T* const Cb = a.C + cmo;
+#pragma unroll 1
+  for (int c1 = cl; c1 < BN; c1 += CPI * CH) {
+    int64_t no[CH];  // read before the stores (which may alias as far as the compiler knows)
+    T v[CH];
 #pragma unroll
-  for (int u = 0; u < ITER; ++u) {
-    const int col = u * CPI + cl;
-    const int64_t no = Cn[col];
-    if (no == NONE) continue;
-    const T* src = Cs + col * BM + 4 * q;
-    T* d = a.C + cmo[0] + no;
-    if (vq && aligned16(d)) {
-      if constexpr (sizeof(T) == 4) {
-        *reinterpret_cast<float4*>(d) = *reinterpret_cast<const float4*>(src);
-      } else {
-        reinterpret_cast<double2*>(d)[0] = reinterpret_cast<const double2*>(src)[0];
-        reinterpret_cast<double2*>(d)[1] = reinterpret_cast<const double2*>(src)[1];
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        if (cmo[i] != NONE) a.C[cmo[i] + no] = src[i];
+    for (int u = 0; u < CH; ++u) {
+      no[u] = Cn[c1 + u * CPI];
+      v[u] = Cs[(c1 + u * CPI) * BM + ml];
     }
+#pragma unroll
+    for (int u = 0; u < CH; ++u)
+      if (no[u] != NONE) Cb[no[u]] = v[u];
   }
 }
 

@@ -86,6 +86,7 @@ struct tccg_plan {
   int32_t* d_status = nullptr;
   int32_t read_k_fast_a = 0, read_k_fast_b = 0;
   bool c_is_mn_dense = false;  // C is already the column-major [M-modes][N-modes] matrix
+  bool c_quads = false;  // every quad of m is 4 consecutive elements of C at offsets % 4 == 0
   int64_t c_ldc = 0;  // > 0: C(m, n) = C[m + c_ldc * n] (a 2-D matrix in the GETT view)
   // SIMT geometry
   int64_t Mp = 0, Np = 0, Kp = 0;
@@ -335,6 +336,16 @@ static bool choose_simt(const tccg_plan* p) {
   if (p->prec == TCCG_PREC_FP64) return true;
   if (p->tune.pair || p->tune.variant > 0 || p->tune.load > 0) return false;
   if (p->tune.variant < 0) return true;
+  // K <= 32 on a 2-D C: the short-K kernel, which streams C in and out in
+  // blocks (9216^2 x 24, BF16: beta = 0 116 us against 157 us on the tensor
+  // cores, whose epilogue stores element by element, beta = 1 136 / 525;
+  // columns off 16-byte boundaries 139 / 145 and 162 / 500)
+  if (p->tune.load == 0 && p->tune.tile_n == 0 && p->K <= SimtShortKCfg<float>::KP &&
+      p->tune.shortk >= 0 && p->tune.ksplit <= 1 && p->tune.method == TCCG_METHOD_GETT &&
+      p->c_ldc > 0 && p->M >= 128 && p->N >= 128 &&
+      cdiv(p->M, 128) * cdiv(p->N, 128) >= 2 * (int64_t)p->num_sms &&
+      choose_simt_shape(p, nullptr) == SIMT_SQUARE && !direct_eligible(p, SIMT_SQUARE))
+    return true;
   // against the tensor-core model (tc_time, with the loader the tuning asks for)
   return simt_time(p) < tc_time(p, p->tune.load == 2 && gather_eligible(p));
 }
@@ -400,17 +411,18 @@ static bool shortk_tma(const tccg_plan* p, int64_t ldc) {
 }
 
 // The short-K kernel that prefetches its C block under the FMA phase:
-// packed operands, the whole K in one panel, no k-split. Automatically only
-// with the TMA C block (the cp.async one measured no faster than the tile
-// kernel) and at least two tiles per SM. TTGT writes the contiguous C'
-// (ldc = M).
+// packed operands, the whole K in one panel, no k-split. Automatically where
+// C is a 2-D matrix (moved by TMA, or with lanes along m where its columns
+// are not 16-byte aligned; for other layouts it measured no faster than the
+// tile kernel) of at least two tiles per SM and one tile in each direction.
+// TTGT writes the contiguous C' (ldc = M).
 static bool choose_shortk(const tccg_plan* p, int64_t tiles) {
   if (p->direct || p->ksplit > 1 || p->tune.shortk < 0 || p->simt_shape != SIMT_SQUARE) return false;
   const int kp = p->prec == TCCG_PREC_FP64 ? SimtShortKCfg<double>::KP : SimtShortKCfg<float>::KP;
   if (p->Kp > kp) return false;
   if (p->tune.shortk > 0) return true;
   const int64_t ldc = p->tune.method == TCCG_METHOD_TTGT ? p->M : p->c_ldc;
-  return shortk_tma(p, ldc) && tiles >= 2 * (int64_t)p->num_sms;
+  return ldc > 0 && p->M >= p->simt_bm && p->N >= p->simt_bn && tiles >= 2 * (int64_t)p->num_sms;
 }
 
 // K slices for `tiles` C tiles over `kblocks` k-blocks when `slots` CTAs run
@@ -980,6 +992,9 @@ extern "C" int tccg_plan_create(const tccg_desc* desc, int32_t dtype, int32_t pr
     for (int i = 0; i < d.nn; ++i) { dense &= d.c_n_stride[i] == s; s *= d.n_ext[i]; }
     p->c_is_mn_dense = dense;
   }
+  p->c_quads = d.c_m_stride[0] == 1 && (d.m_ext[0] % 4 == 0 || p->M == d.m_ext[0]);
+  for (int i = 1; i < d.nm; ++i) p->c_quads &= d.m_ext[i] == 1 || d.c_m_stride[i] % 4 == 0;
+  for (int i = 0; i < d.nn; ++i) p->c_quads &= d.n_ext[i] == 1 || d.c_n_stride[i] % 4 == 0;
   bool m_unit = true;
   for (size_t m = 0; m < h.size() && m_unit; ++m) m_unit = h[m] == (int64_t)m;
   if (!rc) rc = upload(h, &p->t_c_m);
@@ -1195,7 +1210,8 @@ static int plan_layout(tccg_plan* p) {
              BM, BN, BK,
              (long long)p->M, (long long)p->N, (long long)p->K, p->ksplit,
              p->direct ? "none" : "MN", p->prec == TCCG_PREC_BF16 ? " bf16-rounded" : "",
-             !p->shortk ? "" : shortk_tma(p, ttgt ? p->M : p->c_ldc) ? " cblock=tma" : " cblock=cp.async",
+             !p->shortk ? "" : shortk_tma(p, ttgt ? p->M : p->c_ldc) ? " cblock=tma"
+             : !dbl && (ttgt || p->c_ldc > 0) ? " cblock=cp.async.bulk" : " cblock=cp.async",
              p->direct ? "gather_k" : "read_k_fast",
              p->direct ? (int)p->gather_k_a : p->read_k_fast_a,
              p->direct ? (int)p->gather_k_b : p->read_k_fast_b);
@@ -1438,13 +1454,15 @@ static cudaError_t set_attrs() {
                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)simt_smem_bytes<double>()));
   chk(cudaFuncSetAttribute(simt_gett_kernel<double, SIMT_DIRECT>,
                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)simt_smem_bytes<double>()));
-  chk(cudaFuncSetAttribute(simt_shortk_kernel<float, true>,
+  chk(cudaFuncSetAttribute(simt_shortk_kernel<float, SHORTK_TMA>,
                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SimtShortKCfg<float>::SMEM_BYTES));
-  chk(cudaFuncSetAttribute(simt_shortk_kernel<float, false>,
+  chk(cudaFuncSetAttribute(simt_shortk_kernel<float, SHORTK_BULK>,
                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SimtShortKCfg<float>::SMEM_BYTES));
-  chk(cudaFuncSetAttribute(simt_shortk_kernel<double, true>,
+  chk(cudaFuncSetAttribute(simt_shortk_kernel<float, SHORTK_ANY>,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SimtShortKCfg<float>::SMEM_BYTES));
+  chk(cudaFuncSetAttribute(simt_shortk_kernel<double, SHORTK_TMA>,
                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SimtShortKCfg<double>::SMEM_BYTES));
-  chk(cudaFuncSetAttribute(simt_shortk_kernel<double, false>,
+  chk(cudaFuncSetAttribute(simt_shortk_kernel<double, SHORTK_ANY>,
                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SimtShortKCfg<double>::SMEM_BYTES));
   chk(cudaFuncSetAttribute(f32_fallback_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)simt_smem_bytes<float>()));
@@ -1761,6 +1779,13 @@ static void set_direct(SimtArgs<T>& a, const tccg_plan* p, const void* GA, const
   a.b_k_off = p->t_b_k;
 }
 
+// Whether the CUDA-core epilogue may move 4 m of C per thread (SimtArgs::c_vec):
+// C in the plan's layout, or TTGT's contiguous C' (tt).
+template <typename T>
+static int32_t c_vectors(const tccg_plan* p, const T* C, bool tt) {
+  return (tt ? p->M % 4 == 0 : p->c_quads) && reinterpret_cast<uintptr_t>(C) % (4 * sizeof(T)) == 0;
+}
+
 // simt_gett_kernel with the plan's tile shape (FP32: three shapes).
 template <typename T, int LOAD>
 static void launch_simt_tiles(const tccg_plan* p, const SimtArgs<T>& a, dim3 grid, bool after,
@@ -1823,17 +1848,22 @@ static int run_simt(const tccg_plan* p, const void* GA, const void* GB, T* Cout,
   set_direct(a, p, GA, GB);
   a.status = p->d_status;
   a.crun = c_m == p->t_c_m ? p->crun : 0;  // not for TTGT's contiguous C'
+  a.c_vec = c_vectors(p, Cout, c_m != p->t_c_m);
+  a.ldc = c_ldc;
   dim3 grid((unsigned)(p->Mp / p->simt_bm), (unsigned)(p->Np / p->simt_bn), (unsigned)p->ksplit);
   if (grid.y > 65535u || grid.z > 65535u) return fail(TCCG_ERR_UNSUPPORTED, "grid too large");
   mark(1, 0, s);
   CUtensorMap tmC{};
   if (p->shortk && shortk_tma(p, c_ldc) &&
       encode_c2d<T>(&tmC, Cout, p->M, p->N, c_ldc, Cfg::BM, Cfg::BN))
-    launch_after(packed, p, simt_shortk_kernel<T, true>, grid, dim3(256),
+    launch_after(packed, p, simt_shortk_kernel<T, SHORTK_TMA>, grid, dim3(256),
                  SimtShortKCfg<T>::SMEM_BYTES, s, a, tmC);
-  else if (p->shortk)
-    launch_after(packed, p, simt_shortk_kernel<T, false>, grid, dim3(256),
-                 SimtShortKCfg<T>::SMEM_BYTES, s, a, tmC);
+  else if (p->shortk) {
+    auto kernel = simt_shortk_kernel<T, SHORTK_ANY>;
+    if constexpr (sizeof(T) == 4)
+      if (c_ldc > 0) kernel = simt_shortk_kernel<T, SHORTK_BULK>;
+    launch_after(packed, p, kernel, grid, dim3(256), SimtShortKCfg<T>::SMEM_BYTES, s, a, tmC);
+  }
   else if (p->direct)
     launch_simt_tiles<T, SIMT_DIRECT>(p, a, grid, false, s);
   else
@@ -1925,6 +1955,7 @@ static F32FallbackItem f32_fallback_item(const tccg_plan* p, const void* GA, con
   a.direct = 1;
   a.status = p->d_status;
   a.crun = p->crun;
+  a.c_vec = c_vectors(p, C, false);
   it.range = range;
   it.K = (int32_t)p->K;
   it.tiles_m = (int32_t)cdiv(p->M, SimtCfg<float>::BM);
@@ -2636,6 +2667,7 @@ static SimtArgs<T> simt_args_for(const tccg_plan* p, char* w, const void* GA, co
   set_direct(a, p, GA, GB);
   a.status = p->d_status;
   a.crun = p->crun;
+  a.c_vec = c_vectors(p, a.C, false);
   return a;
 }
 
