@@ -384,6 +384,22 @@ __device__ __forceinline__ void cp_async_elem(void* smem_dst, const void* gsrc) 
                "n"(BYTES)
                : "memory");
 }
+// the same where `in` holds, without a branch (a divergent branch per copy
+// costs about 100 cycles)
+__device__ __forceinline__ void cp_async_4_if(void* smem_dst, const void* gsrc, bool in) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t"
+      "@q cp.async.ca.shared.global [%0], [%1], 4;\n\t}" ::"r"(smem_u32(smem_dst)),
+      "l"(gsrc), "r"((uint32_t)in)
+      : "memory");
+}
+__device__ __forceinline__ void cp_async_16_if(void* smem_dst, const void* gsrc, bool in) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t"
+      "@q cp.async.cg.shared.global [%0], [%1], 16;\n\t}" ::"r"(smem_u32(smem_dst)),
+      "l"(gsrc), "r"((uint32_t)in)
+      : "memory");
+}
 // Arrive on `bar` once all of this thread's earlier cp.async copies landed
 // (the barrier's expected count includes this arrival).
 __device__ __forceinline__ void cp_async_mbar_arrive(uint64_t* bar) {

@@ -124,7 +124,9 @@ struct SkinnyArgs {
   int32_t q_kfast;         // Q loads along k (its stride-one index is a K mode)
   int32_t s_run;           // SK_C_SX: extent of C's stride-one S mode
   // SK_P_X with unit x stride, every k offset and P itself 16-byte aligned:
-  // four positions that are consecutive in P move as one 16-byte copy
+  // four positions that are consecutive in P move as one 16-byte copy.
+  // SK_P_K: every position offset and P aligned, every quad of k 4 consecutive
+  // elements: the register path and the tensor-core kernel load quads of k
   int32_t p_vec;
   // C of a box row is one contiguous range (SkinnyCLin): staged in that
   // order and stored as a straight copy
@@ -180,6 +182,24 @@ __device__ __forceinline__ int skinny_kc(const A& a, int c) {
   return a.K - k0 < SK_KC ? (int)(a.K - k0) : SK_KC;
 }
 
+// P offset of box position (xl, yl) of box (ix, iy). Outside the box or the
+// tensor: SK_NONE for the walks along the positions (copies predicated off),
+// for the walk along k (clamp) the offset of a position inside, so that the copy loops test nothing (and touch no other memory: one
+// element for all would be a hot spot of the L2). Such positions' sums are
+// never stored.
+__device__ __forceinline__ int32_t skinny_p_off(const SkinnyArgs& a, int ix, int iy, int xl, int yl,
+                                                bool clamp) {
+  int x = ix * a.tx + xl, y = iy * a.ty + yl;
+  if (xl >= a.tx || yl >= a.ty || x >= a.ex || y >= a.ey) {
+    if (!clamp) return SK_NONE;
+    if (xl >= a.tx) x = ix * a.tx;
+    if (yl >= a.ty) y = iy * a.ty;
+    if (x >= a.ex) x = a.ex - 1;
+    if (y >= a.ey) y = a.ey - 1;
+  }
+  return x * a.px + __ldg(a.p_y_off + y);
+}
+
 // Offsets of block b's box positions (one per thread) into pw / cw, and the
 // C offsets of pass p's rows into cs (when the job stores to C).
 __device__ __forceinline__ void skinny_begin(const SkinnyArgs& a, int b, int p, int sp,
@@ -196,7 +216,7 @@ __device__ __forceinline__ void skinny_begin(const SkinnyArgs& a, int b, int p, 
   }
   const int x = ix * a.tx + xl, y = iy * a.ty + yl;
   const bool ok = w < a.tx * a.ty && x < a.ex && y < a.ey;
-  pw[w] = ok ? x * a.px + __ldg(a.p_y_off + y) : SK_NONE;
+  pw[w] = skinny_p_off(a, ix, iy, xl, yl, a.p_walk == SK_P_K);
   cw[w] = ok ? x * a.cx + __ldg(a.c_y_off + y) : SK_NONE;
   if (!a.partial && w < a.spr) {
     const int s = p * a.spr + w;
@@ -216,73 +236,70 @@ __device__ __forceinline__ int32_t skinny_p_ko(const A& a, int c) {
 }
 
 // Issues the P copies of chunk c ([k][position], k < the chunk's extent) of
-// the box whose offsets pw holds (visible to all threads; positions outside
-// the tensor are zeros); ko = skinny_p_ko(a, c). Threads 0 .. SK_THREADS - 1
-// take part; no commit. SKIP: positions outside the tensor are left
-// unwritten (the consumer substitutes zeros for them).
-template <bool SKIP = false, typename A = SkinnyArgs>
+// the box whose offsets pw holds (visible to all threads); ko =
+// skinny_p_ko(a, c). Thread t of NT (128 or 256; warps of whole position
+// ranges) takes part; no commit.
+template <int NT = SK_THREADS, typename A = SkinnyArgs>
 __device__ __forceinline__ void skinny_issue_p(const A& a, int c, float* ps,
-                                               const int32_t* pw, int32_t ko) {
-  auto zero = [&](float* d) {
-    if (!SKIP) *d = 0.0f;
-  };
-  const int tid = threadIdx.x;
+                                               const int32_t* pw, int32_t ko, int t) {
   const int kc = skinny_kc(a, c);
   // read once: each cp.async clobbers memory, and a grouped launch's item is
   // in global memory, which the compiler would otherwise read again
   const float* const P = a.P;
   if (a.p_walk == SK_P_K) {
-    // lanes along k: thread tid takes k = tid % kr of positions tid / kr + i * 256 / kr
-    const int lg = a.kr_log2, kl = tid & ((1 << lg) - 1);
+    // lanes along k: thread t takes k = t % kr of positions t / kr + i * NT / kr
+    const int lg = a.kr_log2, kl = t & ((1 << lg) - 1);
     if (kl < kc) {
       float* d = ps + kl * SK_LDP;
+      const float* src = P + ko;
 #pragma unroll 4
-      for (int w = tid >> lg; w < SK_BW; w += SK_THREADS >> lg) {
-        const int32_t po = pw[w];
-        if (po != SK_NONE)
-          cp_async_elem<4>(d + w, P + po + ko);
-        else
-          zero(d + w);
-      }
+      for (int w = t >> lg; w < SK_BW; w += NT >> lg) cp_async_elem<4>(d + w, src + pw[w]);
     }
-  } else if (a.p_vec) {
+    return;
+  }
+  if (a.p_vec) {
     // four consecutive positions per 16-byte copy where they are consecutive
-    // and aligned in P (else four element copies): thread tid takes
-    // positions 4 (tid % WG) .. + 3 at k = tid / WG, tid / WG + 4, ...
-    const int g = 4 * (tid % SK_WG);
+    // and aligned in P for the whole warp (else element copies): thread t
+    // takes positions 4 (t % WG) .. + 3 at k = t / WG, t / WG + NT / WG, ...
+    const int g = 4 * (t % SK_WG);
     const int32_t o0 = pw[g], o1 = pw[g + 1], o2 = pw[g + 2], o3 = pw[g + 3];
+    const bool none = o0 == SK_NONE && o1 == SK_NONE && o2 == SK_NONE && o3 == SK_NONE;
     const bool vec = o0 != SK_NONE && (o0 & 3) == 0 && o1 == o0 + 1 && o2 == o0 + 2 && o3 == o0 + 3;
-    for (int k = tid / SK_WG; k < kc; k += SK_SG) {  // warp-uniform k
-      const int32_t kok = __shfl_sync(0xffffffffu, ko, k);
-      float* d = ps + k * SK_LDP + g;
-      if (vec) {
-        cp_async_16(d, P + o0 + kok);
-      } else {
-        const int32_t o[4] = {o0, o1, o2, o3};
+    float* d = ps + g;
+    if (__all_sync(0xffffffffu, vec || none)) {
+      const float* src = P + (none ? 0 : o0);
+#pragma unroll 4
+      for (int k = t / SK_WG; k < kc; k += NT / SK_WG)  // warp-uniform k
+        cp_async_16_if(d + k * SK_LDP, src + __shfl_sync(0xffffffffu, ko, k), !none);
+    } else {
+      const int32_t o[4] = {o0, o1, o2, o3};
+#pragma unroll 2
+      for (int k = t / SK_WG; k < kc; k += NT / SK_WG) {
+        const int32_t kok = __shfl_sync(0xffffffffu, ko, k);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          if (o[e] != SK_NONE)
-            cp_async_elem<4>(d + e, P + o[e] + kok);
-          else
-            zero(d + e);
-        }
+        for (int e = 0; e < 4; ++e)
+          cp_async_4_if(d + k * SK_LDP + e, P + (o[e] != SK_NONE ? o[e] + kok : 0), o[e] != SK_NONE);
       }
     }
-  } else {
-    // lanes along the positions: thread tid takes position tid at every k;
-    // the chunk's k offsets are loaded once per warp (lane k) and passed
-    // around by shuffles, so no copy waits on a table load
-    const int32_t po = pw[tid];
-    float* d = ps + tid;
-    const float* src = P + (po != SK_NONE ? po : 0);
+    return;
+  }
+  // lanes along the positions: thread t takes positions t, t + NT, .. at every
+  // k; the chunk's k offsets are loaded once per warp (lane k) and passed
+  // around by shuffles, so no copy waits on a table load
+  const float* src[SK_BW / NT];
+  bool in[SK_BW / NT];
+#pragma unroll
+  for (int h = 0; h < SK_BW / NT; ++h) {
+    const int32_t o = pw[t + h * NT];
+    in[h] = o != SK_NONE;
+    src[h] = P + (in[h] ? o : 0);
+  }
+  float* d = ps + t;
 #pragma unroll 4
-    for (int k = 0; k < kc; ++k) {
-      const int32_t kok = __shfl_sync(0xffffffffu, ko, k);
-      if (po != SK_NONE)
-        cp_async_elem<4>(d + k * SK_LDP, src + kok);
-      else
-        zero(d + k * SK_LDP);
-    }
+  for (int k = 0; k < kc; ++k) {
+    const int32_t kok = __shfl_sync(0xffffffffu, ko, k);
+#pragma unroll
+    for (int h = 0; h < SK_BW / NT; ++h) cp_async_4_if(d + k * SK_LDP + h * NT, src[h] + kok, in[h]);
   }
 }
 
@@ -292,7 +309,7 @@ __device__ __forceinline__ void skinny_issue_p(const A& a, int c, float* ps,
 // skinny_p_ko(a, c).
 __device__ __forceinline__ void skinny_issue(const SkinnyArgs& a, const SkJob& j, int c, int sp,
                                              float* ps, float* qs, const int32_t* pw, int32_t ko) {
-  skinny_issue_p(a, c, ps, pw, ko);
+  skinny_issue_p(a, c, ps, pw, ko, threadIdx.x);
   const int tid = threadIdx.x, lane = tid & 31;
   const int k0 = c * SK_KC;
   const int kc = skinny_kc(a, c);
@@ -420,14 +437,20 @@ __device__ __forceinline__ void skinny_store(const SkinnyArgs& a, const float* o
   }
 }
 
+// FP32 pairs (fma.rn.f32x2) of two rows and two positions: v[i][2 p + s] holds
+// row 2 i of position 2 p + s and row 2 i + 1 of the pair's other position (a
+// pair of rows times the pair of positions, or times the swapped pair).
 template <int RS>
 struct SkAcc {
-  float v[RS][4];
+  uint64_t v[RS / 2][4];
   __device__ __forceinline__ void clear() {
 #pragma unroll
-    for (int i = 0; i < RS; ++i)
+    for (int i = 0; i < RS / 2; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) v[i][j] = 0.0f;
+      for (int j = 0; j < 4; ++j) v[i][j] = 0;
+  }
+  __device__ __forceinline__ float get(int i, int e) const {
+    return i % 2 == 0 ? f32x2_lo(v[i / 2][e]) : f32x2_hi(v[i / 2][e ^ 1]);
   }
 };
 
@@ -439,19 +462,20 @@ __device__ __forceinline__ void skinny_fma(SkAcc<RS>& acc, const float* ps, cons
   const float* qq = qs + (tid / SK_WG) * RS;
 #pragma unroll 4
   for (int k = 0; k < kc; ++k) {
-    const float4 pv = *reinterpret_cast<const float4*>(pp + k * SK_LDP);
-    float q[RS];
+    const ulonglong2 pv = *reinterpret_cast<const ulonglong2*>(pp + k * SK_LDP);
+    const uint64_t p0 = pv.x, p1 = pv.y, w0 = f32x2_swap(p0), w1 = f32x2_swap(p1);
 #pragma unroll
     for (int i = 0; i < RS; i += 4) {
-      const float4 t = *reinterpret_cast<const float4*>(qq + k * SK_QLD + i);
-      q[i] = t.x; q[i + 1] = t.y; q[i + 2] = t.z; q[i + 3] = t.w;
-    }
+      const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(qq + k * SK_QLD + i);
 #pragma unroll
-    for (int i = 0; i < RS; ++i) {
-      acc.v[i][0] = fmaf(q[i], pv.x, acc.v[i][0]);
-      acc.v[i][1] = fmaf(q[i], pv.y, acc.v[i][1]);
-      acc.v[i][2] = fmaf(q[i], pv.z, acc.v[i][2]);
-      acc.v[i][3] = fmaf(q[i], pv.w, acc.v[i][3]);
+      for (int u = 0; u < 2; ++u) {
+        const uint64_t q = u ? t.y : t.x;
+        uint64_t (&r)[4] = acc.v[i / 2 + u];
+        r[0] = fma_x2(q, p0, r[0]);
+        r[1] = fma_x2(q, w0, r[1]);
+        r[2] = fma_x2(q, p1, r[2]);
+        r[3] = fma_x2(q, w1, r[3]);
+      }
     }
   }
 }
@@ -588,7 +612,7 @@ __device__ __forceinline__ void skinny_finish_lin(const SkinnyArgs& a, const SkJ
         if (r >= 0 && r < SK_SUB) {
 #pragma unroll
           for (int e = 0; e < 4; ++e)
-            if (ob[e] >= 0) os[ob[e] + r * tx] = sc * acc.v[i][e];
+            if (ob[e] >= 0) os[ob[e] + r * tx] = sc * acc.get(i, e);
         }
       }
       if (a.c_bulk) fence_proxy_async_smem();  // the bulk copies read the staging
@@ -606,7 +630,7 @@ __device__ __forceinline__ void skinny_finish_lin(const SkinnyArgs& a, const SkJ
       if (r < S) {
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-          if (ob[e] >= 0) os[ob[e] + r] = acc.v[i][e];
+          if (ob[e] >= 0) os[ob[e] + r] = acc.get(i, e);
       }
     }
     __syncthreads();
@@ -626,7 +650,7 @@ __device__ __forceinline__ void skinny_finish(const SkinnyArgs& a, const SkJob& 
 #pragma unroll
     for (int i = 0; i < RS; ++i)
       *reinterpret_cast<float4*>(dst + (size_t)(sg * RS + i) * SK_BW) =
-          make_float4(acc.v[i][0], acc.v[i][1], acc.v[i][2], acc.v[i][3]);
+          make_float4(acc.get(i, 0), acc.get(i, 1), acc.get(i, 2), acc.get(i, 3));
     return;
   }
   if (a.c_lin == SK_CLIN_XS || a.c_lin == SK_CLIN_SX) {
@@ -645,7 +669,7 @@ __device__ __forceinline__ void skinny_finish(const SkinnyArgs& a, const SkJob& 
       const int r = sg * RS + i - h;
       if (r >= 0 && r < SK_SUB)
         *reinterpret_cast<float4*>(os + r * SK_LDP + 4 * wg) =
-            make_float4(acc.v[i][0], acc.v[i][1], acc.v[i][2], acc.v[i][3]);
+            make_float4(acc.get(i, 0), acc.get(i, 1), acc.get(i, 2), acc.get(i, 3));
     }
     __syncthreads();
     if (a.c_lin == SK_CLIN_RUNS)
@@ -879,32 +903,70 @@ __device__ __forceinline__ int32_t skinny_reg_ko(const SkinnyArgs& a, int kb, in
   return lane < SKR_KR && kb + lane < ke ? __ldg(a.p_k_off + kb + lane) : 0;
 }
 
-// P of the thread's two positions at k [kb, kb + 16) (zeros past ke or the
-// box); ko_lane = skinny_reg_ko(a, kb, ke).
-__device__ __forceinline__ void skinny_reg_p(const SkinnyArgs& a, int kb, int ke, int32_t po0,
-                                             int32_t po1, float (&p0)[SKR_KR], float (&p1)[SKR_KR],
-                                             int32_t ko_lane) {
+// P of the thread's two positions s0, s1 (a pair per k; zeros for null: outside
+// the box) at k [kb, kb + 16), zeros past ke; ko_lane = skinny_reg_ko(a, kb,
+// ke), 0 past ke (those loads read some element of P). quads: every quad of k
+// is 4 consecutive, aligned elements: one 16-byte load each (a warp's loads
+// touch 32 rows of P either way, with a quarter of the instructions: S = 8,
+// K = 720, W = 635040 contracted along its stride-one index 1397 -> 681 us);
+// compiled only into the kernels of such items (KW: with both forms the other
+// items spill, 473 -> 740 us at S = 11, K = 2744).
+template <bool KW>
+__device__ __forceinline__ void skinny_reg_p(int kb, int ke, const float* s0, const float* s1,
+                                             uint64_t (&p)[SKR_KR], int32_t ko_lane, bool quads) {
+  const int n = ke - kb;
+  if (KW && quads) {
 #pragma unroll
-  for (int kk = 0; kk < SKR_KR; ++kk) {
-    const int32_t ko = __shfl_sync(0xffffffffu, ko_lane, kk);
-    const bool kok = kb + kk < ke;
-    p0[kk] = kok && po0 != SK_NONE ? __ldg(a.P + po0 + ko) : 0.0f;
-    p1[kk] = kok && po1 != SK_NONE ? __ldg(a.P + po1 + ko) : 0.0f;
+    for (int kk = 0; kk < SKR_KR; kk += 4) {
+      const int32_t ko = __shfl_sync(0xffffffffu, ko_lane, kk);
+      const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      const float4 x = s0 ? __ldg(reinterpret_cast<const float4*>(s0 + ko)) : z;
+      const float4 y = s1 ? __ldg(reinterpret_cast<const float4*>(s1 + ko)) : z;
+      p[kk] = f32x2(x.x, y.x);
+      p[kk + 1] = f32x2(x.y, y.y);
+      p[kk + 2] = f32x2(x.z, y.z);
+      p[kk + 3] = f32x2(x.w, y.w);
+    }
+  } else {
+#pragma unroll
+    for (int kk = 0; kk < SKR_KR; ++kk) {
+      const int32_t ko = __shfl_sync(0xffffffffu, ko_lane, kk);
+      p[kk] = f32x2(s0 ? __ldg(s0 + ko) : 0.0f, s1 ? __ldg(s1 + ko) : 0.0f);
+    }
+  }
+  if (n < SKR_KR) {
+#pragma unroll
+    for (int kk = 0; kk < SKR_KR; ++kk)
+      if (kk >= n) p[kk] = 0;
   }
 }
+
+// A thread's sums of 2 positions x ROWS rows as pairs (fma.rn.f32x2): v[i][s] =
+// (row 2 i of position s, row 2 i + 1 of position 1 - s).
+template <int ROWS>
+struct SkrAcc {
+  uint64_t v[ROWS / 2][2];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int i = 0; i < ROWS / 2; ++i) v[i][0] = v[i][1] = 0;
+  }
+  __device__ __forceinline__ float get(int h, int r) const {
+    return r % 2 == 0 ? f32x2_lo(v[r / 2][h]) : f32x2_hi(v[r / 2][1 - h]);
+  }
+};
 
 // The end of a job: raw sums to its k slice, or the rows to C (staged in os).
 template <int ROWS>
 __device__ __forceinline__ void skinny_reg_finish(const SkinnyArgs& a, const SkJob& j,
-                                                  const float (&acc)[2][ROWS], float* os,
+                                                  const SkrAcc<ROWS>& acc, float* os,
                                                   const int32_t* cw, const int32_t* cs) {
   const int tid = threadIdx.x;
   if (a.partial) {  // layout of the 16-row (RS = 4) tile path; rows >= ROWS not written
     float* dst = a.partial + (((size_t)j.z * a.nblk + j.b) * a.npass + j.p) * SKR_ROWS * SK_BW + tid;
 #pragma unroll
     for (int r = 0; r < ROWS; ++r) {
-      dst[(size_t)r * SK_BW] = acc[0][r];
-      dst[(size_t)r * SK_BW + SKR_THREADS] = acc[1][r];
+      dst[(size_t)r * SK_BW] = acc.get(0, r);
+      dst[(size_t)r * SK_BW + SKR_THREADS] = acc.get(1, r);
     }
     return;
   }
@@ -922,7 +984,7 @@ __device__ __forceinline__ void skinny_reg_finish(const SkinnyArgs& a, const SkJ
       float* o = os + yl * plane + (xs ? xl : xl * S);
 #pragma unroll
       for (int r = 0; r < ROWS; ++r)
-        if (r < S) o[xs ? r * tx : r] = sc * acc[h][r];
+        if (r < S) o[xs ? r * tx : r] = sc * acc.get(h, r);
     }
     if (a.c_bulk) fence_proxy_async_smem();
     __syncthreads();
@@ -937,8 +999,8 @@ __device__ __forceinline__ void skinny_reg_finish(const SkinnyArgs& a, const SkJ
   }
 #pragma unroll
   for (int r = 0; r < ROWS; ++r) {
-    os[r * SK_LDP + tid] = acc[0][r];
-    os[r * SK_LDP + tid + SKR_THREADS] = acc[1][r];
+    os[r * SK_LDP + tid] = acc.get(0, r);
+    os[r * SK_LDP + tid + SKR_THREADS] = acc.get(1, r);
   }
   __syncthreads();
   skinny_store<SKR_THREADS>(a, os, cw, cs, 0, S, tid);
@@ -946,7 +1008,7 @@ __device__ __forceinline__ void skinny_reg_finish(const SkinnyArgs& a, const SkJ
 
 // One job of the register path with ROWS computed rows (16, or 8 for a
 // narrow side of at most 8: half the FMAs and Q copies).
-template <int ROWS>
+template <int ROWS, bool KW>
 __device__ __forceinline__ void skinny_reg_job(const SkinnyArgs& a, const SkJob& job, float* Qs,
                                                float* os, const int32_t* pw, const int32_t* cw,
                                                const int32_t* cs) {
@@ -954,22 +1016,24 @@ __device__ __forceinline__ void skinny_reg_job(const SkinnyArgs& a, const SkJob&
   const int32_t po0 = pw[tid], po1 = pw[tid + SKR_THREADS];
   const int kbeg = job.c0 * SK_KC;
   const int kend = job.c1 * SK_KC < a.K ? job.c1 * SK_KC : a.K;
-  float acc[2][ROWS];
-#pragma unroll
-  for (int r = 0; r < ROWS; ++r) acc[0][r] = acc[1][r] = 0.0f;
-  float pc0[SKR_KR], pc1[SKR_KR];
+  SkrAcc<ROWS> acc;
+  acc.clear();
+  const bool quads = KW && a.p_vec;
+  uint64_t pc[SKR_KR];
+  const float* s0 = po0 != SK_NONE ? a.P + po0 : nullptr;
+  const float* s1 = po1 != SK_NONE ? a.P + po1 : nullptr;
   skinny_reg_q<ROWS>(a, kbeg, kend, Qs);
-  skinny_reg_p(a, kbeg, kend, po0, po1, pc0, pc1, skinny_reg_ko(a, kbeg, kend));
+  skinny_reg_p<KW>(kbeg, kend, s0, s1, pc, skinny_reg_ko(a, kbeg, kend), quads);
   int32_t ko_next = skinny_reg_ko(a, kbeg + SKR_KR, kend);  // the next step's
   int st = 0;
 #pragma unroll 1
   for (int kb = kbeg; kb < kend; kb += SKR_KR) {
     const int nb = kb + SKR_KR;
-    float pn0[SKR_KR], pn1[SKR_KR];
+    uint64_t pn[SKR_KR];
     if (nb < kend) {
       __syncthreads();  // stage st ^ 1 was read by the previous step
       skinny_reg_q<ROWS>(a, nb, kend, Qs + (st ^ 1) * SKR_KR * SKR_ROWS);
-      skinny_reg_p(a, nb, kend, po0, po1, pn0, pn1, ko_next);
+      skinny_reg_p<KW>(nb, kend, s0, s1, pn, ko_next, quads);
       ko_next = skinny_reg_ko(a, nb + SKR_KR, kend);
       cp_async_wait<1>();
     } else {
@@ -979,31 +1043,26 @@ __device__ __forceinline__ void skinny_reg_job(const SkinnyArgs& a, const SkJob&
     const float* q = Qs + st * SKR_KR * SKR_ROWS;
 #pragma unroll
     for (int kk = 0; kk < SKR_KR; ++kk) {
-      float qv[ROWS];
+      const uint64_t w = f32x2_swap(pc[kk]);
 #pragma unroll
       for (int r = 0; r < ROWS; r += 4) {
-        const float4 t = *reinterpret_cast<const float4*>(q + kk * ROWS + r);
-        qv[r] = t.x; qv[r + 1] = t.y; qv[r + 2] = t.z; qv[r + 3] = t.w;
-      }
-#pragma unroll
-      for (int r = 0; r < ROWS; ++r) {
-        acc[0][r] = fmaf(qv[r], pc0[kk], acc[0][r]);
-        acc[1][r] = fmaf(qv[r], pc1[kk], acc[1][r]);
+        const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(q + kk * ROWS + r);
+        acc.v[r / 2][0] = fma_x2(t.x, pc[kk], acc.v[r / 2][0]);
+        acc.v[r / 2][1] = fma_x2(t.x, w, acc.v[r / 2][1]);
+        acc.v[r / 2 + 1][0] = fma_x2(t.y, pc[kk], acc.v[r / 2 + 1][0]);
+        acc.v[r / 2 + 1][1] = fma_x2(t.y, w, acc.v[r / 2 + 1][1]);
       }
     }
     if (nb < kend) {
 #pragma unroll
-      for (int kk = 0; kk < SKR_KR; ++kk) {
-        pc0[kk] = pn0[kk];
-        pc1[kk] = pn1[kk];
-      }
+      for (int kk = 0; kk < SKR_KR; ++kk) pc[kk] = pn[kk];
     }
     st ^= 1;
   }
   skinny_reg_finish<ROWS>(a, job, acc, os, cw, cs);
 }
 
-template <int ROWS, typename Resolve>
+template <int ROWS, bool KW, typename Resolve>
 __device__ __forceinline__ void skinny_reg_loop(int j0, int jstep, int njobs, Resolve&& resolve,
                                                 uint8_t* smem) {
   float* Qs = reinterpret_cast<float*>(smem);  // [2][KR][ROWS], stages SKR_ROWS rows apart
@@ -1019,23 +1078,24 @@ __device__ __forceinline__ void skinny_reg_loop(int j0, int jstep, int njobs, Re
     __syncthreads();  // the previous job's stores are done with os, pw, cw, cs
     skinny_reg_begin(a, job.b, pw, cw, cs);
     __syncthreads();
-    skinny_reg_job<ROWS>(a, job, Qs, os, pw, cw, cs);
+    skinny_reg_job<ROWS, KW>(a, job, Qs, os, pw, cw, cs);
   }
 }
 
 // ROWS = 16, or 8 for a narrow side of at most 8 (one kernel per row count:
 // both in one kernel would need more registers than four CTAs per SM leave)
-template <int ROWS>
+// KW: items whose stride-one index of P is contracted (SK_P_K).
+template <int ROWS, bool KW>
 __global__ void __launch_bounds__(SKR_THREADS, SKR_CTAS_PER_SM)
     skinny_reg_kernel(const __grid_constant__ SkinnyArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
   grid_dep_wait();
   auto resolve = [&](int J) { return SkRef{&a, J}; };
-  skinny_reg_loop<ROWS>(blockIdx.x, gridDim.x, a.njobs, resolve, smem);
+  skinny_reg_loop<ROWS, KW>(blockIdx.x, gridDim.x, a.njobs, resolve, smem);
   bulk_wait_all();  // bulk C copies complete before the CTA exits
 }
 
-template <int ROWS>
+template <int ROWS, bool KW>
 __global__ void __launch_bounds__(SKR_THREADS, SKR_CTAS_PER_SM)
     skinny_reg_group_kernel(const SkinnyItem* items, const int64_t* begin, int n, int njobs) {
   extern __shared__ __align__(16) uint8_t smem[];
@@ -1043,7 +1103,7 @@ __global__ void __launch_bounds__(SKR_THREADS, SKR_CTAS_PER_SM)
     const SkinnyItem& it = items[find_segment(begin, n, J)];
     return SkRef{&it.args, (int)(J - it.begin)};
   };
-  skinny_reg_loop<ROWS>(blockIdx.x, gridDim.x, njobs, resolve, smem);
+  skinny_reg_loop<ROWS, KW>(blockIdx.x, gridDim.x, njobs, resolve, smem);
   bulk_wait_all();
 }
 

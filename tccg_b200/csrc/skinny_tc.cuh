@@ -8,10 +8,15 @@
 // products run on the tensor cores:
 //
 //   warps 0-7   (256 threads): copy P's chunks of 32 k from the caller's
-//               tensor into a ring of FP32 staging slots ([k][position],
-//               the skinny kernel's copies, cp.async) as fast as slots free
-//               up; each thread's copies arrive on the slot's barrier as
-//               they land (cp.async.mbarrier.arrive);
+//               tensor into a ring of FP32 staging slots. 16-byte cp.async
+//               where four positions are consecutive and aligned; else 32
+//               loads per thread into registers, in flight while the slot
+//               frees up, then shared-memory stores: 4-byte cp.async moves at
+//               most 2.7 TB/s over 148 SMs whatever its pattern (13 cycles a
+//               warp instruction), the loads 5.1. Slots are [k][position],
+//               or [position][k] where P's stride-one index is contracted
+//               (pitch 33; 36 where rows of 4 k are aligned and move as
+//               16-byte loads): conflict-free for copies and conversion;
 //   warps 8-15  (256 threads, thread = box position = TMEM lane of its
 //               half): per chunk, split the position's 32 staged values into
 //               bf16 hi / lo and write them to its TMEM lane of the chunk's A
@@ -35,10 +40,9 @@
 //
 // Copies, conversion and MMAs run in separate warps: with one set of warps
 // issuing a chunk's copies, its Q load and its conversion in turn, a chunk
-// took 1.7-2.8 us against the 0.7 us of its HBM bytes (the copy pattern
-// alone streams at 4.9-6.6 TB/s).
+// took 1.7-2.8 us against the 0.7 us of its HBM bytes.
 //
-// One CTA per SM (216 KB of shared memory: five 33 KB staging slots, two
+// One CTA per SM (201 KB of shared memory: four 36 KB staging slots, two
 // 8 KB Q stages, the 33 KB epilogue staging and the offset tables; 25
 // warps); TMEM 512 columns (accumulators, running sums, A stages). Every
 // wait is bounded (TCCG_DEVICE_WAIT_NS): a wait that runs out records a
@@ -60,16 +64,22 @@ constexpr int SKT_EPI_THREADS = SK_BW;  // one position each: TMEM lane of its h
 constexpr int SKT_THREADS = SKT_COPY_THREADS + SKT_CONV_THREADS + 32 + SKT_EPI_THREADS;  // 800
 constexpr int SKT_SMAX = 64;   // rows per pass (a narrow side above 64 runs passes of 64)
 constexpr int SKT_HALF = 128;  // MMA rows: positions per half box
-constexpr int SKT_SLOTS = 5;   // FP32 staging ring
+constexpr int SKT_SLOTS = 2;   // FP32 staging ring
 constexpr int SKT_STAGES = 2;  // MMA operand stages (P in TMEM, Q in shared memory)
 constexpr size_t SKT_B_STAGE = (size_t)SKT_SMAX * 128;  // up to 64 Q rows x 128 B
-constexpr size_t SKT_SLOT = (size_t)SK_KC * SK_LDP * 4;
+// staging slot layouts: [k][position], pitch SK_LDP; [position][k], pitch
+// SKT_LDK (4-byte copies); or [position][32 k] with the 16-byte chunk c of
+// position w at c ^ (w % 8) (16-byte copies along k)
+enum SktLayout : int { SKT_W = 0, SKT_K = 1, SKT_K4 = 2 };
+constexpr int SKT_LDK = SK_KC + 1;
+constexpr size_t SKT_SLOT = (size_t)SK_BW * SKT_LDK * 4;
+static_assert(SKT_SLOT >= (size_t)SK_KC * SK_LDP * 4 && SKT_SLOT % 16 == 0, "either layout fits");
 constexpr size_t SKT_OFF_B = 0;
 constexpr size_t SKT_OFF_SLOT = SKT_OFF_B + SKT_STAGES * SKT_B_STAGE;
 constexpr size_t SKT_OFF_OS = SKT_OFF_SLOT + SKT_SLOTS * SKT_SLOT;
 constexpr size_t SKT_OFF_TAB = SKT_OFF_OS + (size_t)SK_SUB * SK_LDP * 4;
-// tables: pw[2][BW] (copy warps), cw[BW] and cs[SMAX] (epilogue)
-constexpr size_t SKT_OFF_BAR = SKT_OFF_TAB + (size_t)(3 * SK_BW + SKT_SMAX) * 4;
+// tables: pw[2 groups][2][BW] (copy warps), cw[BW] and cs[SMAX] (epilogue)
+constexpr size_t SKT_OFF_BAR = SKT_OFF_TAB + (size_t)(5 * SK_BW + SKT_SMAX) * 4;
 constexpr size_t SKT_SMEM_BYTES = 1024 + SKT_OFF_BAR + 24 * 8;
 // TMEM columns: accumulator b of half h at b * 2 SMAX + h SMAX, the job's
 // running sums of half h at SKT_SUMCOL + h SMAX, and the converted P (the
@@ -111,7 +121,8 @@ __device__ __forceinline__ bool skt_inside(const SkinnyArgs& a, int b, int w) {
   return w < a.tx * a.ty && ix * a.tx + xl < a.ex && iy * a.ty + yl < a.ey;
 }
 
-// Box position w's P offset (loaders) / C offset (epilogue); SK_NONE outside.
+// Box position w's P offset (copies: skinny_p_off) / C offset (epilogue;
+// SK_NONE outside).
 __device__ __forceinline__ int32_t skt_box(const SkinnyArgs& a, int b, int w, bool c) {
   const int ix = a.bxn == 1 ? 0 : b % a.bxn, iy = a.bxn == 1 ? b : b / a.bxn;
   int xl, yl;
@@ -123,8 +134,8 @@ __device__ __forceinline__ int32_t skt_box(const SkinnyArgs& a, int b, int w, bo
     yl = w / a.tx;
   }
   const int x = ix * a.tx + xl, y = iy * a.ty + yl;
-  const bool ok = w < a.tx * a.ty && x < a.ex && y < a.ey;
-  return !ok ? SK_NONE : c ? x * a.cx + __ldg(a.c_y_off + y) : x * a.px + __ldg(a.p_y_off + y);
+  if (!c) return skinny_p_off(a, ix, iy, xl, yl, a.p_walk == SK_P_K);
+  return w < a.tx * a.ty && x < a.ex && y < a.ey ? x * a.cx + __ldg(a.c_y_off + y) : SK_NONE;
 }
 
 __device__ __forceinline__ void skt_epi_sync() { named_barrier_sync(2, SKT_EPI_THREADS); }
@@ -145,23 +156,111 @@ __device__ __forceinline__ bool skt_epi_and(bool v) {
   return out != 0;
 }
 
-// Converts position w's column of a staging slot ([k][position], k < kc
-// valid) into its TMEM lane of an A stage (ta: the warp's lane quarter, the
-// stage and half's first column): hi = bf16(x) in 16 columns, then lo =
-// bf16(x - hi) in 16, two k per column (the lower k in the low half); k past
-// kc, and every k of a position outside the tensor (kc = 0: the copies skip
-// it), are zeros. Warp-collective (tcgen05.st).
-__device__ __forceinline__ void skt_convert(const float* slot, uint32_t ta, int w, int kc) {
-  // shared-window addresses: the reads stay shared-memory loads
-  const uint32_t src = smem_u32(slot + w);
-  uint32_t hw[16], lw[16];
+template <typename A>
+__device__ __forceinline__ int skt_layout(const A& a) {
+  return a.p_walk != SK_P_K ? SKT_W : a.p_vec ? SKT_K4 : SKT_K;
+}
+
+// Loads that stay where they are written, in flight across the wait for a
+// slot (the compiler moves ordinary read-only loads down to their stores,
+// where each waits for memory: 7 us a chunk instead of 1).
+__device__ __forceinline__ float skt_ldg(const float* p) {
+  float x;
+  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(x) : "l"(p));
+  return x;
+}
+__device__ __forceinline__ float4 skt_ldg4(const float* p) {
+  float4 x;
+  asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w)
+               : "l"(p));
+  return x;
+}
+
+// The copies of half a chunk (128 of the box's positions) through registers, by
+// the 128 threads of a copy group. load(): thread t's 32 values of the half
+// whose offsets pw holds, with lanes along k (SKT_K: positions t >> lg + i * 128
+// >> lg; SKT_K4: 16-byte quads of k, 8 lanes a position). store(): into the
+// slot. ko = skinny_p_ko's offset for this lane. No load is predicated (25
+// warps share the instruction caches; the shorter code is the faster): a
+// position outside the tensor has the offset of one inside in pw and a k past
+// K offset 0 in ko, so its load reads some element of P, which the conversion
+// replaces by zero.
+struct SktHalf {
+  float v[SK_KC];
+  __device__ __forceinline__ void load(const SkPFields& a, int lay, int t, const int32_t* pw,
+                                       int32_t ko) {
+    const int lane = t & 31;
+    if (lay == SKT_K) {
+      const int lg = a.kr_log2;
+      const float* src = a.P + ko;
+#pragma unroll
+      for (int i = 0; i < SK_KC; ++i)  // lg < 5: repeats positions
+        v[i] = skt_ldg(src + pw[((t >> lg) + i * (SKT_HALF >> lg)) & (SKT_HALF - 1)]);
+    } else {
+      const float* src = a.P + __shfl_sync(0xffffffffu, ko, 4 * (lane & 7));
+#pragma unroll
+      for (int i = 0; i < SK_KC / 4; ++i) {
+        const float4 x = skt_ldg4(src + pw[(t >> 3) + i * (SKT_HALF / 8)]);
+        v[4 * i] = x.x; v[4 * i + 1] = x.y; v[4 * i + 2] = x.z; v[4 * i + 3] = x.w;
+      }
+    }
+  }
+  __device__ __forceinline__ void store(const SkPFields& a, int lay, int t, float* slot) const {
+    const int lane = t & 31;
+    if (lay == SKT_K) {
+      const int lg = a.kr_log2;
+      float* d = slot + (t & ((1 << lg) - 1));
+#pragma unroll
+      for (int i = 0; i < SK_KC; ++i)
+        d[(((t >> lg) + i * (SKT_HALF >> lg)) & (SKT_HALF - 1)) * SKT_LDK] = v[i];
+    } else {
+      float* d = slot + (t >> 3) * SK_KC + 4 * ((lane ^ (t >> 3)) & 7);
+#pragma unroll
+      for (int i = 0; i < SK_KC / 4; ++i)
+        *reinterpret_cast<float4*>(d + i * (SKT_HALF / 8) * SK_KC) =
+            make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+    }
+  }
+};
+
+// hi and lo of 32 staged values STEP bytes apart (zeros from kc on).
+template <int STEP>
+__device__ __forceinline__ void skt_split_lds(uint32_t src, int kc, uint32_t (&hw)[16],
+                                              uint32_t (&lw)[16]) {
 #pragma unroll
   for (int e = 0; e < SK_KC; e += 2) {
     float x0 = 0.0f, x1 = 0.0f;
-    if (e < kc) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x0) : "r"(src + e * SK_LDP * 4));
-    if (e + 1 < kc)
-      asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x1) : "r"(src + (e + 1) * SK_LDP * 4));
+    if (e < kc) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x0) : "r"(src + e * STEP));
+    if (e + 1 < kc) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x1) : "r"(src + (e + 1) * STEP));
     split_bf16x2(x0, x1, hw[e / 2], lw[e / 2]);
+  }
+}
+
+// Converts position w's values of a staging slot (k < kc
+// valid) into its TMEM lane of an A stage (ta: the warp's lane quarter, the
+// stage and half's first column): hi = bf16(x) in 16 columns, then lo =
+// bf16(x - hi) in 16, two k per column (the lower k in the low half); k past
+// kc, and every k of a position outside the tensor (kc = 0), are zeros. Warp-collective (tcgen05.st).
+__device__ __forceinline__ void skt_convert(const float* slot, int lay, uint32_t ta, int w, int kc) {
+  // shared-window addresses: the reads stay shared-memory loads
+  uint32_t hw[16], lw[16];
+  if (lay == SKT_K4) {
+    const uint32_t src = smem_u32(slot + w * SK_KC);
+#pragma unroll
+    for (int e = 0; e < SK_KC; e += 4) {
+      float x[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      if (e < kc)  // quads are whole
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3])
+                     : "r"(src + (((e >> 2) ^ (w & 7)) << 4)));
+      split_bf16x2(x[0], x[1], hw[e / 2], lw[e / 2]);
+      split_bf16x2(x[2], x[3], hw[e / 2 + 1], lw[e / 2 + 1]);
+    }
+  } else if (lay == SKT_W) {
+    skt_split_lds<SK_LDP * 4>(smem_u32(slot + w), kc, hw, lw);
+  } else {
+    skt_split_lds<4>(smem_u32(slot + w * SKT_LDK), kc, hw, lw);
   }
   tmem_st_32x32b_x16(ta, hw);
   tmem_st_32x32b_x16(ta + 16, lw);
@@ -264,8 +363,8 @@ __device__ __forceinline__ void skinny_tc_body(int njobs, Resolve&& resolve, int
   uint8_t* sB = smem + SKT_OFF_B;
   float* slots = reinterpret_cast<float*>(smem + SKT_OFF_SLOT);
   float* os = reinterpret_cast<float*>(smem + SKT_OFF_OS);
-  int32_t* pw = reinterpret_cast<int32_t*>(smem + SKT_OFF_TAB);  // [2][BW]
-  int32_t* cw = pw + 2 * SK_BW;                                  // [BW]
+  int32_t* pw = reinterpret_cast<int32_t*>(smem + SKT_OFF_TAB);  // [2][2][BW]
+  int32_t* cw = pw + 4 * SK_BW;                                  // [BW]
   int32_t* cs = cw + SK_BW;                                      // [SMAX]
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SKT_OFF_BAR);
   uint64_t* full = bars;                    // [STAGES] P stage converted + Q landed
@@ -286,7 +385,7 @@ __device__ __forceinline__ void skinny_tc_body(int njobs, Resolve&& resolve, int
       mbar_init(&empty[s], 1);
     }
     for (int s = 0; s < SKT_SLOTS; ++s) {
-      mbar_init(&sfull[s], SKT_COPY_THREADS);  // each copy thread, when its copies landed
+      mbar_init(&sfull[s], SKT_HALF);  // each thread of a copy group, when its copies landed
       mbar_init(&sempty[s], SKT_CONV_THREADS);
     }
     for (int b = 0; b < 2; ++b) {
@@ -307,7 +406,10 @@ __device__ __forceinline__ void skinny_tc_body(int njobs, Resolve&& resolve, int
 
   if (warp < SKT_CONV_WARP0) {
     // ---------------- copy warps ----------------
-    const int tid = threadIdx.x;
+    // two groups of four warps take the CTA's chunks in turn, so that one
+    // group's waits and table loads run under the other's copies
+    const int grp = warp >> 2, t = threadIdx.x & (SKT_HALF - 1);
+    int32_t* const gpw = pw + grp * 2 * SK_BW;  // [2][BW]
     // job ig, chunk ic of [.., ic1), its box offsets slot and the k offset
     // its next copies start from (loaded a chunk ahead: the copies would
     // otherwise wait for the table load)
@@ -328,31 +430,57 @@ __device__ __forceinline__ void skinny_tc_body(int njobs, Resolve&& resolve, int
         inew = true;
       }
     };
+    auto inext = [&](int n) {  // n chunks on
+      while (n > 0 && ig < njobs) {
+        const int d = ic1 - ic < n ? ic1 - ic : n;
+        ic += d;
+        n -= d;
+        if (ic >= ic1) {
+          ig += js;
+          iseek();
+        }
+      }
+    };
     iseek();
+    inext(grp);
     if (ig < njobs) iko = skinny_p_ko(ipf, ic);
-    int slot = 0;
-    uint32_t sphase = 0;
+    int slot = grp % SKT_SLOTS;
+    uint32_t sphase = (uint32_t)(grp / SKT_SLOTS);
     while (ig < njobs) {
+      const int lay = skt_layout(ipf);
+      const bool async = lay == SKT_W;  // cp.async
+      if (inew) {  // the other box slot is no longer read: its job's copies were issued
+        ipw ^= 1;
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          gpw[ipw * SK_BW + t + h * SKT_HALF] = skt_box(*ia, ib, t + h * SKT_HALF, false);
+        named_barrier_sync(grp ? 3 : 1, SKT_HALF);  // walks read other threads' offsets
+        inew = false;
+      }
+      const int32_t* const bpw = gpw + ipw * SK_BW;
+      SktHalf hf;
+      if (!async) hf.load(ipf, lay, t, bpw, iko);  // in flight during the wait
       if (!mbar_wait(&sempty[slot], sphase ^ 1, wait_ns)) {
         record_error(status, 1);
         break;
       }
-      if (inew) {  // the other box slot is no longer read: its job's copies were issued
-        ipw ^= 1;
-        pw[ipw * SK_BW + tid] = skt_box(*ia, ib, tid, false);
-        named_barrier_sync(1, SKT_COPY_THREADS);  // walks read other threads' offsets
-        inew = false;
+      float* const ps = slots + slot * (SKT_SLOT / 4);
+      if (async) {
+        skinny_issue_p<SKT_HALF>(ipf, ic, ps, bpw, iko, t);
+        cp_async_mbar_arrive(&sfull[slot]);
+      } else {
+        const int pitch = lay == SKT_K ? SKT_LDK : SK_KC;
+        hf.store(ipf, lay, t, ps);
+        hf.load(ipf, lay, t, bpw + SKT_HALF, iko);
+        hf.store(ipf, lay, t, ps + SKT_HALF * pitch);
+        mbar_arrive(&sfull[slot]);
       }
-      skinny_issue_p<true>(ipf, ic, slots + slot * (SKT_SLOT / 4), pw + ipw * SK_BW, iko);
-      cp_async_mbar_arrive(&sfull[slot]);
-      if (++slot == SKT_SLOTS) {
-        slot = 0;
+      slot += 2;
+      while (slot >= SKT_SLOTS) {
+        slot -= SKT_SLOTS;
         sphase ^= 1;
       }
-      if (++ic >= ic1) {
-        ig += js;
-        iseek();
-      }
+      inext(2);
       if (ig < njobs) iko = skinny_p_ko(ipf, ic);
     }
     cp_async_wait<0>();  // no copy in flight when the copy warps leave
@@ -360,7 +488,7 @@ __device__ __forceinline__ void skinny_tc_body(int njobs, Resolve&& resolve, int
     // ---------------- converters ----------------
     const int w = threadIdx.x - SKT_COPY_THREADS;  // the thread's box position
     int cg = j0, cc = 0, cc1 = 0, cq = 0;  // cq: the job's first Q row (its pass)
-    int cK = 0, cspad = 0;  // the item's K and rows per pass, read once per job
+    int cK = 0, cspad = 0, clay = 0;  // the item's K, rows per pass and slot layout, read once per job
     bool inside = false;  // the position is inside the tensor (else the copies skip it)
     SktRef cr{};
     auto cseek = [&]() {
@@ -371,6 +499,7 @@ __device__ __forceinline__ void skinny_tc_body(int njobs, Resolve&& resolve, int
         cc1 = jb.c1;
         cK = cr.a->sk.K;
         cspad = cr.a->spad;
+        clay = skt_layout(cr.a->sk);
         cq = jb.p * cspad;
         inside = skt_inside(cr.a->sk, jb.b, w);
       }
@@ -392,7 +521,7 @@ __device__ __forceinline__ void skinny_tc_body(int njobs, Resolve&& resolve, int
         break;
       }
       tc_fence_after();  // the stage's MMAs (waited for above) are done with its TMEM columns
-      skt_convert(slots + slot * (SKT_SLOT / 4),
+      skt_convert(slots + slot * (SKT_SLOT / 4), clay,
                   tbase + ((uint32_t)((warp & 3) * 32) << 16) +
                       (uint32_t)(SKT_ACOL + stage * 64 + (w / SKT_HALF) * 32),
                   w, inside ? (cK - cc * SK_KC < SK_KC ? cK - cc * SK_KC : SK_KC) : 0);

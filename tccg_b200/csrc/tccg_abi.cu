@@ -668,6 +668,11 @@ static bool skinny_geometry(tccg_plan* p, std::vector<int>& ym, int* xmode, bool
   bool k4 = true;
   for (int64_t v : t) k4 &= v % 4 == 0;
   p->sk_p_vec = a.p_walk == SK_P_X && a.px == 1 && k4;
+  // P's stride-one index contracted: quads of k as 16-byte loads (the run
+  // checks P's alignment); on the register path only for 8 chunks and more
+  // (S = 9, K = 168: 811 us with them off, 830 on)
+  if (a.p_walk == SK_P_K)
+    p->sk_p_vec = (sn ? p->ks_a : p->ks_b) && p->K % 4 == 0 && (tc || a.nchunks >= 8);
   build_offsets(nsm, sext, sc, t);
   auto affine = [&](int64_t st) {
     for (size_t i = 0; i < t.size(); ++i)
@@ -743,14 +748,12 @@ static bool choose_skinny_tc(const tccg_plan* p) {
       t.tile_n != 0 || t.ksplit != 0)
     return false;
   // a narrow side of at most 16 takes the CUDA-core register path instead
-  // (choose_skinny): on the 8 such items 1.36 ms in sum against 1.50 ms here
-  // -- except where P's stride-one index is contracted and K spans at least
-  // 8 chunks: the register path's loads (16 consecutive k per lane) then
-  // touch 32 rows per warp load (items 40 / 48 of the 256-item batched
-  // workload: 0.21 / 0.31 ms there, 0.20 / 0.25 ms here)
-  if (p->K > SK_KC && p->sk.nblk >= 48 && p->sk.S <= 16 && p->sk.p_walk == SK_P_K &&
-      p->sk.nchunks >= 8)
-    return true;
+  // (choose_skinny; 12 x 21 boxes of S = 11, K = 2744: 453 us against 469
+  // here, S = 13, K = 3240: 197 / 225) -- except where P's stride-one index is
+  // contracted: the register path's loads (16 consecutive k per lane) then
+  // touch 32 rows per warp load (S = 8, K = 1024: 283 us against 143; S = 8,
+  // K = 720: 1412 / 513; S = 9, K = 168: 777 / 629)
+  if (p->K > SK_KC && p->sk.nblk >= 48 && p->sk.S <= 16 && p->sk.p_walk == SK_P_K) return true;
   return p->K > SK_KC && p->sk.nblk >= 48 && p->sk.S > 16 && p->sk.S <= SKT_SMAX;
 }
 
@@ -1493,11 +1496,17 @@ static cudaError_t set_attrs() {
                            (int)SKT_SMEM_BYTES));
   chk(cudaFuncSetAttribute(skinny_tc_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)SKT_SMEM_BYTES));
-  chk(cudaFuncSetAttribute(skinny_reg_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  chk(cudaFuncSetAttribute(skinny_reg_kernel<8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)SKR_SMEM_BYTES));
-  chk(cudaFuncSetAttribute(skinny_reg_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  chk(cudaFuncSetAttribute(skinny_reg_kernel<8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)SKR_SMEM_BYTES));
-  chk(cudaFuncSetAttribute(skinny_reg_group_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  chk(cudaFuncSetAttribute(skinny_reg_kernel<16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)SKR_SMEM_BYTES));
+  chk(cudaFuncSetAttribute(skinny_reg_kernel<16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)SKR_SMEM_BYTES));
+  chk(cudaFuncSetAttribute(skinny_reg_group_kernel<16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)SKR_SMEM_BYTES));
+  chk(cudaFuncSetAttribute(skinny_reg_group_kernel<16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)SKR_SMEM_BYTES));
   chk(cudaFuncSetAttribute(skinny_reduce_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)SK_SMEM_BYTES));
@@ -2155,7 +2164,10 @@ static int run_skinny(const tccg_plan* p, const void* GA, const void* GB, float*
   if (p->sk_reg) {
     const int64_t grid = std::min<int64_t>(a.njobs, (int64_t)SKR_CTAS_PER_SM * p->num_sms);
     // 8 computed rows for a narrow side of at most 8, else 16
-    launch_after(false, p, a.S <= 8 ? skinny_reg_kernel<8> : skinny_reg_kernel<16>,
+    const bool kw = a.p_walk == SK_P_K;
+    launch_after(false, p,
+                 a.S <= 8 ? (kw ? skinny_reg_kernel<8, true> : skinny_reg_kernel<8, false>)
+                          : (kw ? skinny_reg_kernel<16, true> : skinny_reg_kernel<16, false>),
                  dim3((unsigned)grid), dim3(SKR_THREADS), SKR_SMEM_BYTES, s, a);
   } else {
     const int64_t grid = std::min<int64_t>(a.njobs, (int64_t)SK_CTAS_PER_SM * p->num_sms);
@@ -2431,6 +2443,13 @@ extern "C" int tccg_transpose(int32_t dtype, int32_t dim, const int32_t* perm,
 // --------------------------------------------------------------------------
 // grouped launches
 // --------------------------------------------------------------------------
+// Lane of a CUDA-core skinny item: its rows per thread (4, 8 or 12), and one
+// for the register path on items whose P has its stride-one index contracted.
+static constexpr int SK_CLASSES = 4;
+static int skinny_class(const tccg_plan* p) {
+  return p->sk_reg && p->sk.p_walk == SK_P_K ? 3 : p->sk.rs / 4 - 1;
+}
+
 struct tccg_group {
   std::vector<const tccg_plan*> plans;
   int32_t prec = 0, dtype = 0;
@@ -2488,11 +2507,11 @@ struct tccg_group {
     int32_t tcj0 = 0, ntcj = 0;  // pack jobs of the packed-operand lanes (two per item)
     int64_t simt_tiles = 0, simt_pack_ctas = 0, tc_pack_ctas = 0, red_ctas = 0;
     int32_t fb0 = 0;  // the TCV_F32X6 lane's items are [fb0, fb0 + nlane) of d_fb / d_range
-    // skinny lanes, one per rows-per-thread class (rs / 4 - 1: 4, 8, 12): items
-    // [sk0[c], sk0[c] + nsk[c]) of d_sk with sk_jobs[c] jobs; reductions
-    int32_t sk0[3] = {}, nsk[3] = {}, skr0 = 0, nskr = 0;
-    int64_t sk_jobs[3] = {}, skr_ctas = 0;
-    bool sk_reg[3] = {};  // the lane runs the register path
+    // skinny lanes, one per class (skinny_class): items [sk0[c], sk0[c] +
+    // nsk[c]) of d_sk with sk_jobs[c] jobs; reductions
+    int32_t sk0[SK_CLASSES] = {}, nsk[SK_CLASSES] = {}, skr0 = 0, nskr = 0;
+    int64_t sk_jobs[SK_CLASSES] = {}, skr_ctas = 0;
+    bool sk_reg[SK_CLASSES] = {};  // the lane runs the register path
     // the tensor-core skinny lane: items [sktc0, sktc0 + nsktc) of d_sktc
     int32_t sktc0 = 0, nsktc = 0;
     int64_t sktc_jobs = 0;
@@ -2582,14 +2601,14 @@ extern "C" int tccg_group_create(const tccg_plan* const* plans, int32_t count, t
     if (p->sk_tc) {
       wv.sktc_jobs += p->sk.njobs;
     } else if (p->skinny) {
-      wv.sk_jobs[p->sk.rs / 4 - 1] += p->sk.njobs;
+      wv.sk_jobs[skinny_class(p)] += p->sk.njobs;
     } else if (simt_path(p)) {
       wv.simt_tiles += (p->Mp / p->simt_bm) * (p->Np / p->simt_bn) * p->ksplit;
     } else {
       wv.lane_tiles[p->tcv] += (int64_t)p->tiles_m * p->tiles_n * p->ksplit;
     }
     bool too_many = wv.simt_tiles > INT32_MAX || wv.sktc_jobs > INT32_MAX;
-    for (int c = 0; c < 3; ++c) too_many |= wv.sk_jobs[c] > INT32_MAX;
+    for (int c = 0; c < SK_CLASSES; ++c) too_many |= wv.sk_jobs[c] > INT32_MAX;
     for (int v = 0; v < TCV_COUNT; ++v) too_many |= wv.lane_tiles[v] > INT32_MAX;
     if (too_many) {
       group_free(g);
@@ -2865,11 +2884,11 @@ static void bind_skinny(tccg_group* g, tccg_group::Wave& wv, const void* const* 
                         std::vector<SkinnyItem>& red) {
   wv.skr0 = (int32_t)red.size();
   int64_t rctas = 0;
-  for (int cls = 0; cls < 3; ++cls) {
+  for (int cls = 0; cls < SK_CLASSES; ++cls) {
     wv.sk0[cls] = (int32_t)items.size();
     std::vector<size_t> idx;
     for (size_t i : wv.items)
-      if (g->plans[i]->skinny && !g->plans[i]->sk_tc && g->plans[i]->sk.rs / 4 - 1 == cls)
+      if (g->plans[i]->skinny && !g->plans[i]->sk_tc && skinny_class(g->plans[i]) == cls)
         idx.push_back(i);
     std::stable_sort(idx.begin(), idx.end(), [&](size_t a, size_t b) {
       return g->plans[a]->sk.chunks_per_split > g->plans[b]->sk.chunks_per_split;
@@ -3065,7 +3084,7 @@ static int run_wave(const tccg_group* g, const tccg_group::Wave& wv, cudaStream_
   const dim3 blk(32, 8);
   const int sj = 2 * wv.n_simt, tj = wv.ntcj;
   bool skinny_side = false;
-  for (int cls = 0; cls < 3; ++cls) skinny_side |= wv.nsk[cls] > 0;
+  for (int cls = 0; cls < SK_CLASSES; ++cls) skinny_side |= wv.nsk[cls] > 0;
   const bool simt_side = wv.n_simt > 0;
   cudaStream_t s_sk = skinny_side ? g->side[0] : s, s_simt = simt_side ? g->side[1] : s;
   if (skinny_side || simt_side) {
@@ -3096,7 +3115,7 @@ static int run_wave(const tccg_group* g, const tccg_group::Wave& wv, cudaStream_
   }
   // CUDA-core skinny lanes on theirs
   if constexpr (sizeof(T) == 4) {
-    for (int cls = 0; cls < 3; ++cls) {
+    for (int cls = 0; cls < SK_CLASSES; ++cls) {
       if (wv.nsk[cls] == 0) continue;
       if (wv.sk_reg[cls]) {  // the register path (its items all take it)
         // one launch of 16 computed rows for all of them: splitting the lane
@@ -3106,7 +3125,8 @@ static int run_wave(const tccg_group* g, const tccg_group::Wave& wv, cudaStream_
         // item alone
         const unsigned grid =
             (unsigned)std::min<int64_t>(wv.sk_jobs[cls], (int64_t)SKR_CTAS_PER_SM * g->num_sms);
-        skinny_reg_group_kernel<16><<<grid, SKR_THREADS, SKR_SMEM_BYTES, s_sk>>>(
+        auto kernel = cls == 3 ? skinny_reg_group_kernel<16, true> : skinny_reg_group_kernel<16, false>;
+        kernel<<<grid, SKR_THREADS, SKR_SMEM_BYTES, s_sk>>>(
             g->d_sk + wv.sk0[cls], g->b_sk + wv.sk0[cls], wv.nsk[cls], (int)wv.sk_jobs[cls]);
       } else {
         const unsigned grid =
