@@ -1090,8 +1090,9 @@ __global__ void __launch_bounds__(256) simt_reduce_kernel(const T* __restrict__ 
                                                           int64_t M, int64_t N, T* C,
                                                           const int64_t* c_m_off,
                                                           const int64_t* c_n_off, T alpha,
-                                                          T beta) {
+                                                          T beta, const uint32_t* range, int K) {
   grid_dep_wait();  // partial sums written by the GETT kernel before
+  if (range && !f32_split_exact(range, K)) return;  // computed by f32_fallback_kernel
   const int64_t m = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (m >= M) return;
   const int64_t cmo = c_m_off[m];
@@ -1120,6 +1121,8 @@ struct ReduceJob {
   int64_t begin;
   int32_t splits, mblocks;
   int32_t ncols;  // columns per CTA: fewer when there are many slices
+  int32_t K;
+  const uint32_t* range;  // FP32 on the tensor cores: the item's range words, or null
 };
 
 template <typename T>
@@ -1127,6 +1130,7 @@ __global__ void __launch_bounds__(256) reduce_group_kernel(const ReduceJob<T>* j
                                                            const int64_t* begin, int n_jobs) {
   const int64_t t = blockIdx.x;
   const ReduceJob<T> j = jobs[find_segment(begin, n_jobs, t)];  // fields loaded up front
+  if (j.range && !f32_split_exact(j.range, j.K)) return;  // computed by f32_fallback_group_kernel
   const int64_t local = t - j.begin;
   const int64_t m = (local % j.mblocks) * 256 + threadIdx.x;
   if (m >= j.M) return;

@@ -1084,7 +1084,7 @@ __device__ __forceinline__ void skinny_reg_loop(int j0, int jstep, int njobs, Re
 
 // ROWS = 16, or 8 for a narrow side of at most 8 (one kernel per row count:
 // both in one kernel would need more registers than four CTAs per SM leave)
-// KW: items whose stride-one index of P is contracted (SK_P_K).
+// KW: items with quads of k (SK_P_K).
 template <int ROWS, bool KW>
 __global__ void __launch_bounds__(SKR_THREADS, SKR_CTAS_PER_SM)
     skinny_reg_kernel(const __grid_constant__ SkinnyArgs a) {

@@ -241,6 +241,8 @@ static int choose_simt_shape(const tccg_plan* p, double* padded_work) {
 }
 
 static bool direct_eligible(const tccg_plan* p, int shape);
+static int64_t choose_ksplit(int32_t requested, int64_t tiles, int64_t kblocks, int64_t slots,
+                             int64_t min_kb, int32_t* splits);
 static bool unit_first(int n, const int64_t* ext, const int64_t* str);
 
 // The gather loader of the tcgen05 BF16X3 kernel (TC_LOAD_GATHER) can serve
@@ -302,16 +304,19 @@ static double simt_time(const tccg_plan* p) {
 // against FP64 on N(0, 1) values is below FFMA's at every K measured (K = 64:
 // 0.7e-7 against 1.4e-7, 256: 1.2e-7 / 2.9e-7, 1024: 1.3e-7 / 5.7e-7, 4096:
 // 1.6e-7 / 1.15e-6; the same order for uniform and for wide-ranged values),
-// so time decides: tiles of 128 x 160 at 0.72 us per 32 k and round of the
-// persistent grid (half rounds where the tail split applies), the pack's 4 + 6
-// and the loads' 6 bytes per element at 4.5 TB/s and 20 us of launches,
-// against FFMA at 45 TFLOP/s on padded tiles. 2048 x 2080 x K, us: K = 128
-// 31.8 against 35.6 (both near the launch floor; the rule keeps FFMA), 256: 38
-// / 59, 512: 54 / 106, 4096: 228 / 773. Half a round of tiles at least (no
-// k-split here). A tuning that names a CUDA-core form (variant < 0, direct,
-// shortk, simt_tile, an explicit k-split) keeps the CUDA cores; variant > 0
-// asks for this path.
+// so time decides: tiles of 128 x 160 (the MMAs of one column of tiles only as
+// wide as N) at 0.72 us per 32 k and round of the persistent grid (half rounds
+// where the tail split applies), the pack's 4 + 6 and the loads' 6 bytes per
+// element at 4.5 TB/s, the k-split's partial sums and 20 us of launches,
+// against FFMA at 45 TFLOP/s on padded tiles with its own operand passes and 8
+// us. 2048 x 2080 x K, us: K = 128 31.8 against 35.6 (both near the launch
+// floor; the rule keeps FFMA), 256: 38 / 59, 512: 54 / 106, 4096: 228 / 773.
+// Plans for groups (tail_split < 0) share their launches: 5 us. With a
+// k-split the model is less sure of both sides: by 1.25x at least. A tuning that
+// names a CUDA-core form (variant < 0, direct, shortk, simt_tile, an explicit
+// k-split) keeps the CUDA cores; variant > 0 asks for this path.
 static constexpr int64_t F32X6_MIN_K = 128;  // an accumulation chunk
+static constexpr int64_t F32X6_MIN_KB = 8;   // k-blocks of a k-split slice
 static constexpr int F32X6_BM = TcCfgT<TC_F32X6>::BM, F32X6_BN = TcCfgT<TC_F32X6>::BN;
 static bool choose_f32x6(const tccg_plan* p) {
   const tccg_tuning& t = p->tune;
@@ -321,14 +326,25 @@ static bool choose_f32x6(const tccg_plan* p) {
   const int64_t lim = int64_t(1) << 30;
   if (p->M >= lim || p->N >= lim || p->K >= lim) return false;
   if (t.variant > 0) return true;
-  const int64_t tiles = cdiv(p->M, F32X6_BM) * cdiv(p->N, F32X6_BN);
-  if (p->K < F32X6_MIN_K || 2 * tiles < p->num_sms) return false;
-  const double rounds = std::max(1.0, 0.5 * (double)cdiv(2 * tiles, p->num_sms));
-  const double K = (double)p->K;
-  const double t_tc = rounds * (K / 32) * 0.72e-6 +
-                      (double)(p->M + p->N) * K * 16.0 / 4.5e12 + 20e-6;
-  const double t_ffma = 2.0 * (double)round_up(p->M, 128) * (double)round_up(p->N, 128) * K / 45e12;
-  return t_tc < t_ffma;
+  if (p->K < F32X6_MIN_K) return false;
+  const int64_t tiles = cdiv(p->M, F32X6_BM) * cdiv(p->N, F32X6_BN), kb = cdiv(p->K, 32);
+  int32_t split = 1;
+  const int64_t per =
+      choose_ksplit(t.ksplit, tiles, kb, p->num_sms, F32X6_MIN_KB, &split);
+  const double rounds =
+      split > 1 ? 1.0 : std::max(1.0, 0.5 * (double)cdiv(2 * tiles, p->num_sms));
+  const double width =
+      p->N >= F32X6_BN ? 1.0 : std::max(0.4, (double)round_up(p->N, 32) / F32X6_BN);
+  const double M = (double)p->M, N = (double)p->N, K = (double)p->K;
+  double t_tc = rounds * (double)per * 0.72e-6 * width + (M + N) * K * 16.0 / 4.5e12 +
+                (t.tail_split < 0 ? 5e-6 : 20e-6);
+  if (split > 1) t_tc += 8.0 * split * M * N / 3e12 + 3e-6;
+  double work = 0;
+  const int shape = choose_simt_shape(p, &work);
+  const double t_ffma = 2.0 * work * K / 45e12 +
+                        (direct_eligible(p, shape) ? 4.0 : 12.0) * (M + N) * K / 4.5e12 +
+                        (t.tail_split < 0 ? 2e-6 : 8e-6);
+  return (split > 1 || 2 * tiles < p->num_sms ? 1.25 : 1.0) * t_tc < t_ffma;
 }
 
 static bool choose_simt(const tccg_plan* p) {
@@ -1257,8 +1273,8 @@ static int plan_layout(tccg_plan* p) {
     int ctas = p->tune.max_ctas > 0 ? std::min(p->tune.max_ctas, p->num_sms) : p->num_sms;
     // one CTA per SM; a slice is at least one accumulation chunk (BF16X3) or
     // 512 k (BF16). The CTA-pair kernel does not split.
-    p->kb_per_split = (int32_t)choose_ksplit(pair || x6 ? 1 : p->tune.ksplit, tiles, p->num_kb, ctas,
-                                             x3 ? p->chunk_kb : 8, &p->ksplit);
+    p->kb_per_split = (int32_t)choose_ksplit(pair ? 1 : p->tune.ksplit, tiles, p->num_kb, ctas,
+                                             x3 ? p->chunk_kb : x6 ? F32X6_MIN_KB : 8, &p->ksplit);
     tiles *= p->ksplit;
     // Tail split: whole rounds of the persistent grid plus a short tail (at
     // most half a round) -- the tail's tiles run as k slices that fill the
@@ -1884,7 +1900,7 @@ static int run_simt(const tccg_plan* p, const void* GA, const void* GB, T* Cout,
     dim3 g2((unsigned)cdiv(p->M, 256), (unsigned)std::min<int64_t>(p->N, 65535));
     mark(2, 0, s);
     launch_after(true, p, simt_reduce_kernel<T>, g2, dim3(256), 0, s, a.partial, (int)p->ksplit,
-                 p->Mp, p->Np, p->M, p->N, Cout, c_m, c_n, alpha, beta);
+                 p->Mp, p->Np, p->M, p->N, Cout, c_m, c_n, alpha, beta, (const uint32_t*)nullptr, 0);
     mark(2, 1, s);
     rc = launch_check("simt_reduce");
   }
@@ -2006,7 +2022,7 @@ static int tc_reduce(const tccg_plan* p, const TcArgs& a, float* Cout, const int
   mark(2, 0, s);
   launch_after(true, p, simt_reduce_kernel<float>, g2, dim3(256), 0, s, (const float*)a.partial,
                (int)p->ksplit, (int64_t)p->M, (int64_t)p->N, (int64_t)p->M, (int64_t)p->N, Cout, c_m,
-               c_n, alpha, beta);
+               c_n, alpha, beta, a.range, (int)p->K);
   mark(2, 1, s);
   return launch_check("tc_reduce");
 }
@@ -2156,6 +2172,12 @@ static int run_skinny_tc(const tccg_plan* p, const void* GA, const void* GB, flo
   return rc;
 }
 
+// The register path with 16-byte loads along k (its own kernel; an operand off
+// a 16-byte boundary is read element by element there).
+static bool reg_quads(const tccg_plan* p) {
+  return p->sk_reg && p->sk.p_walk == SK_P_K && p->sk_p_vec;
+}
+
 static int run_skinny(const tccg_plan* p, const void* GA, const void* GB, float* C, float alpha,
                       float beta, char* w, cudaStream_t s) {
   if (p->sk_tc) return run_skinny_tc(p, GA, GB, C, alpha, beta, w, s);
@@ -2164,7 +2186,7 @@ static int run_skinny(const tccg_plan* p, const void* GA, const void* GB, float*
   if (p->sk_reg) {
     const int64_t grid = std::min<int64_t>(a.njobs, (int64_t)SKR_CTAS_PER_SM * p->num_sms);
     // 8 computed rows for a narrow side of at most 8, else 16
-    const bool kw = a.p_walk == SK_P_K;
+    const bool kw = reg_quads(p);
     launch_after(false, p,
                  a.S <= 8 ? (kw ? skinny_reg_kernel<8, true> : skinny_reg_kernel<8, false>)
                           : (kw ? skinny_reg_kernel<16, true> : skinny_reg_kernel<16, false>),
@@ -2444,10 +2466,10 @@ extern "C" int tccg_transpose(int32_t dtype, int32_t dim, const int32_t* perm,
 // grouped launches
 // --------------------------------------------------------------------------
 // Lane of a CUDA-core skinny item: its rows per thread (4, 8 or 12), and one
-// for the register path on items whose P has its stride-one index contracted.
+// for the register path's items with quads of k.
 static constexpr int SK_CLASSES = 4;
 static int skinny_class(const tccg_plan* p) {
-  return p->sk_reg && p->sk.p_walk == SK_P_K ? 3 : p->sk.rs / 4 - 1;
+  return reg_quads(p) ? 3 : p->sk.rs / 4 - 1;
 }
 
 struct tccg_group {
@@ -2708,6 +2730,8 @@ static ReduceJob<T> reduce_job_for(const T* partial, int32_t splits, int64_t Mp,
   j.beta = (T)beta;
   j.begin = begin;
   j.splits = splits;
+  j.range = nullptr;
+  j.K = (int32_t)std::min<int64_t>(p->K, INT32_MAX);
   j.mblocks = (int32_t)cdiv(p->M, 256);
   // about 256 loads per thread: many slices -> few columns per CTA
   j.ncols = (int32_t)std::max<int64_t>(1, std::min<int64_t>(64, 256 / splits));
@@ -2863,6 +2887,7 @@ static int bind_tc(tccg_group* g, tccg_group::Wave& wv, const void* const* A, co
       if (p->ksplit > 1) {
         red.push_back(reduce_job_for<float>(it.args.partial, p->ksplit, p->M, p->N, p, C[i],
                                             alpha[i], beta[i], rctas));
+        red.back().range = it.args.range;
         rctas += reduce_ctas(red.back());
       }
     }

@@ -30,6 +30,8 @@ CASES = {
     # more tiles than CTAs, C's runs shorter than a warp (staged stores)
     "runs": ("anbm", "mak", "bkn", dict(a=11, n=40, b=61, m=97, k=70), 1.0, 0.0, 4),
     "swap": ("pqr", "qs", "spr", dict(p=37, q=129, r=31, s=253), 0.75, -0.5, 1),
+    # few tiles: k slices added by the reduction
+    "split": ("mn", "mk", "kn", dict(m=96, n=70, k=3 * 4096 + 65), 1.25, 0.5, 4),
     "k_modes": ("abij", "iman", "mnjb", dict(a=9, b=33, i=21, j=17, m=12, n=20), 1.0, 0.0, 4),
 }
 
@@ -82,10 +84,11 @@ SPECIAL = {"inf": np.inf, "nan": np.nan, "near_max": 3.3e38, "min_normal": 1.2e-
 @pytest.mark.gpu
 @pytest.mark.parametrize("where", ["A", "B"])
 @pytest.mark.parametrize("value", sorted(SPECIAL))
-@pytest.mark.parametrize("shape", [dict(m=300, n=170, k=97), dict(m=3000, n=2000, k=300)])
+@pytest.mark.parametrize("shape", [dict(m=300, n=170, k=97), dict(m=3000, n=2000, k=300),
+                                   dict(m=100, n=60, k=3000)])
 def test_values_the_split_does_not_represent(cuda, value, where, shape):
     """Such operands run on the CUDA cores, bit for bit as with variant = -1,
-    C read with beta as it was (also behind a tail split); infinities and NaN
+    C read with beta as it was (also behind a tail split and a k-split); infinities and NaN
     come out where FFMA puts them."""
     con = make_contraction("mn", "mk", "kn", shape, 1.5, 0.5)
     _, A, B, C = _data("", ("mn", "mk", "kn", shape))
@@ -122,7 +125,7 @@ def test_group(cuda):
     with CUDA-core items, under a graph: bit for bit the per-item runs."""
     import torch
     from tccg_b200.grouped import Group
-    names = ["runs", "fills_past", "swap", "k_modes"]
+    names = ["runs", "fills_past", "swap", "k_modes", "split"]
     items = [make_contraction(*CASES[n][:4], CASES[n][4], CASES[n][5]) for n in names]
     items += [make_contraction("mn", "mk", "kn", dict(m=300, n=260, k=200), 1.0, 0.5)] * 2
     tunings = [Tuning(variant=CASES[n][6]) for n in names] + [Tuning(variant=4), Tuning(variant=-1)]
@@ -132,7 +135,7 @@ def test_group(cuda):
     As[2][7] = float("inf")
     Cs = [c.clone() for c in C0]
     grp = Group(items, "fp32", tunings=tunings)
-    assert sum("F32X6" in p.describe() for p in grp.plans) == 5
+    assert sum("F32X6" in p.describe() for p in grp.plans) == 6
     grp.bind(As, Bs, Cs)
     grp.capture()
     for c, c0 in zip(Cs, C0):
