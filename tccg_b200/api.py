@@ -50,18 +50,18 @@ class Compiled:
         return self.contraction.beta
 
     def workspace(self, device):
-        import torch
         n = self.plan.workspace_bytes
         if n == 0:
             return None
+        import torch
         if self._ws is None or self._ws.device != device or self._ws.numel() < n:
             self._ws = torch.empty(n, dtype=torch.uint8, device=device)
         return self._ws
 
     def __call__(self, A, B, C=None, alpha: Optional[float] = None, beta: Optional[float] = None,
                  stream=None):
-        import torch
         if C is None:
+            import torch
             dt = torch.float64 if self.plan.c_dtype == "f64" else torch.float32
             C = torch.empty(self.contraction.C0.num_elements(), dtype=dt, device=A.device)
             if beta is None and self.beta != 0:

@@ -222,6 +222,8 @@ class Plan:
         ws = ctypes.c_size_t()
         N.check(self._lib.tccg_plan_workspace(self._h, ctypes.byref(ws)))
         self.workspace_bytes = int(ws.value)
+        self._numel = (con.A0.num_elements(), con.B0.num_elements(), con.C0.num_elements())
+        self._run = self._lib.tccg_plan_run
 
     # -- info -------------------------------------------------------------
     def describe(self) -> str:
@@ -245,10 +247,9 @@ class Plan:
     # -- execution --------------------------------------------------------
     def run_ptr(self, A: int, B: int, C: int, alpha: float, beta: float, ws: int, ws_bytes: int,
                 stream: int) -> None:
-        N.check(self._lib.tccg_plan_run(self._h, ctypes.c_void_p(A), ctypes.c_void_p(B),
-                                        ctypes.c_void_p(C), float(alpha), float(beta),
-                                        ctypes.c_void_p(ws), ctypes.c_size_t(ws_bytes),
-                                        ctypes.c_void_p(stream)))
+        rc = self._run(self._h, A, B, C, float(alpha), float(beta), ws, ws_bytes, stream)
+        if rc:
+            N.check(rc)
 
     def run(self, A, B, C, alpha: Optional[float] = None, beta: Optional[float] = None,
             workspace=None, stream=None) -> None:
@@ -256,20 +257,33 @@ class Plan:
         memory is the column-major tensor of the contraction (the first index
         has stride one; e.g. a contiguous tensor of the reversed shape, or a
         flat one)."""
-        import torch
-        alpha = self.con.alpha if alpha is None else alpha
-        beta = self.con.beta if beta is None else beta
-        _check_buffer(A, self.con.A0.num_elements(), self.dtype, "A")
-        _check_buffer(B, self.con.B0.num_elements(), self.dtype, "B")
-        _check_buffer(C, self.con.C0.num_elements(), self.c_dtype, "C")
+        if alpha is None:
+            alpha = self.con.alpha
+        if beta is None:
+            beta = self.con.beta
+        # a call's host time is its latency where the kernels are small: one
+        # expression per operand, the messages only for what fails it
+        torch = _torch()
+        na, nb, nc = self._numel
+        dt, ct = _torch_dtype(self.dtype), _torch_dtype(self.c_dtype)
+        if not (_is_buffer(torch, A, na, dt) and _is_buffer(torch, B, nb, dt)
+                and _is_buffer(torch, C, nc, ct)):
+            _check_buffer(A, na, self.dtype, "A")
+            _check_buffer(B, nb, self.dtype, "B")
+            _check_buffer(C, nc, self.c_dtype, "C")
         if workspace is None and self.workspace_bytes:
             workspace = torch.empty(self.workspace_bytes, dtype=torch.uint8, device=C.device)
-        ws_ptr = workspace.data_ptr() if workspace is not None else 0
-        ws_n = workspace.numel() * workspace.element_size() if workspace is not None else 0
-        if stream is None:
-            stream = torch.cuda.current_stream(C.device)
-        self.run_ptr(A.data_ptr(), B.data_ptr(), C.data_ptr(), alpha, beta, ws_ptr, ws_n,
-                     stream.cuda_stream)
+        if workspace is not None:
+            ws_ptr, ws_n = workspace.data_ptr(), workspace.nbytes
+        else:
+            ws_ptr = ws_n = 0
+        # the current stream's handle without building a Stream object (2 us)
+        handle = (stream.cuda_stream if stream is not None
+                  else torch._C._cuda_getCurrentRawStream(C.device.index))
+        rc = self._run(self._h, A.data_ptr(), B.data_ptr(), C.data_ptr(), float(alpha), float(beta),
+                       ws_ptr, ws_n, handle)
+        if rc:
+            N.check(rc)
 
     def run_timed(self, A, B, C, alpha: Optional[float] = None, beta: Optional[float] = None,
                   workspace=None, stream=None) -> Tuple[float, float, float]:
@@ -327,6 +341,30 @@ class Plan:
 
 
 _TORCH_DT = {"f32": "float32", "f64": "float64", "bf16": "bfloat16"}
+_TORCH = None
+_DTYPES = {}
+
+
+def _torch():
+    """torch, imported on first use."""
+    global _TORCH
+    if _TORCH is None:
+        import torch
+        _TORCH = torch
+    return _TORCH
+
+
+def _torch_dtype(name: str):
+    dt = _DTYPES.get(name)
+    if dt is None:
+        dt = _DTYPES[name] = getattr(_torch(), _TORCH_DT[name])
+    return dt
+
+
+def _is_buffer(torch, t, numel: int, dtype) -> bool:
+    """What ``_check_buffer`` accepts."""
+    return (isinstance(t, torch.Tensor) and t.is_cuda and t.dtype == dtype and t.numel() == numel
+            and t.is_contiguous())
 
 
 def _check_buffer(t, numel: int, dtype: str, name: str) -> None:
