@@ -189,6 +189,9 @@ struct TcArgs {
   int32_t crun;
   // TC_F32X6: the operands' range words (AbsRange, GA's two then GB's)
   const uint32_t* range;
+  // C's element offsets all fit 31 bits: the epilogue passes column offsets
+  // around as 32-bit values
+  int32_t c32;
 };
 
 // Grouped launch: one entry per contraction, in device memory. The tensor maps
@@ -597,6 +600,39 @@ __device__ __forceinline__ void gather_producer(const TcArgs* a1, const TcGroup&
   cp_async_wait<0>();  // no copy in flight when the producers leave
 }
 
+// NC columns of this lane's row to C[row + column offset], columns j < lim of
+// them (LIMIT; else all): column j's offset is held by lane (j0 + j) % 32 of
+// off[(j0 + j) / 32] (32-bit, TcArgs::c32), val(j) gives its sum. Four or five
+// instructions a column -- shuffle, address, scale, (test,) store -- where
+// 64-bit offsets with tests per element took 25, which bound the short-K tiles
+// (9216^2 x 64 split-BF16x3: 169 us; 103 with this).
+template <int NC, bool LIMIT, int NO, typename F>
+__device__ __forceinline__ void store_cols(float* row, const int32_t (&off)[NO], int j0, int lim,
+                                           float alpha, float beta, F&& val) {
+  if (beta != 0.0f) {
+    constexpr int NB = NC > 32 ? 8 : 16;  // more spill the sums: 32^6 split-BF16x3 23.3 -> 25.3 ms
+#pragma unroll
+    for (int c = 0; c < NC; c += NB) {
+      float* d[NB];
+      float old[NB];
+#pragma unroll
+      for (int j = 0; j < NB; ++j) {
+        d[j] = row + __shfl_sync(0xffffffffu, off[(j0 + c + j) / 32], (j0 + c + j) % 32);
+        old[j] = !LIMIT || c + j < lim ? *d[j] : 0.0f;
+      }
+#pragma unroll
+      for (int j = 0; j < NB; ++j)
+        if (!LIMIT || c + j < lim) *d[j] = fmaf(beta, old[j], alpha * val(c + j));
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < NC; ++j) {
+      float* d = row + __shfl_sync(0xffffffffu, off[(j0 + j) / 32], (j0 + j) % 32);
+      if (!LIMIT || j < lim) *d = alpha * val(j);
+    }
+  }
+}
+
 // TC_F32X6: chunks of `chunk_kb` k-blocks (at most 4) per fill of the small
 // products' accumulator.
 template <int SMALL_KB>
@@ -883,6 +919,7 @@ __device__ __forceinline__ void gett_tc_body(const CUtensorMap* tmA, const CUten
         pld = a.M;
         pc0 = n0;
       }
+      const bool full = __all_sync(0xffffffffu, m_ok);  // every row of this warp inside C
       if constexpr (MODE == TC_BF16) {
         // one accumulator per tile: stream TMEM -> C
         if (!mbar_wait(&accf[acc], acc_phase, wait_ns)) {
@@ -909,11 +946,14 @@ __device__ __forceinline__ void gett_tc_body(const CUtensorMap* tmA, const CUten
             __syncwarp();
             if (lane == 0) mbar_arrive(&acce[acc]);
           }
-          if (m_ok && part) {
+          // warp-uniform branches: all but the last pass values between lanes
+          if (part) {
+            if (m_ok) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (cc + j < nlim) part[(size_t)(pc0 + cc + j) * pld] = __uint_as_float(r[j]);
-          } else if (a.crun > 0 && !part) {
+              for (int j = 0; j < 32; ++j)
+                if (cc + j < nlim) part[(size_t)(pc0 + cc + j) * pld] = __uint_as_float(r[j]);
+            }
+          } else if (a.crun > 0) {
 #pragma unroll
             for (int hh = 0; hh < 32; hh += 16) {
               if (cc + hh < nlim) {  // warp-uniform
@@ -928,6 +968,14 @@ __device__ __forceinline__ void gett_tc_body(const CUtensorMap* tmA, const CUten
                            a.crun, alpha, beta, lane, cmo, cn_lane);
               }
             }
+          } else if (a.c32) {
+            const int32_t off[1] = {cc + lane < nlim ? (int32_t)__ldg(cno + cc + lane) : 0};
+            auto val = [&](int j) { return __uint_as_float(r[j]); };
+            if (full && cc + 32 <= nlim)
+              store_cols<32, false>(Cb + cmo, off, 0, 32, alpha, beta, val);
+            else
+              store_cols<32, true>(Cb + cmo, off, 0, m_ok ? (int)(nlim - cc < 32 ? nlim - cc : 32) : 0,
+                                   alpha, beta, val);
           } else if (m_ok) {
             if (beta != 0.0f) {
               float old[32];
@@ -958,10 +1006,13 @@ __device__ __forceinline__ void gett_tc_body(const CUtensorMap* tmA, const CUten
         // cn[i] (loaded while the MMAs run; passed around by shuffles when
         // storing, so no store waits on a table load)
         constexpr int CG = (HC + 31) / 32;
-        int64_t cn[CG];
+        // (as 32 bits: the registers of the sums leave room for no more; the
+        // far columns of c32 == 0 are loaded again when storing)
+        const int ncol = nlim < HC ? (nlim > 0 ? (int)nlim : 0) : HC;
+        int32_t cn[CG];
 #pragma unroll
         for (int i = 0; i < CG; ++i)
-          cn[i] = 32 * i + lane < nlim ? __ldg(cno + 32 * i + lane) : 0;
+          cn[i] = 32 * i + lane < ncol ? (int32_t)__ldg(cno + 32 * i + lane) : 0;
         float sum[HC];
         const int seg = small_chunks<Cfg::SMALL_KB>(a.chunk_kb);
         int seg_ch = 0;
@@ -975,7 +1026,7 @@ __device__ __forceinline__ void gett_tc_body(const CUtensorMap* tmA, const CUten
           const uint32_t tsrc = tbase + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * Cfg::ACC_STRIDE + h * HC);
 #pragma unroll
           for (int cc = 0; cc < HC; cc += 16) {
-            if (cc < nlim) {  // warp-uniform: groups past C's last column are not read
+            if (cc < ncol) {  // warp-uniform: groups past C's last column are not read
               uint32_t r[16];
               tmem_ld_32x32b_x16(tsrc + (uint32_t)cc, r);
               tmem_ld_wait();
@@ -1006,7 +1057,7 @@ __device__ __forceinline__ void gett_tc_body(const CUtensorMap* tmA, const CUten
                   tbase + ((uint32_t)(q * 32) << 16) + (uint32_t)(2 * Cfg::ACC_STRIDE + h * HC);
 #pragma unroll
               for (int cc = 0; cc < HC; cc += 16) {
-                if (cc < nlim) {
+                if (cc < ncol) {
                   uint32_t r[16];
                   tmem_ld_32x32b_x16(ssrc + (uint32_t)cc, r);
                   tmem_ld_wait();
@@ -1024,47 +1075,41 @@ __device__ __forceinline__ void gett_tc_body(const CUtensorMap* tmA, const CUten
         if (!ok) break;
         if (part) {  // warp-uniform, like the branches below
           if (m_ok) {
+            float* d = part + (size_t)pc0 * pld;
 #pragma unroll
-            for (int j = 0; j < HC; ++j)
-              if (j < nlim) part[(size_t)(pc0 + j) * pld] = sum[j];
+            for (int j = 0; j < HC; ++j) {
+              if (j < ncol) *d = sum[j];
+              d += pld;
+            }
           }
         } else if (a.crun > 0) {
           constexpr int NC = Cfg::EPI_NC;
 #pragma unroll
           for (int cc = 0; cc < HC; cc += NC) {
-            if (cc < nlim) {  // warp-uniform
+            if (cc < ncol) {  // warp-uniform
               __syncwarp();
 #pragma unroll
               for (int j = 0; j < NC; ++j) wstg[j * Cfg::EPI_LD + lane] = sum[cc + j];
               __syncwarp();
-              const int64_t left = nlim - cc;
+              const int left = ncol - cc;
               const int64_t cn_lane =
-                  lane < NC && cc + lane < nlim ? __ldg(cno + cc + lane) : 0;
-              store_runs(wstg, a, (int64_t)t.tm * Cfg::BM + q * 32, left < NC ? (int)left : NC,
+                  lane < NC && cc + lane < ncol ? __ldg(cno + cc + lane) : 0;
+              store_runs(wstg, a, (int64_t)t.tm * Cfg::BM + q * 32, left < NC ? left : NC,
                          a.crun, alpha, beta, lane, cmo, cn_lane);
             }
           }
-        } else {
-          // every lane takes part in the shuffles; rows past M store nothing
-          if (beta != 0.0f) {
+        } else if (a.c32) {
+          auto val = [&](int j) { return sum[j]; };
+          if (full && ncol == HC)
+            store_cols<HC, false>(Cb + cmo, cn, 0, HC, alpha, beta, val);
+          else
+            store_cols<HC, true>(Cb + cmo, cn, 0, m_ok ? ncol : 0, alpha, beta, val);
+        } else if (m_ok) {
 #pragma unroll
-            for (int cc = 0; cc < HC; cc += 8) {
-              int64_t o[8];
-              float old[8];
-#pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                o[j] = cmo + __shfl_sync(0xffffffffu, cn[(cc + j) / 32], (cc + j) % 32);
-                old[j] = m_ok && cc + j < nlim ? Cb[o[j]] : 0.0f;
-              }
-#pragma unroll
-              for (int j = 0; j < 8; ++j)
-                if (m_ok && cc + j < nlim) Cb[o[j]] = fmaf(beta, old[j], alpha * sum[cc + j]);
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < HC; ++j) {
-              const int64_t o = cmo + __shfl_sync(0xffffffffu, cn[j / 32], j % 32);
-              if (m_ok && j < nlim) Cb[o] = alpha * sum[j];
+          for (int j = 0; j < HC; ++j) {
+            if (j < ncol) {
+              float* d = Cb + cmo + __ldg(cno + j);
+              *d = beta != 0.0f ? fmaf(beta, *d, alpha * sum[j]) : alpha * sum[j];
             }
           }
         }

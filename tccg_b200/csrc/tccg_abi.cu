@@ -86,6 +86,7 @@ struct tccg_plan {
   int32_t* d_status = nullptr;
   int32_t read_k_fast_a = 0, read_k_fast_b = 0;
   bool c_is_mn_dense = false;  // C is already the column-major [M-modes][N-modes] matrix
+  bool c32 = false;      // C's element offsets fit 31 bits
   bool c_quads = false;  // every quad of m is 4 consecutive elements of C at offsets % 4 == 0
   int64_t c_ldc = 0;  // > 0: C(m, n) = C[m + c_ldc * n] (a 2-D matrix in the GETT view)
   // SIMT geometry
@@ -1014,6 +1015,12 @@ extern "C" int tccg_plan_create(const tccg_desc* desc, int32_t dtype, int32_t pr
   p->c_quads = d.c_m_stride[0] == 1 && (d.m_ext[0] % 4 == 0 || p->M == d.m_ext[0]);
   for (int i = 1; i < d.nm; ++i) p->c_quads &= d.m_ext[i] == 1 || d.c_m_stride[i] % 4 == 0;
   for (int i = 0; i < d.nn; ++i) p->c_quads &= d.n_ext[i] == 1 || d.c_n_stride[i] % 4 == 0;
+  {
+    double span = 0;
+    for (int i = 0; i < d.nm; ++i) span += (double)(d.m_ext[i] - 1) * std::abs((double)d.c_m_stride[i]);
+    for (int i = 0; i < d.nn; ++i) span += (double)(d.n_ext[i] - 1) * std::abs((double)d.c_n_stride[i]);
+    p->c32 = span < 2147483647.0;
+  }
   bool m_unit = true;
   for (size_t m = 0; m < h.size() && m_unit; ++m) m_unit = h[m] == (int64_t)m;
   if (!rc) rc = upload(h, &p->t_c_m);
@@ -1946,6 +1953,7 @@ static TcArgs tc_args(const tccg_plan* p, float* Cout, const int64_t* c_m, const
   a.tail_partial = p->tail_split > 1 ? reinterpret_cast<float*>(ws + p->off_tail) : nullptr;
   a.crun = c_m == p->t_c_m ? p->crun : 0;  // not for TTGT's contiguous C'
   a.sm_order = sm_order_enabled() ? 1 : 0;
+  a.c32 = c_m == p->t_c_m ? p->c32 : p->M * p->N <= INT32_MAX;
   a.range = p->f32x6 ? reinterpret_cast<uint32_t*>(ws + p->off_range) : nullptr;
   return a;
 }
