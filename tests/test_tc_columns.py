@@ -1,62 +1,63 @@
-"""Column stores of the tensor-core epilogue: whole and ragged tiles, k slices
-(lanes past M take part in no column store there), beta read or not, and a C
-whose column offsets pass 32 bits (the 64-bit path).
-
-Tolerances: products of bf16 operands (and of the parts of a split) are exact;
-K <= 500 terms with truncating sums stay below K * 2^-23 / sqrt(K) = 2.7e-6 of
-the result's norm plus, for split-BF16x3, the dropped low product's 2^-16
-(rms 2^-17.6): 1e-5 for both, 1e-6 for the six-product split."""
+"""TMEM columns of the tcgen05 GETT kernel, on the CPU. The MMAs of a tile
+stop at the tile's last column of C rounded up to 32 (N of the per-tile
+instruction descriptor, tc_gemm.cuh). This restates that width and the two
+epilogues' TMEM reads -- BF16: 32-column loads up to the warp's last group
+that holds a column of C; BF16x3: 16-column loads below the warp's last
+column -- and checks, for every count of columns left in a tile: the MMA
+shape is one tcgen05.mma kind::f16 takes with M = 128 (N a multiple of 16,
+16..256) and the descriptor's fields hold it; no epilogue load reads a column
+the MMAs did not write; every column of C is read; an accumulator stays in
+its 256-column half of the 512 allocated. The kernel itself is checked on a
+B200 by the parity tests, whose N tails cover these widths."""
 import pytest
 
-from tccg_b200 import make_contraction
-from tccg_b200.plan import Plan, Tuning
-
-pytestmark = pytest.mark.gpu
-
-TOL = {"bf16": 1e-5, "bf16x3": 1e-5, "fp32": 1e-6}
+BM = 128
+ACC_STRIDE, TMEM_COLS = 256, 512
+TILE_N = {"bf16": 256, "bf16x3": 192}
 
 
-def _check(prec, m, n, k, beta, ksplit, ldc=None):
-    import torch
-    con = make_contraction("mn", "mk", "kn", dict(m=m, n=n, k=k), 1.25, beta)
-    g = torch.Generator(device="cuda").manual_seed(m + n + k)
-    A = torch.randn(k, m, generator=g, device="cuda")
-    B = torch.randn(n, k, generator=g, device="cuda")
-    if prec == "bf16":
-        A, B = A.bfloat16().float(), B.bfloat16().float()
-    far = ldc is not None
-    ldc = ldc or m + 3
-    buf = torch.empty(ldc * (n - 1) + m, device="cuda")
-    C = torch.as_strided(buf, (n, m), (ldc, 1))
-    if not far:
-        buf.fill_(7.0)
-    C.copy_(torch.randn(n, m, generator=g, device="cuda"))
-    want = 1.25 * (B.double() @ A.double()) + beta * C.double()
-    p = Plan(con, prec, tuning=Tuning(variant=1 if prec == "bf16" else 4, ksplit=ksplit, skinny=-1),
-             strides={"C": {"n": ldc}})
-    assert "gett_tc<" in p.describe()
-    assert ("ksplit=1 " in p.describe()) == (ksplit == 1)
-    ws = torch.empty(max(p.workspace_bytes, 1), dtype=torch.uint8, device="cuda")
-    p.run_ptr(A.data_ptr(), B.data_ptr(), buf.data_ptr(), 1.25, beta, ws.data_ptr(), ws.numel(),
-              torch.cuda.current_stream().cuda_stream)
-    torch.cuda.synchronize()
-    assert p.status() == 0
-    err = ((C.double() - want).norm() / want.norm()).item()
-    assert err <= TOL[prec], err
-    if not far:
-        assert torch.all(torch.as_strided(buf, (n - 1, 3), (ldc, 1), m) == 7.0)
+def idesc_bf16_f32(m, n):  # the descriptor built by common.cuh's idesc_bf16_f32
+    return (1 << 4) | (1 << 7) | (1 << 10) | ((n >> 3) << 17) | ((m >> 4) << 24)
 
 
-@pytest.mark.parametrize("beta", [0.0, -0.5])
-@pytest.mark.parametrize("m,n,k", [(128, 192, 200), (129, 161, 180), (31, 97, 500), (256, 320, 130),
-                                   (160, 33, 260), (300, 1, 200), (1, 200, 333), (2000, 3001, 150)])
-@pytest.mark.parametrize("prec,ksplit", [("bf16", 1), ("bf16", 3), ("bf16x3", 1), ("bf16x3", 3),
-                                         ("fp32", 1)])  # FP32: a split asked for stays off them
-def test_tiles(cuda, prec, m, n, k, ksplit, beta):
-    _check(prec, m, n, k, beta, ksplit)
+def mma_n(ncols, bn):
+    return bn if ncols >= bn else (ncols + 31) // 32 * 32
 
 
-@pytest.mark.parametrize("beta", [0.0, 0.5])
-@pytest.mark.parametrize("prec", ["bf16", "bf16x3", "fp32"])
-def test_far_columns(cuda, prec, beta):
-    _check(prec, 150, 4, 140, beta, 1, ldc=1 << 30)
+def epilogue_reads(mode, ncols, bn):
+    """TMEM columns each of the two column halves loads, per tile."""
+    hc = bn // 2
+    cols = set()
+    for h in range(2):
+        nlim = ncols - h * hc
+        if mode == "bf16":
+            last = hc - 32 if nlim >= hc else ((nlim - 1) // 32 * 32 if nlim > 0 else -32)
+            for cc in range(0, last + 1, 32):
+                cols.update(h * hc + cc + j for j in range(32))
+        else:
+            for cc in range(0, hc, 16):
+                if cc < nlim:
+                    cols.update(h * hc + cc + j for j in range(16))
+    return cols
+
+
+@pytest.mark.parametrize("mode", sorted(TILE_N))
+def test_mma_width_covers_the_epilogue(mode):
+    bn = TILE_N[mode]
+    for ncols in range(1, bn + 40):
+        n = mma_n(ncols, bn)
+        assert n % 16 == 0 and 16 <= n <= 256
+        d = idesc_bf16_f32(BM, n)
+        assert (d >> 17) & 0x3F == n >> 3 and (d >> 24) & 0x1F == BM >> 4
+        assert (d >> 23) & 1 == 0  # reserved bit between N and M stays clear
+        reads = epilogue_reads(mode, ncols, bn)
+        assert max(reads) < n, (ncols, n, max(reads))  # only columns the MMAs wrote
+        assert set(range(min(ncols, bn))) <= reads  # every column of C is read
+        for acc in range(2):  # both ping-pong accumulators inside the allocation
+            assert acc * ACC_STRIDE + n <= min((acc + 1) * ACC_STRIDE, TMEM_COLS)
+
+
+def test_full_tiles_keep_the_tile_width():
+    for mode, bn in TILE_N.items():
+        assert mma_n(bn, bn) == bn and mma_n(10 * bn, bn) == bn
+        assert epilogue_reads(mode, bn, bn) == set(range(bn))
