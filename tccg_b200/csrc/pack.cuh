@@ -55,6 +55,10 @@ struct PackOperand {
   // 16-byte aligned source elements (the first K mode has unit stride): the
   // pass streams 16-byte loads straight into K-major stores.
   int32_t kstream;
+  // PACK_K_BF16 only: 1 = every quad of tile rows (r % 4 == 0; the visit order
+  // where there is one) is 4 consecutive source elements, aligned to 4 of them
+  // at every k, and R % 4 == 0: tiles of 128 rows x 64 k by quads of rows.
+  int32_t rquad;
   // tile grid of this operand: tiles along k and in total (set by the host)
   int64_t ktiles, tiles;
   // PACK_K_F32X6: the operand's two range words (AbsRange), 0xffffffff before
@@ -234,6 +238,70 @@ __device__ __forceinline__ void pack_tile_wide(const PackOperand& o, int64_t kt,
   }
 }
 
+// Row-quad tile (PackOperand::rquad, PACK_K_BF16): 128 rows x 64 k, a lane per
+// 4 consecutive rows, so a warp reads 256 bytes (FP32: 512) of one k where the
+// 32-row tiles read 64 (128) with four times the instructions. A thread turns
+// 4 rows x 4 k in registers and leaves 4 k of a row as one 8-byte word in
+// shared memory; a row's 16 words are permuted by its row quad, so the lanes'
+// stores of one k quad and the 16-byte reads of a row touch every bank once.
+// 8 lanes then write a row's 128 bytes. Bound by memory traffic: 1024 x 4096 x
+// 4096 with both operands read along rows takes 48 us instead of 80 with BF16
+// operands, 57 instead of 66 with FP32 ones.
+constexpr int PACK_RQ_ROWS = 128, PACK_RQ_K = 64;
+
+__device__ __forceinline__ void row_quads_t(const uint2 (&v)[4], uint2 (&o)[4]) {
+  o[0] = make_uint2(__byte_perm(v[0].x, v[1].x, 0x5410), __byte_perm(v[2].x, v[3].x, 0x5410));
+  o[1] = make_uint2(__byte_perm(v[0].x, v[1].x, 0x7632), __byte_perm(v[2].x, v[3].x, 0x7632));
+  o[2] = make_uint2(__byte_perm(v[0].y, v[1].y, 0x5410), __byte_perm(v[2].y, v[3].y, 0x5410));
+  o[3] = make_uint2(__byte_perm(v[0].y, v[1].y, 0x7632), __byte_perm(v[2].y, v[3].y, 0x7632));
+}
+__device__ __forceinline__ uint32_t bf16_pair(float a, float b) {
+  const __nv_bfloat162 x = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&x);
+}
+__device__ __forceinline__ void row_quads_t(const float4 (&v)[4], uint2 (&o)[4]) {
+  o[0] = make_uint2(bf16_pair(v[0].x, v[1].x), bf16_pair(v[2].x, v[3].x));
+  o[1] = make_uint2(bf16_pair(v[0].y, v[1].y), bf16_pair(v[2].y, v[3].y));
+  o[2] = make_uint2(bf16_pair(v[0].z, v[1].z), bf16_pair(v[2].z, v[3].z));
+  o[3] = make_uint2(bf16_pair(v[0].w, v[1].w), bf16_pair(v[2].w, v[3].w));
+}
+
+template <typename Tin>
+__device__ __forceinline__ void pack_row_quads(const PackOperand& o, int64_t kt, int64_t rt, uint2* sm) {
+  using Quad = std::conditional_t<sizeof(Tin) == 2, uint2, float4>;
+  const int lane = threadIdx.x, w = threadIdx.y, t = w * 32 + lane;
+  const int64_t k0 = kt * PACK_RQ_K, r0 = rt * PACK_RQ_ROWS;
+  if (k0 >= o.Kcover || r0 >= o.Rcover) return;
+  const bool row = r0 + 4 * lane < o.R;  // R % 4 == 0
+  const Tin* src = static_cast<const Tin*>(o.src) + (row ? o.row_off[r0 + 4 * lane] : 0);
+  Quad v[2][4];
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int64_t k = k0 + 4 * (w + 8 * h) + j;
+      v[h][j] = row && k < o.Kk ? __ldg(reinterpret_cast<const Quad*>(src + o.col_off[k])) : Quad{};
+    }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint2 q[4];
+    row_quads_t(v[h], q);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sm[(4 * lane + i) * 16 + ((w + 8 * h) ^ (lane & 15))] = q[i];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < PACK_RQ_ROWS * PACK_RQ_K / 8 / 256; ++i) {
+    const int rl = (t >> 3) + 32 * i, c = t & 7, f = (rl >> 2) & 15;
+    const int64_t r = r0 + rl, k = k0 + 8 * c;
+    if (r >= o.Rcover || k >= o.Kcover) continue;  // Kcover % 8 == 0
+    const uint4 x = *reinterpret_cast<const uint4*>(&sm[rl * 16 + (((2 * c) ^ f) & ~1)]);
+    const int64_t rd = o.row_dst ? o.row_dst[r] : r;
+    *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(o.dst) + rd * o.ld + k) =
+        f & 1 ? make_uint4(x.z, x.w, x.x, x.y) : x;
+  }
+}
+
 // Position (r, l, u) of element f = r * T + l * run + u of a k-block tile,
 // stepped by `step` elements without divisions (one carry per level: the
 // step is below T and run).
@@ -315,21 +383,25 @@ __device__ __forceinline__ void pack_kblock(const PackOperand& o, int64_t kt, in
   }
 }
 
-// k-block tile with 16-byte copies (kb_quad): the tile is kept as the source
-// lays it out, raw[r][l][u] (u contiguous), 4 consecutive u per cp.async; the
-// 16-byte chunks of row (r, l) are rotated by l / 4 so that the write-out,
-// which reads 4 consecutive l of one u per quad of k, spreads over the banks.
-// Quads past K or the last row are read element by element (or zero).
-template <int LAYOUT>
+// k-block tile with copies of 4 elements (kb_quad; 16 bytes, 8 for bf16
+// sources): the tile is kept as the source lays it out, raw[r][l][u] (u
+// contiguous), 4 consecutive u per cp.async; the chunks of row (r, l) are
+// rotated by l / 4 so that the write-out, which reads 4 consecutive l of one u
+// per quad of k, spreads over the banks. Quads past K or the last row are read
+// element by element (or zero). bf16 sources have this form only (cp.async
+// takes no 2-byte element); 4096 rows x 1024 k of 32-element runs, with a
+// streamed operand of the same size: 23 us by the 32-row tiles, 20 by this.
+template <typename Tin, int LAYOUT>
 __device__ __forceinline__ void pack_kblock_quad(const PackOperand& o, int64_t kt, int64_t rt,
-                                                 float* tile, PackRange<LAYOUT>& rng) {
-  constexpr int NQ = PACK_KB_ELEMS / 4 / 256;  // 16-byte copies per thread at most
+                                                 float* smem, PackRange<LAYOUT>& rng) {
+  Tin* const tile = reinterpret_cast<Tin*>(smem);
+  constexpr int NQ = PACK_KB_ELEMS / 4 / 256;  // copies per thread at most
   const int lo = o.kb_lo, run = o.kb_run, T = lo * run, R = o.kb_rows;
-  const int nch = run / 4;  // 16-byte chunks per (r, l) row
+  const int nch = run / 4;  // chunks per (r, l) row
   const int64_t k0 = kt * T, r0 = rt * R;
   if (k0 >= o.Kcover || r0 >= o.Rcover) return;
   const int tid = threadIdx.x + 32 * threadIdx.y;
-  const float* src = static_cast<const float*>(o.src);
+  const Tin* src = static_cast<const Tin*>(o.src);
   const int u0 = (int)((kt * run) % o.kb_ext);  // u of the tile's first run (a multiple of 4)
   // chunk c of row (r, l) lives at raw position ((r lo + l) run + 4 ((c + l/4) % nch))
   auto chunk = [&](int r, int l, int c) {
@@ -342,15 +414,18 @@ __device__ __forceinline__ void pack_kblock_quad(const PackOperand& o, int64_t k
     const int c = f % nch, rl = f / nch, l = rl % lo, r = rl / lo;
     const int u = 4 * c;
     const int64_t row = r0 + r, k = k0 + l + (int64_t)lo * u;
-    float* d = chunk(r, l, c);
+    Tin* d = chunk(r, l, c);
     if (row < o.R && k + 3 * (int64_t)lo < o.Kk) {
       const int64_t coff = u0 + u < o.kb_ext ? o.col_off[k0 + l] + u : o.col_off[k];
-      cp_async_16(d, src + o.row_off[row] + coff);
+      if constexpr (sizeof(Tin) == 4)
+        cp_async_16(d, src + o.row_off[row] + coff);
+      else
+        cp_async_elem<8>(d, src + o.row_off[row] + coff);
     } else {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int64_t kj = k + (int64_t)lo * j;
-        d[j] = (row < o.R && kj < o.Kk) ? src[o.row_off[row] + o.col_off[kj]] : 0.f;
+        d[j] = (row < o.R && kj < o.Kk) ? src[o.row_off[row] + o.col_off[kj]] : Tin(0.0f);
       }
     }
   }
@@ -365,7 +440,7 @@ __device__ __forceinline__ void pack_kblock_quad(const PackOperand& o, int64_t k
     const int l = kq % lo, u = kq / lo;
     float x[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) x[j] = chunk(r, l + j, u >> 2)[u & 3];
+    for (int j = 0; j < 4; ++j) x[j] = load_as_acc<Tin>(chunk(r, l + j, u >> 2) + (u & 3));
     store_k4<LAYOUT>(static_cast<__nv_bfloat16*>(o.dst) + row * o.ld, k, o.Kcover, o.ld, x, rng);
   }
 }
@@ -432,14 +507,15 @@ __device__ __forceinline__ void pack_kstream(const PackOperand& o, int64_t blk, 
 }
 
 // Read schedules compiled into one pack kernel: the 32-row tiles, the
-// streaming pass or the k-block tiles only, or all three (chosen per operand
-// at run time: the grouped kernel). The narrower kernels keep their register
+// streaming pass, the k-block tiles or the row-quad tiles only, or all of them
+// (chosen per operand at run time: the grouped kernel). The narrower kernels keep their register
 // counts -- and so their occupancy -- free of the paths they do not run.
 enum PackRead : int {
   PACK_READ_WIDE = 0,
   PACK_READ_STREAM = 1,
   PACK_READ_KBLOCK = 2,
-  PACK_READ_ANY = 3
+  PACK_READ_ANY = 3,
+  PACK_READ_RQUAD = 4
 };
 
 template <typename Tin, typename Tout, int LAYOUT, int READ>
@@ -456,12 +532,19 @@ __device__ __forceinline__ void pack_tiles(const PackOperand& o, int64_t kt, int
       return;
     }
   }
-  if constexpr (KMAJOR && sizeof(Tin) == 4 && (READ == PACK_READ_KBLOCK || READ == PACK_READ_ANY)) {
+  if constexpr (KMAJOR && (READ == PACK_READ_KBLOCK || READ == PACK_READ_ANY)) {
     if (READ == PACK_READ_KBLOCK || o.kb_lo > 0) {
-      if (o.kb_quad)
-        pack_kblock_quad<LAYOUT>(o, kt, rt, &tile[0][0], rng);
-      else
+      if (sizeof(Tin) == 2 || o.kb_quad)
+        pack_kblock_quad<Tin, LAYOUT>(o, kt, rt, &tile[0][0], rng);
+      else if constexpr (sizeof(Tin) == 4)
         pack_kblock<Tin, LAYOUT>(o, kt, rt, &tile[0][0], rng);
+      return;
+    }
+  }
+  if constexpr (LAYOUT == PACK_K_BF16 && (READ == PACK_READ_RQUAD || READ == PACK_READ_ANY)) {
+    static_assert(PACK_RQ_ROWS * PACK_RQ_K * 2 <= sizeof(tile), "row-quad tile fits");
+    if (READ == PACK_READ_RQUAD || o.rquad) {
+      pack_row_quads<Tin>(o, kt, rt, reinterpret_cast<uint2*>(&tile[0][0]));
       return;
     }
   }

@@ -81,6 +81,8 @@ struct tccg_plan {
   // offset tables allow the streaming K-major pack (every quad of k is 4
   // consecutive elements, every quad start and row offset a multiple of 4)
   bool ks_a = false, ks_b = false;
+  // BF16 packs read A / B by quads of rows (row-quad tiles)
+  bool rq_a = false, rq_b = false;
   // the k-block tiles of A / B may move 16-byte quads along u (kb_quad)
   bool kbq_a = false, kbq_b = false;
   int32_t* d_status = nullptr;
@@ -943,6 +945,25 @@ static int mode_product(const char* cls, int n, const int64_t* ext, int64_t* out
   return TCCG_OK;
 }
 
+// Whether a BF16 pack that reads along the rows (of n modes) may read by quads
+// of them: the quads' elements consecutive and aligned in the order the rows
+// are read (visit: along the smallest-stride mode), at every k. From 64 rows
+// on, where half a tile's lanes have rows: 64 x 64 x 4096 with BF16 operands
+// takes 14.5 us against 16.7 by the 32-row tiles (FP32 operands 14.5 | 14.6),
+// 68 x 16384 x 2048 58 | 106 (72 | 85), and no size measured is slower.
+static bool row_quad_pack(const tccg_plan* p, int n, const int64_t* ext, const int64_t* str,
+                          const int64_t* kstr, bool visit, int32_t k_fast) {
+  if (p->prec != TCCG_PREC_BF16 || k_fast) return false;
+  std::vector<int64_t> rows, dst, ks;
+  if (!visit || !build_visit(n, ext, str, rows, dst)) build_offsets(n, ext, str, rows);
+  build_offsets(p->d.nk, p->d.k_ext, kstr, ks);
+  if (rows.size() < 64 || rows.size() % 4) return false;
+  for (size_t r = 0; r < rows.size(); r += 4)
+    if (rows[r] % 4 || rows[r + 1] != rows[r] + 1 || rows[r + 2] != rows[r] + 2 || rows[r + 3] != rows[r] + 3)
+      return false;
+  return rows_by_4(ks);
+}
+
 extern "C" int tccg_plan_create(const tccg_desc* desc, int32_t dtype, int32_t precision,
                                 const tccg_tuning* tuning, tccg_plan** out) {
   if (!desc || !out) return fail(TCCG_ERR_INVALID, "null descriptor or output pointer");
@@ -1116,9 +1137,9 @@ extern "C" int tccg_plan_create(const tccg_desc* desc, int32_t dtype, int32_t pr
     // tensor-core packs: unit stride on a later K mode -> k-block tiles read
     // along it; else walk the rows along the smallest-stride row mode when
     // that beats both the first row mode and reading along k
-    // (FP32 sources only: the tiles move 4-byte elements by cp.async)
-    if (!p->ks_a && p->dtype != TCCG_BF16) kblock_tiles(d.nk, d.k_ext, d.a_k_stride, p->kb_a);
-    if (!p->ks_b && p->dtype != TCCG_BF16) kblock_tiles(d.nk, d.k_ext, d.b_k_stride, p->kb_b);
+    // (BF16 sources: where the tiles move quads; cp.async takes no 2-byte element)
+    if (!p->ks_a && (p->dtype != TCCG_BF16 || p->kbq_a)) kblock_tiles(d.nk, d.k_ext, d.a_k_stride, p->kb_a);
+    if (!p->ks_b && (p->dtype != TCCG_BF16 || p->kbq_b)) kblock_tiles(d.nk, d.k_ext, d.b_k_stride, p->kb_b);
     std::vector<int64_t> vs, vd;
     auto kstride = [&](const int64_t* kst) {
       for (int i = 0; i < d.nk; ++i)
@@ -1137,6 +1158,8 @@ extern "C" int tccg_plan_create(const tccg_desc* desc, int32_t dtype, int32_t pr
       rc = upload(vs, &p->t_b_vsrc);
       if (!rc) rc = upload(vd, &p->t_b_vdst);
     }
+    p->rq_a = row_quad_pack(p, d.nm, d.m_ext, d.a_m_stride, d.a_k_stride, p->t_a_vsrc != nullptr, p->read_k_fast_a);
+    p->rq_b = row_quad_pack(p, d.nn, d.n_ext, d.b_n_stride, d.b_k_stride, p->t_b_vsrc != nullptr, p->read_k_fast_b);
   }
   if (!rc) rc = plan_layout(p);
   if (rc) {
@@ -1354,7 +1377,7 @@ static int plan_layout(tccg_plan* p) {
     snprintf(p->describe, sizeof(p->describe),
              "method=%s prec=%s kernel=gett_tc%s<%s> tile=%dx%d stages=%d M=%lld N=%lld K=%lld "
              "kblocks=%d chunk=%d ksplit=%d tail=%dx%d grid=%d raster=%d pack=K-major bf16%s(read_k_fast a=%d b=%d "
-             "visit a=%d b=%d kblock a=%dx%dx%d%s b=%dx%dx%d%s kstream a=%d b=%d)",
+             "visit a=%d b=%d kblock a=%dx%dx%d%s b=%dx%dx%d%s kstream a=%d b=%d rquad a=%d b=%d)",
              ttgt ? "TTGT" : "GETT", x6 ? "fp32" : x3 ? "bf16x3" : "bf16", pair ? "2" : "",
              x6 ? "F32X6" : x3 ? "BF16X3" : "BF16",
              pair ? 256 : 128, p->bn, stages,
@@ -1363,7 +1386,8 @@ static int plan_layout(tccg_plan* p) {
              p->tail_split, p->grid, p->raster, x6 ? " hi|mid|lo " : x3 ? " hi|lo " : " ", p->read_k_fast_a, p->read_k_fast_b,
              p->t_a_vsrc ? 1 : 0, p->t_b_vsrc ? 1 : 0, p->kb_a[0], p->kb_a[1], p->kb_a[2],
              p->kb_a[0] && p->kbq_a ? " x16B" : "", p->kb_b[0], p->kb_b[1], p->kb_b[2],
-             p->kb_b[0] && p->kbq_b ? " x16B" : "", p->ks_a ? 1 : 0, p->ks_b ? 1 : 0);
+             p->kb_b[0] && p->kbq_b ? " x16B" : "", p->ks_a ? 1 : 0, p->ks_b ? 1 : 0,
+             p->rq_a ? 1 : 0, p->rq_b ? 1 : 0);
   }
   if (ttgt) {
     // contiguous C' = [M][N] (column-major) in the workspace, then C' -> C
@@ -1708,7 +1732,7 @@ static PackOperand pack_op(const void* src, const int64_t* roff, const int64_t* 
   o.active = 1;
   o.row_dst = nullptr;
   o.kb_lo = o.kb_run = o.kb_rows = o.kb_ext = o.kb_step = o.kb_quad = 0;
-  o.kstream = 0;
+  o.kstream = o.rquad = 0;
   o.ktiles = o.tiles = 0;
   o.range = nullptr;
   return o;
@@ -1716,19 +1740,21 @@ static PackOperand pack_op(const void* src, const int64_t* roff, const int64_t* 
 
 // The read schedule of a K-major pack chosen at plan creation: the streaming
 // pass (when the source is aligned for its vector loads; es = source element
-// bytes) or k-block tiles, else unchanged.
+// bytes), k-block tiles or row-quad tiles, else unchanged.
 static PackOperand with_kread(PackOperand o, bool kstream, const int32_t (&kb)[5], bool kb_quad,
-                              size_t es) {
+                              bool rquad, size_t es) {
   const bool aligned = (reinterpret_cast<uintptr_t>(o.src) % (4 * es)) == 0;
   if (kstream && aligned) {
     o.kstream = 1;
-  } else if (kb[0] > 0) {
+  } else if (kb[0] > 0 && (es == 4 || aligned)) {  // BF16 sources: quads only
     o.kb_lo = kb[0];
     o.kb_run = kb[1];
     o.kb_rows = kb[2];
     o.kb_ext = kb[3];
     o.kb_step = kb[4];
     o.kb_quad = kb_quad && aligned ? 1 : 0;
+  } else if (rquad && aligned) {
+    o.rquad = 1;
   }
   return o;
 }
@@ -1744,6 +1770,9 @@ static void pack_geometry(PackOperand& o, int ktile) {
   if (o.kb_lo > 0) {
     kt = (int64_t)o.kb_lo * o.kb_run;
     rows = o.kb_rows;
+  } else if (o.rquad) {
+    kt = PACK_RQ_K;
+    rows = PACK_RQ_ROWS;
   }
   o.ktiles = cdiv(o.Kcover, kt);
   o.tiles = o.ktiles * cdiv(o.Rcover, rows);
@@ -1760,7 +1789,8 @@ static PackOperand with_visit(PackOperand o, const int64_t* vsrc, const int64_t*
 
 // Read schedule of one operand (PackRead).
 static int pack_read(const PackOperand& o) {
-  return o.kstream ? PACK_READ_STREAM : o.kb_lo > 0 ? PACK_READ_KBLOCK : PACK_READ_WIDE;
+  return o.kstream ? PACK_READ_STREAM : o.kb_lo > 0 ? PACK_READ_KBLOCK
+                   : o.rquad ? PACK_READ_RQUAD : PACK_READ_WIDE;
 }
 
 // One launch for both operands, with the kernel of their common read
@@ -1790,8 +1820,10 @@ static int launch_pack(PackArgs pa, cudaStream_t s, bool* launched = nullptr) {
       pack_kernel<Tin, Tout, LAYOUT, PACK_READ_STREAM><<<grid, block, 0, s>>>(pa);
     else if (read == PACK_READ_KBLOCK)
       pack_kernel<Tin, Tout, LAYOUT, PACK_READ_KBLOCK><<<grid, block, 0, s>>>(pa);
-    else
+    else if (read == PACK_READ_ANY || LAYOUT != PACK_K_BF16)
       pack_kernel<Tin, Tout, LAYOUT, PACK_READ_ANY><<<grid, block, 0, s>>>(pa);
+    else if constexpr (LAYOUT == PACK_K_BF16)
+      pack_kernel<Tin, Tout, LAYOUT, PACK_READ_RQUAD><<<grid, block, 0, s>>>(pa);
   }
   mark(0, 1, s);
   return launch_check("pack");
@@ -2057,10 +2089,10 @@ static int run_tc(const tccg_plan* p, const void* GA, const void* GB, float* Cou
     const size_t es = p->dtype == TCCG_BF16 ? 2 : 4;
     pa.op[0] = with_kread(with_visit(pack_op(GA, p->t_a_m, p->t_a_k, p->M, p->K, p->M, kcover, Ap,
                                              p->Kc, p->read_k_fast_a), p->t_a_vsrc, p->t_a_vdst),
-                          p->ks_a, p->kb_a, p->kbq_a, es);
+                          p->ks_a, p->kb_a, p->kbq_a, p->rq_a, es);
     pa.op[1] = with_kread(with_visit(pack_op(GB, p->t_b_n, p->t_b_k, p->N, p->K, p->N, kcover, Bp,
                                              p->Kc, p->read_k_fast_b), p->t_b_vsrc, p->t_b_vdst),
-                          p->ks_b, p->kb_b, p->kbq_b, es);
+                          p->ks_b, p->kb_b, p->kbq_b, p->rq_b, es);
     if (x6) {
       uint32_t* range = reinterpret_cast<uint32_t*>(ws + p->off_range);
       CUDA_TRY(cudaMemsetAsync(range, 0xff, 4 * sizeof(uint32_t), s));
@@ -2869,10 +2901,10 @@ static int bind_tc(tccg_group* g, tccg_group::Wave& wv, const void* const* A, co
         add_pack_jobs(jobs, pctas,
                       with_kread(with_visit(pack_op(GA, p->t_a_m, p->t_a_k, p->M, p->K, p->M, kcover,
                                                     w + p->off_a, p->Kc, p->read_k_fast_a),
-                                            p->t_a_vsrc, p->t_a_vdst), p->ks_a, p->kb_a, p->kbq_a, es),
+                                            p->t_a_vsrc, p->t_a_vdst), p->ks_a, p->kb_a, p->kbq_a, p->rq_a, es),
                       with_kread(with_visit(pack_op(GB, p->t_b_n, p->t_b_k, p->N, p->K, p->N, kcover,
                                                     w + p->off_b, p->Kc, p->read_k_fast_b),
-                                            p->t_b_vsrc, p->t_b_vdst), p->ks_b, p->kb_b, p->kbq_b, es),
+                                            p->t_b_vsrc, p->t_b_vdst), p->ks_b, p->kb_b, p->kbq_b, p->rq_b, es),
                       pack_k_tile<PACK_K_BF16>(), true);
         int rc;
         if (p->f32x6) {
