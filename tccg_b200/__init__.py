@@ -2,7 +2,8 @@
 
 ``C = alpha * A * B + beta * C`` for column-major tensors described in TCCG's
 ``.tccg`` format, computed by hand-written sm_100a CUDA kernels (tcgen05/TMA
-for BF16 and split-BF16x3, CUDA cores for FP32/FP64) behind a C ABI
+for BF16, split-BF16x3 and large FP32 contractions, CUDA cores and the FP64
+tensor pipe for the rest) behind a C ABI
 (include/tccg_b200.h).
 """
 from .spec import (Contraction, Index, Tensor, TccgSyntaxError, TccgUnsupported, fuse_indices,

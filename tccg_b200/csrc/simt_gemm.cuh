@@ -1,4 +1,5 @@
-// SIMT GETT kernels: FP32 FFMA and FP64 DFMA on the CUDA cores.
+// SIMT GETT kernels: FP32 FFMA (packed pairs) on the CUDA cores, FP64 on the
+// FP64 tensor pipe (mma.sync m16n8k8; the short-K kernel: DFMA).
 //
 // Operands come packed MN-major by pack_kernel (Ap[k][Mp], Bp[k][Np], zero
 // padded), so the main loop is a dense 16-byte cp.async pipeline -- or, for

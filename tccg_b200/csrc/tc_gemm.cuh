@@ -1,5 +1,6 @@
-// tcgen05 GETT kernel (sm_100a): BF16 and split-BF16x3 products on the 5th
-// generation tensor cores with FP32 accumulation in tensor memory.
+// tcgen05 GETT kernel (sm_100a): BF16, split-BF16x3 and FP32 (as six bf16
+// products, TC_F32X6) on the 5th generation tensor cores with FP32 accumulation
+// in tensor memory.
 //
 // Operands arrive packed K-major by pack_kernel: GA as [M][Kc] and GB as
 // [N][Kc] bf16 rows. In BF16 mode a 128-byte row chunk holds 64 consecutive k;
