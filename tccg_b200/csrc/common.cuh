@@ -384,6 +384,15 @@ __device__ __forceinline__ void cp_async_elem(void* smem_dst, const void* gsrc) 
                "n"(BYTES)
                : "memory");
 }
+// the same where `in` holds, else zeros (a copy of no source bytes: nothing is
+// read); without a branch
+template <int BYTES>
+__device__ __forceinline__ void cp_async_elem_or_zero(void* smem_dst, const void* gsrc, bool in) {
+  static_assert(BYTES == 4 || BYTES == 8, "cp.async.ca copies 4, 8 or 16 bytes");
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(smem_u32(smem_dst)),
+               "l"(gsrc), "n"(BYTES), "r"(in ? BYTES : 0)
+               : "memory");
+}
 // the same where `in` holds, without a branch (a divergent branch per copy
 // costs about 100 cycles)
 __device__ __forceinline__ void cp_async_4_if(void* smem_dst, const void* gsrc, bool in) {

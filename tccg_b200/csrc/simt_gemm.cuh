@@ -410,45 +410,40 @@ __device__ __forceinline__ void simt_gett_tile(const SimtArgs<T>& a, int bx, int
 #pragma unroll
         for (int j = 0; j < JAK; ++j) {
           T* dst = as + kk * LDA + kr + j * KR;
-          if (kfa[j] != NONE && koa != NONE)
-            cp_async_elem<sizeof(T)>(dst, a.Asrc + kfa[j] + koa);
-          else
-            *dst = T(0);
+          const bool in = kfa[j] != NONE && koa != NONE;
+          cp_async_elem_or_zero<sizeof(T)>(dst, a.Asrc + (in ? kfa[j] + koa : 0), in);
         }
       } else {
 #pragma unroll
         for (int j = 0; j < JA; ++j) {
           const int64_t kj = krow + drow_a + j * (256 / BM);
           T* dst = as + (drow_a + j * (256 / BM)) * LDA + dcol_a;
-          if (dm_off != NONE && kj < a.K)
-            cp_async_elem<sizeof(T)>(dst, a.Asrc + dm_off + __ldg(a.a_k_off + kj));
-          else
-            *dst = T(0);
+          const bool in = dm_off != NONE && kj < a.K;
+          cp_async_elem_or_zero<sizeof(T)>(dst, a.Asrc + (in ? dm_off + __ldg(a.a_k_off + kj) : 0), in);
         }
       }
       if (kfast_b) {
 #pragma unroll
         for (int j = 0; j < JBK; ++j) {
           T* dst = bs + kk * LDB + kr + j * KR;
-          if (kfb[j] != NONE && kob != NONE)
-            cp_async_elem<sizeof(T)>(dst, a.Bsrc + kfb[j] + kob);
-          else
-            *dst = T(0);
+          const bool in = kfb[j] != NONE && kob != NONE;
+          cp_async_elem_or_zero<sizeof(T)>(dst, a.Bsrc + (in ? kfb[j] + kob : 0), in);
         }
       } else {
 #pragma unroll
         for (int j = 0; j < JB; ++j) {
           const int64_t kj = krow + drow_b + j * (256 / BN);
           T* dst = bs + (drow_b + j * (256 / BN)) * LDB + dcol_b;
-          if (dn_off != NONE && kj < a.K)
-            cp_async_elem<sizeof(T)>(dst, a.Bsrc + dn_off + __ldg(a.b_k_off + kj));
-          else
-            *dst = T(0);
+          const bool in = dn_off != NONE && kj < a.K;
+          cp_async_elem_or_zero<sizeof(T)>(dst, a.Bsrc + (in ? dn_off + __ldg(a.b_k_off + kj) : 0), in);
         }
       }
     } else if (direct) {
       // all k offsets first (independent loads), then the copies: an offset
       // load between two asynchronous copies would serialise them
+      // Elements outside the operands are copies of no bytes, not branches
+      // (2048^2 x 256 FP32 98.7 -> 89.4 us, FP64 512^3 31.3 -> 24.9 with the
+      // mma.sync tiles, 20000 x 32 x 1000 90.1 -> 82.3).
       constexpr int JA = BK * BM / 256, JB = BK * BN / 256;
       int64_t koa[JA], kob[JB];
 #pragma unroll
@@ -464,18 +459,14 @@ __device__ __forceinline__ void simt_gett_tile(const SimtArgs<T>& a, int bx, int
 #pragma unroll
       for (int j = 0; j < JA; ++j) {
         T* dst = as + (drow_a + j * (256 / BM)) * LDA + dcol_a;
-        if (dm_off != NONE && koa[j] != NONE)
-          cp_async_elem<sizeof(T)>(dst, a.Asrc + dm_off + koa[j]);
-        else
-          *dst = T(0);
+        const bool in = dm_off != NONE && koa[j] != NONE;
+        cp_async_elem_or_zero<sizeof(T)>(dst, a.Asrc + (in ? dm_off + koa[j] : 0), in);
       }
 #pragma unroll
       for (int j = 0; j < JB; ++j) {
         T* dst = bs + (drow_b + j * (256 / BN)) * LDB + dcol_b;
-        if (dn_off != NONE && kob[j] != NONE)
-          cp_async_elem<sizeof(T)>(dst, a.Bsrc + dn_off + kob[j]);
-        else
-          *dst = T(0);
+        const bool in = dn_off != NONE && kob[j] != NONE;
+        cp_async_elem_or_zero<sizeof(T)>(dst, a.Bsrc + (in ? dn_off + kob[j] : 0), in);
       }
     } else if constexpr (LOAD != SIMT_DIRECT) {
 #pragma unroll
