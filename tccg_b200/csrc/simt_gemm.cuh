@@ -711,30 +711,32 @@ __global__ void __launch_bounds__(256, SimtCfg<T, S>::MIN_BLOCKS) simt_gett_kern
 
 // FP32 contractions that run as products of the operands' three-way bf16
 // splits (TC_F32X6) but whose values the splits do not represent: the tile
-// kernel on the caller's tensors. Launched behind the tensor-core kernel;
+// kernel on operands packed by the tensor-core kernel (f32_fallback_pack; in a
+// group: on the caller's tensors). Launched behind the tensor-core kernel;
 // its CTAs read the range words and leave at once in the ordinary case, so
 // the grid is one persistent wave, not one CTA per tile.
 struct F32FallbackItem {
-  SimtArgs<float> args;  // direct loads, no k-split
+  SimtArgs<float> args;  // no k-split
   const uint32_t* range;
   int32_t K, tiles_m;
   int64_t tiles;
 };
 
+template <int LOAD>
 __device__ __forceinline__ void f32_fallback(const F32FallbackItem& it) {
   if (f32_split_exact(it.range, it.K)) return;
   for (int64_t t = blockIdx.x; t < it.tiles; t += gridDim.x)
-    simt_gett_tile<float, SIMT_DIRECT>(it.args, (int)(t % it.tiles_m), (int)(t / it.tiles_m), 0);
+    simt_gett_tile<float, LOAD>(it.args, (int)(t % it.tiles_m), (int)(t / it.tiles_m), 0);
 }
 
 __global__ void __launch_bounds__(256, 2) f32_fallback_kernel(const F32FallbackItem it) {
   grid_dep_wait();  // range words of the packing pass; C written by nobody before this
-  f32_fallback(it);
+  f32_fallback<SIMT_PACKED>(it);
 }
 
 __global__ void __launch_bounds__(256, 2)
     f32_fallback_group_kernel(const F32FallbackItem* items, int n_items) {
-  for (int i = 0; i < n_items; ++i) f32_fallback(items[i]);
+  for (int i = 0; i < n_items; ++i) f32_fallback<SIMT_DIRECT>(items[i]);
 }
 
 // ---------------------------------------------------------------------------

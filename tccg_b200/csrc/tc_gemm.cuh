@@ -188,8 +188,10 @@ struct TcArgs {
   // C by the first N mode: stores go through shared memory in runs of e0 m
   // by 32 / e0 columns, which are consecutive addresses of C
   int32_t crun;
-  // TC_F32X6: the operands' range words (AbsRange, GA's two then GB's)
+  // TC_F32X6: the operands' range words (AbsRange, GA's two then GB's); where
+  // the fallback takes packed operands (not in groups), their place
   const uint32_t* range;
+  float* fb_pack[2];
   // C's element offsets all fit 31 bits: the epilogue passes column offsets
   // around as 32-bit values
   int32_t c32;
@@ -1140,6 +1142,32 @@ __global__ void __launch_bounds__(TcCfgT<MODE, LOAD, BNV>::NUM_THREADS, 1)
   gett_tc_body<MODE, LOAD, BNV, true>(nullptr, nullptr, nullptr, g, status);
 }
 
+// Operands of the FFMA fallback, packed as PACK_MN does (rows padded to 128, k
+// to 16, zeros) in the memory of the split ones, which nobody reads then: by
+// the tensor-core kernel, which has nothing else to do, so that the ordinary
+// case pays no launch. 4096 x 4096 x 1024 with one element of 1e-37: 0.97 ms;
+// 1.39 with the fallback reading the caller's tensors element by element. (The
+// FFMA plan, with its 16-byte packs and k slices, 0.66; split products 0.21.)
+static __device__ __noinline__ void f32_fallback_pack(const TcArgs& a, int threads) {
+  constexpr int U = 4;
+#pragma unroll 1
+  for (int o = 0; o < 2; ++o) {
+    const int64_t R = o ? a.N : a.M, Rp = (R + 127) / 128 * 128, Kp = ((int64_t)a.K + 15) / 16 * 16;
+    const int64_t step = (int64_t)gridDim.x * threads, total = Rp * Kp;
+    for (int64_t i0 = (int64_t)blockIdx.x * threads + threadIdx.x; i0 < total; i0 += U * step) {
+      float v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int64_t i = i0 + u * step, k = i / Rp, r = i - k * Rp;
+        v[u] = i < total && k < a.K && r < R ? __ldg(a.gsrc[o] + a.grow[o][r] + a.gk[o][k]) : 0.0f;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (i0 + u * step < total) a.fb_pack[o][i0 + u * step] = v[u];
+    }
+  }
+}
+
 // FP32 results (TC_F32X6): the hi | mid parts through tmA / tmB, the lo parts
 // through tmAl / tmBl, all on the packed operands.
 template <int MODE, int LOAD = TC_LOAD_TMA, int BNV = 0>
@@ -1147,10 +1175,12 @@ __global__ void __launch_bounds__(TcCfgT<MODE, LOAD, BNV>::NUM_THREADS, 1)
     gett_tc_f32_kernel(const __grid_constant__ CUtensorMap tmA,
                        const __grid_constant__ CUtensorMap tmB,
                        const __grid_constant__ CUtensorMap tmAl,
-                       const __grid_constant__ CUtensorMap tmBl, const TcArgs a) {
+                       const __grid_constant__ CUtensorMap tmBl, const __grid_constant__ TcArgs a) {
   static_assert(MODE == TC_F32X6, "FP32 split");
   TcGroup g{nullptr, nullptr, 0, 0};
   gett_tc_body<MODE, LOAD, BNV, false>(&tmA, &tmB, &a, g, a.status, &tmAl, &tmBl);
+  grid_dep_wait();  // the range words: not every warp has waited
+  if (!f32_split_exact(a.range, a.K)) f32_fallback_pack(a, TcCfgT<MODE, LOAD, BNV>::NUM_THREADS);
 }
 
 // Tail split: C = alpha * (slice 0 + slice 1 + ...) + beta * C over the tail

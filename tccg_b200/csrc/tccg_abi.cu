@@ -136,6 +136,7 @@ struct tccg_plan {
   int32_t* t_sk = nullptr;
   size_t sk_tab[6] = {};
   // workspace layout
+  size_t off_fb = 0;  // FP32 on the tensor cores: the fallback's B (its A at off_a)
   size_t off_a = 0, off_b = 0, off_part = 0, off_cprime = 0, off_tail = 0, ws_bytes = 0;
   char describe[512] = "";
 };
@@ -1170,6 +1171,11 @@ extern "C" int tccg_plan_create(const tccg_desc* desc, int32_t dtype, int32_t pr
   return TCCG_OK;
 }
 
+// Elements of one operand packed for the FP32 fallback (f32_fallback_pack).
+static int64_t f32_fallback_elems(int64_t rows, int64_t K) {
+  return round_up(rows, SimtCfg<float>::BM) * round_up(K, SimtCfg<float>::BK);
+}
+
 static int plan_layout(tccg_plan* p) {
   size_t ws = 0;
   const bool ttgt = p->tune.method == TCCG_METHOD_TTGT;
@@ -1351,7 +1357,9 @@ static int plan_layout(tccg_plan* p) {
       p->off_b = ws;
       ws = align_up(ws + (size_t)(p->N * p->Kc) * 2, 256);
     }
-    if (x6) {  // the operands' range words
+    if (x6) {  // the operands' range words, past the fallback's packed operands too
+      p->off_fb = align_up((size_t)f32_fallback_elems(p->M, p->K) * 4, 256);
+      ws = std::max(ws, align_up(p->off_fb + (size_t)f32_fallback_elems(p->N, p->K) * 4, 256));
       p->off_range = ws;
       ws += 256;
     }
@@ -2107,6 +2115,9 @@ static int run_tc(const tccg_plan* p, const void* GA, const void* GB, float* Cou
       rc = launch_pack<float, __nv_bfloat16, PACK_K_BF16>(pa, s, &packed);
     if (rc) return rc;
     if (x6) {
+      set_gather(a, p, GA, GB);
+      a.fb_pack[0] = static_cast<float*>(Ap);
+      a.fb_pack[1] = reinterpret_cast<float*>(ws + p->off_fb);
       rc = encode_f32x6(p, Ap, Bp, &tmA, &tmB, &tmAl, &tmBl);
     } else {
       rc = encode_kmajor(&tmA, Ap, p->M, p->Kc, 128);
@@ -2138,7 +2149,12 @@ static int run_tc(const tccg_plan* p, const void* GA, const void* GB, float* Cou
   if (rc) return rc;
   rc = tc_reduce(p, a, Cout, c_m, c_n, alpha, beta, s);
   if (rc || !x6) return rc;
-  const F32FallbackItem it = f32_fallback_item(p, GA, GB, Cout, a.range, alpha, beta);
+  F32FallbackItem it = f32_fallback_item(p, GA, GB, Cout, a.range, alpha, beta);
+  it.args.direct = 0;
+  it.args.Ap = a.fb_pack[0];
+  it.args.Bp = a.fb_pack[1];
+  it.args.Mp = round_up(p->M, SimtCfg<float>::BM);
+  it.args.Np = round_up(p->N, SimtCfg<float>::BN);
   launch_after(true, p, f32_fallback_kernel, dim3((unsigned)std::min<int64_t>(it.tiles, 2 * p->num_sms)),
                dim3(256), simt_smem_bytes<float>(), s, it);
   return launch_check("f32_fallback");
