@@ -30,7 +30,7 @@ def nvcc_path() -> str:
 
 def sources():
     return sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh"))
-                  + [os.path.join(INCLUDE, "tccg_b200.h")])
+                  + glob.glob(os.path.join(CSRC, "*.h")) + [os.path.join(INCLUDE, "tccg_b200.h")])
 
 
 def needs_build() -> bool:

@@ -17,6 +17,7 @@
 
 #include "../../include/tccg_b200.h"
 #include "common.cuh"
+#include "f32_split_rule.h"
 #include "pack.cuh"
 #include "simt_gemm.cuh"
 #include "skinny_gett.cuh"
@@ -327,8 +328,7 @@ static bool choose_f32x6(const tccg_plan* p) {
   if (p->prec != TCCG_PREC_FP32 || p->dtype != TCCG_F32 || t.method != TCCG_METHOD_GETT || t.pair ||
       t.variant < 0 || t.ksplit > 1 || t.direct > 0 || t.shortk > 0 || t.simt_tile != 0)
     return false;
-  const int64_t lim = int64_t(1) << 30;
-  if (p->M >= lim || p->N >= lim || p->K >= lim) return false;
+  if (!f32_split_fits(p->M, p->N, p->K)) return false;
   if (t.variant > 0) return true;
   if (p->K < F32X6_MIN_K) return false;
   const int64_t tiles = cdiv(p->M, F32X6_BM) * cdiv(p->N, F32X6_BN), kb = cdiv(p->K, 32);
