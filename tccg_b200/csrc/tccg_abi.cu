@@ -770,10 +770,15 @@ static bool choose_skinny_tc(const tccg_plan* p) {
   // a narrow side of at most 16 takes the CUDA-core register path instead
   // (choose_skinny; 12 x 21 boxes of S = 11, K = 2744: 453 us against 469
   // here, S = 13, K = 3240: 197 / 225) -- except where P's stride-one index is
-  // contracted: the register path's loads (16 consecutive k per lane) then
-  // touch 32 rows per warp load (S = 8, K = 1024: 283 us against 143; S = 8,
-  // K = 720: 1412 / 513; S = 9, K = 168: 777 / 629)
-  if (p->K > SK_KC && p->sk.nblk >= 48 && p->sk.S <= 16 && p->sk.p_walk == SK_P_K) return true;
+  // contracted and K spans at least 8 chunks: the register path's loads (16
+  // consecutive k per lane) then touch 32 rows per warp load (S = 8, K = 1024:
+  // 283 us against 143; S = 8, K = 720: 1412 / 513). With fewer chunks the
+  // register path's FP32 products are kept: error 1e-7 against 4e-6 of the
+  // split ones, for the same call (S = 9, K = 168: 777 us against 629; S = 9,
+  // K = 77, W = 37911: 15 against 20; S = 6, K = 70, W = 14726: 12.4 / 14.5)
+  if (p->K > SK_KC && p->sk.nblk >= 48 && p->sk.S <= 16 && p->sk.p_walk == SK_P_K &&
+      p->sk.nchunks >= 8)
+    return true;
   return p->K > SK_KC && p->sk.nblk >= 48 && p->sk.S > 16 && p->sk.S <= SKT_SMAX;
 }
 
