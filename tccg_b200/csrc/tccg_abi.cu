@@ -835,6 +835,14 @@ static bool rows_by_4(const std::vector<int64_t>& roff) {
     if (o % 4 != 0) return false;
   return true;
 }
+// Every whole quad (i % 4 == 0) starts at a multiple of 4 and runs over 4
+// consecutive elements.
+static bool quads_by_4(const std::vector<int64_t>& off) {
+  for (size_t i = 0; i + 3 < off.size(); i += 4)
+    if (off[i] % 4 != 0 || off[i + 1] != off[i] + 1 || off[i + 2] != off[i] + 2 || off[i + 3] != off[i] + 3)
+      return false;
+  return true;
+}
 static bool k_quads(const std::vector<int64_t>& coff) {
   if (coff.size() < 4) return false;
   for (size_t k = 0; k + 3 < coff.size(); k += 4) {
@@ -1039,9 +1047,9 @@ extern "C" int tccg_plan_create(const tccg_desc* desc, int32_t dtype, int32_t pr
     for (int i = 0; i < d.nn; ++i) { dense &= d.c_n_stride[i] == s; s *= d.n_ext[i]; }
     p->c_is_mn_dense = dense;
   }
-  p->c_quads = d.c_m_stride[0] == 1 && (d.m_ext[0] % 4 == 0 || p->M == d.m_ext[0]);
-  for (int i = 1; i < d.nm; ++i) p->c_quads &= d.m_ext[i] == 1 || d.c_m_stride[i] % 4 == 0;
-  for (int i = 0; i < d.nn; ++i) p->c_quads &= d.n_ext[i] == 1 || d.c_n_stride[i] % 4 == 0;
+  // from the offsets, not the modes: quads may run on from one M mode into the
+  // next (1036 = 37 x 28 rows, dense in C)
+  p->c_quads = quads_by_4(h);
   {
     double span = 0;
     for (int i = 0; i < d.nm; ++i) span += (double)(d.m_ext[i] - 1) * std::abs((double)d.c_m_stride[i]);
@@ -1052,6 +1060,7 @@ extern "C" int tccg_plan_create(const tccg_desc* desc, int32_t dtype, int32_t pr
   for (size_t m = 0; m < h.size() && m_unit; ++m) m_unit = h[m] == (int64_t)m;
   if (!rc) rc = upload(h, &p->t_c_m);
   build_offsets(d.nn, d.n_ext, d.c_n_stride, h);
+  p->c_quads = p->c_quads && rows_by_4(h);
   if (m_unit) {
     const int64_t ldc = h.size() > 1 ? h[1] : std::max<int64_t>(p->M, 1);
     bool two_d = ldc > 0;
@@ -1265,7 +1274,7 @@ static int plan_layout(tccg_plan* p) {
     static const char* pn[] = {"fp32", "fp64", "bf16", "bf16x3"};
     snprintf(p->describe, sizeof(p->describe),
              "method=%s prec=%s kernel=simt_%s<%s> tile=%dx%dx%d M=%lld N=%lld K=%lld "
-             "ksplit=%d pack=%s%s%s(%s a=%d b=%d)",
+             "ksplit=%d pack=%s%s%s(%s a=%d b=%d) cquads=%d",
              ttgt ? "TTGT" : "GETT", pn[p->prec], p->shortk ? "shortk" : "gett", dbl ? "f64" : "f32",
              BM, BN, BK,
              (long long)p->M, (long long)p->N, (long long)p->K, p->ksplit,
@@ -1274,7 +1283,7 @@ static int plan_layout(tccg_plan* p) {
              : !dbl && (ttgt || p->c_ldc > 0) ? " cblock=cp.async.bulk" : " cblock=cp.async",
              p->direct ? "gather_k" : "read_k_fast",
              p->direct ? (int)p->gather_k_a : p->read_k_fast_a,
-             p->direct ? (int)p->gather_k_b : p->read_k_fast_b);
+             p->direct ? (int)p->gather_k_b : p->read_k_fast_b, ttgt ? p->M % 4 == 0 : p->c_quads);
   } else {
     const bool x3 = p->prec == TCCG_PREC_BF16X3, x6 = p->f32x6;
     if (x3 || x6) {
