@@ -507,15 +507,18 @@ __device__ __forceinline__ void pack_kstream(const PackOperand& o, int64_t blk, 
 }
 
 // Read schedules compiled into one pack kernel: the 32-row tiles, the
-// streaming pass, the k-block tiles or the row-quad tiles only, or all of them
-// (chosen per operand at run time: the grouped kernel). The narrower kernels keep their register
-// counts -- and so their occupancy -- free of the paths they do not run.
+// streaming pass, the k-block tiles or the row-quad tiles only, or several,
+// chosen per operand at run time: all but the row quads (ANY), or all (ALL).
+// The narrower kernels keep their register counts -- and so their occupancy --
+// free of the paths they do not run (FP32 sources: 40 registers for ANY, 60
+// for ALL; 205920 x 1792 by k-blocks beside a small operand: 578 and 639 us).
 enum PackRead : int {
   PACK_READ_WIDE = 0,
   PACK_READ_STREAM = 1,
   PACK_READ_KBLOCK = 2,
   PACK_READ_ANY = 3,
-  PACK_READ_RQUAD = 4
+  PACK_READ_RQUAD = 4,
+  PACK_READ_ALL = 5
 };
 
 template <typename Tin, typename Tout, int LAYOUT, int READ>
@@ -526,13 +529,14 @@ __device__ __forceinline__ void pack_tiles(const PackOperand& o, int64_t kt, int
   static_assert(PACK_KB_ELEMS + PACK_KB_ELEMS / 32 <= PACK_KT_WIDE * 33, "k-block tile fits");
   static_assert(PACK_KS_Q * 256 * 4 <= PACK_KT_WIDE * 33, "streaming buffer fits");
   constexpr bool KMAJOR = pack_k_major(LAYOUT);
-  if constexpr (KMAJOR && (READ == PACK_READ_STREAM || READ == PACK_READ_ANY)) {
+  constexpr bool ANY = READ == PACK_READ_ANY || READ == PACK_READ_ALL;
+  if constexpr (KMAJOR && (READ == PACK_READ_STREAM || ANY)) {
     if (READ == PACK_READ_STREAM || o.kstream) {
       pack_kstream<Tin, LAYOUT>(o, rt, &tile[0][0], rng);  // one tile along k
       return;
     }
   }
-  if constexpr (KMAJOR && (READ == PACK_READ_KBLOCK || READ == PACK_READ_ANY)) {
+  if constexpr (KMAJOR && (READ == PACK_READ_KBLOCK || ANY)) {
     if (READ == PACK_READ_KBLOCK || o.kb_lo > 0) {
       if (sizeof(Tin) == 2 || o.kb_quad)
         pack_kblock_quad<Tin, LAYOUT>(o, kt, rt, &tile[0][0], rng);
@@ -541,14 +545,14 @@ __device__ __forceinline__ void pack_tiles(const PackOperand& o, int64_t kt, int
       return;
     }
   }
-  if constexpr (LAYOUT == PACK_K_BF16 && (READ == PACK_READ_RQUAD || READ == PACK_READ_ANY)) {
+  if constexpr (LAYOUT == PACK_K_BF16 && (READ == PACK_READ_RQUAD || READ == PACK_READ_ALL)) {
     static_assert(PACK_RQ_ROWS * PACK_RQ_K * 2 <= sizeof(tile), "row-quad tile fits");
     if (READ == PACK_READ_RQUAD || o.rquad) {
       pack_row_quads<Tin>(o, kt, rt, reinterpret_cast<uint2*>(&tile[0][0]));
       return;
     }
   }
-  if constexpr (!KMAJOR || READ == PACK_READ_WIDE || READ == PACK_READ_ANY)
+  if constexpr (!KMAJOR || READ == PACK_READ_WIDE || ANY)
     pack_tile_wide<Tin, Tout, LAYOUT>(o, kt, rt, tile, rng);
 }
 
@@ -577,7 +581,8 @@ struct PackJob {
   int64_t begin;  // first CTA of this job
 };
 
-template <typename Tin, typename Tout, int LAYOUT>
+// READ: PACK_READ_ANY, or PACK_READ_ALL where a job moves row quads.
+template <typename Tin, typename Tout, int LAYOUT, int READ = PACK_READ_ANY>
 __global__ void __launch_bounds__(256) pack_group_kernel(const PackJob* jobs, const int64_t* begin,
                                                          int n_jobs) {
   const int64_t t = blockIdx.x + (int64_t)gridDim.x * blockIdx.y;
@@ -585,7 +590,7 @@ __global__ void __launch_bounds__(256) pack_group_kernel(const PackJob* jobs, co
   // dependent global load at a time inside the tile code
   const PackJob j = jobs[find_segment(begin, n_jobs, t)];
   const int64_t local = t - j.begin;
-  pack_any<Tin, Tout, LAYOUT, PACK_READ_ANY>(j.op, local % j.op.ktiles, local / j.op.ktiles);
+  pack_any<Tin, Tout, LAYOUT, READ>(j.op, local % j.op.ktiles, local / j.op.ktiles);
 }
 
 }  // namespace tccg

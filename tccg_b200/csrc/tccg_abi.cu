@@ -1815,20 +1815,43 @@ static int pack_read(const PackOperand& o) {
                    : o.rquad ? PACK_READ_RQUAD : PACK_READ_WIDE;
 }
 
+// Whether operand o may move row quads beside `other`, which reads another way:
+// both then run the kernel of all reads (PACK_READ_ALL), whose registers cost
+// the other operand occupancy. So only where o has the larger part of the work,
+// a quarter of it for BF16 sources, whose 32-row tiles take twice as long.
+// o : other rows, without / with quads, us: FP32 1024 : 4096 x 4096 35.5 / 37.2,
+// 4096 : 1024 41.3 / 30.9; BF16 1024 : 4096 34.9 / 26.8, 216 : 3600 x 8976 83.6 /
+// 89.6, 420 : 7440 x 420 12.4 / 13.3.
+static bool quads_beside(const PackOperand& o, const PackOperand& other, size_t es) {
+  return o.Rcover * (es == 2 ? 4 : 1) >= other.Rcover;
+}
+
+// Drops the row quads of an operand that is packed beside one of another read
+// where they do not pay.
+static void settle_quads(PackOperand& a, PackOperand& b, size_t es) {
+  if (!a.active || !b.active || pack_read(a) == pack_read(b)) return;
+  if (a.rquad && !quads_beside(a, b, es)) a.rquad = 0;
+  if (b.rquad && !quads_beside(b, a, es)) b.rquad = 0;
+}
+
 // One launch for both operands, with the kernel of their common read
-// schedule, or the kernel holding all schedules when they differ (a second
+// schedule, or a kernel holding several schedules when they differ (a second
 // launch costs more than the wider kernel's extra registers).
 template <typename Tin, typename Tout, int LAYOUT>
 static int launch_pack(PackArgs pa, cudaStream_t s, bool* launched = nullptr) {
   if (launched) *launched = false;
   int64_t ctas = 0;
   int read = -1;
+  bool quads = false;
+  settle_quads(pa.op[0], pa.op[1], sizeof(Tin));
   for (PackOperand& o : pa.op) {
     pack_geometry(o, pack_k_tile<LAYOUT>());
     if (!o.active) continue;
     ctas = std::max(ctas, o.tiles);
+    quads |= pack_read(o) == PACK_READ_RQUAD;
     read = read < 0 || read == pack_read(o) ? pack_read(o) : PACK_READ_ANY;
   }
+  if (read == PACK_READ_ANY && quads) read = PACK_READ_ALL;
   if (ctas > INT32_MAX) return fail(TCCG_ERR_UNSUPPORTED, "operand too large to pack (%lld tiles)", (long long)ctas);
   if (ctas == 0) return TCCG_OK;
   if (launched) *launched = true;
@@ -1844,8 +1867,12 @@ static int launch_pack(PackArgs pa, cudaStream_t s, bool* launched = nullptr) {
       pack_kernel<Tin, Tout, LAYOUT, PACK_READ_KBLOCK><<<grid, block, 0, s>>>(pa);
     else if (read == PACK_READ_ANY || LAYOUT != PACK_K_BF16)
       pack_kernel<Tin, Tout, LAYOUT, PACK_READ_ANY><<<grid, block, 0, s>>>(pa);
-    else if constexpr (LAYOUT == PACK_K_BF16)
-      pack_kernel<Tin, Tout, LAYOUT, PACK_READ_RQUAD><<<grid, block, 0, s>>>(pa);
+    else if constexpr (LAYOUT == PACK_K_BF16) {
+      if (read == PACK_READ_RQUAD)
+        pack_kernel<Tin, Tout, LAYOUT, PACK_READ_RQUAD><<<grid, block, 0, s>>>(pa);
+      else
+        pack_kernel<Tin, Tout, LAYOUT, PACK_READ_ALL><<<grid, block, 0, s>>>(pa);
+    }
   }
   mark(0, 1, s);
   return launch_check("pack");
@@ -2597,6 +2624,7 @@ struct tccg_group {
     int32_t lane0[TCV_COUNT] = {}, nlane[TCV_COUNT] = {};
     int64_t lane_tiles[TCV_COUNT] = {};
     int32_t tcj0 = 0, ntcj = 0;  // pack jobs of the packed-operand lanes (two per item)
+    bool rquads = false;         // a pack job of these moves row quads
     int64_t simt_tiles = 0, simt_pack_ctas = 0, tc_pack_ctas = 0, red_ctas = 0;
     int32_t fb0 = 0;  // the TCV_F32X6 lane's items are [fb0, fb0 + nlane) of d_fb / d_range
     // skinny lanes, one per class (skinny_class): items [sk0[c], sk0[c] +
@@ -2965,6 +2993,8 @@ static int bind_tc(tccg_group* g, tccg_group::Wave& wv, const void* const* A, co
   }
   if (pctas > INT32_MAX) return fail(TCCG_ERR_UNSUPPORTED, "grouped packing grid too large");
   wv.ntcj = (int32_t)jobs.size() - wv.tcj0;
+  wv.rquads = false;
+  for (size_t j = (size_t)wv.tcj0; j < jobs.size(); ++j) wv.rquads |= jobs[j].op.rquad != 0;
   wv.tc_pack_ctas = pctas;
   return TCCG_OK;
 }
@@ -3248,9 +3278,11 @@ static int run_wave(const tccg_group* g, const tccg_group::Wave& wv, cudaStream_
     else if (x3)
       pack_group_kernel<float, __nv_bfloat16, PACK_K_BF16X3><<<pg, blk, 0, s>>>(tjobs, tb, tj);
     else if (g->dtype == TCCG_BF16)
-      pack_group_kernel<__nv_bfloat16, __nv_bfloat16, PACK_K_BF16><<<pg, blk, 0, s>>>(tjobs, tb, tj);
+      (wv.rquads ? pack_group_kernel<__nv_bfloat16, __nv_bfloat16, PACK_K_BF16, PACK_READ_ALL>
+                 : pack_group_kernel<__nv_bfloat16, __nv_bfloat16, PACK_K_BF16>)<<<pg, blk, 0, s>>>(tjobs, tb, tj);
     else
-      pack_group_kernel<float, __nv_bfloat16, PACK_K_BF16><<<pg, blk, 0, s>>>(tjobs, tb, tj);
+      (wv.rquads ? pack_group_kernel<float, __nv_bfloat16, PACK_K_BF16, PACK_READ_ALL>
+                 : pack_group_kernel<float, __nv_bfloat16, PACK_K_BF16>)<<<pg, blk, 0, s>>>(tjobs, tb, tj);
     if ((rc = launch_check("pack_group"))) return rc;
   }
   for (int v = 0; v < TCV_COUNT; ++v) {
