@@ -903,47 +903,89 @@ __device__ __forceinline__ int32_t skinny_reg_ko(const SkinnyArgs& a, int kb, in
   return lane < SKR_KR && kb + lane < ke ? __ldg(a.p_k_off + kb + lane) : 0;
 }
 
-// P of the thread's two positions s0, s1 (a pair per k; zeros for null: outside
-// the box) at k [kb, kb + 16), zeros past ke; ko_lane = skinny_reg_ko(a, kb,
-// ke), 0 past ke (those loads read some element of P). quads: every quad of k
-// is 4 consecutive, aligned elements: one 16-byte load each (a warp's loads
-// touch 32 rows of P either way, with a quarter of the instructions: S = 8,
-// K = 720, W = 635040 contracted along its stride-one index 1397 -> 681 us);
-// compiled only into the kernels of such items (KW: with both forms the other
-// items spill, 473 -> 740 us at S = 11, K = 2744).
-template <bool KW>
-__device__ __forceinline__ void skinny_reg_p(int kb, int ke, const float* s0, const float* s1,
-                                             uint64_t (&p)[SKR_KR], int32_t ko_lane, bool quads) {
-  const int n = ke - kb;
-  if (KW && quads) {
+// How a register-path job multiplies and loads P:
+//   SKR_SCALAR  single values (FFMA). For one wave of jobs: a CTA then has its
+//               SM nearly to itself and waits for its own loads, which the
+//               compiler sets earlier in this form (W = 22749, S = 14, K = 152:
+//               22.6 us against 25.2 by pairs; 5060, 9, 334: 31 / 34; 151360, 4,
+//               23: 9.2 / 9.9).
+//   SKR_PAIRS   FP32 pairs (fma.rn.f32x2). With several CTAs on an SM the issue
+//               slots count, of which pairs take half (W = 349920, S = 16, K =
+//               672: 286 us, scalar 316; 635040, 8, 720: 373 / 440; 100000, 13,
+//               3240: 442 / 474).
+//   SKR_QUADS   pairs, and every quad of k is 4 consecutive, aligned elements of
+//               P: one 16-byte load each (a warp's loads touch 32 rows of P
+//               either way, with a quarter of the instructions: S = 8, K = 720, W
+//               = 635040 contracted along its stride-one index 1437 -> 641 us).
+//               A kernel of its own: with both forms in one the other items
+//               spill (473 -> 740 us at S = 11, K = 2744).
+// The same products and order of sums in every form.
+enum SkrForm : int { SKR_SCALAR = 0, SKR_PAIRS = 1, SKR_QUADS = 2 };
+
+// P of the thread's two positions (pw offsets o0, o1, SK_NONE outside the box:
+// zeros; s0, s1: the pair forms' pointers to them, null outside) at k [kb, kb + 16), zeros past ke; ko_lane = skinny_reg_ko(a, kb,
+// ke), 0 past ke (the loads of the pair forms there read some element of P).
+template <int FORM>
+struct SkrP {  // pairs
+  uint64_t v[SKR_KR];
+  __device__ __forceinline__ void load(const SkinnyArgs&, int kb, int ke, int32_t, int32_t,
+                                       const float* s0, const float* s1, int32_t ko_lane, bool quads) {
+    const int n = ke - kb;
+    if (FORM == SKR_QUADS && quads) {
 #pragma unroll
-    for (int kk = 0; kk < SKR_KR; kk += 4) {
-      const int32_t ko = __shfl_sync(0xffffffffu, ko_lane, kk);
-      const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      const float4 x = s0 ? __ldg(reinterpret_cast<const float4*>(s0 + ko)) : z;
-      const float4 y = s1 ? __ldg(reinterpret_cast<const float4*>(s1 + ko)) : z;
-      p[kk] = f32x2(x.x, y.x);
-      p[kk + 1] = f32x2(x.y, y.y);
-      p[kk + 2] = f32x2(x.z, y.z);
-      p[kk + 3] = f32x2(x.w, y.w);
+      for (int kk = 0; kk < SKR_KR; kk += 4) {
+        const int32_t ko = __shfl_sync(0xffffffffu, ko_lane, kk);
+        const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const float4 x = s0 ? __ldg(reinterpret_cast<const float4*>(s0 + ko)) : z;
+        const float4 y = s1 ? __ldg(reinterpret_cast<const float4*>(s1 + ko)) : z;
+        v[kk] = f32x2(x.x, y.x);
+        v[kk + 1] = f32x2(x.y, y.y);
+        v[kk + 2] = f32x2(x.z, y.z);
+        v[kk + 3] = f32x2(x.w, y.w);
+      }
+    } else {
+#pragma unroll
+      for (int kk = 0; kk < SKR_KR; ++kk) {
+        const int32_t ko = __shfl_sync(0xffffffffu, ko_lane, kk);
+        v[kk] = f32x2(s0 ? __ldg(s0 + ko) : 0.0f, s1 ? __ldg(s1 + ko) : 0.0f);
+      }
     }
-  } else {
+    if (n < SKR_KR) {
+#pragma unroll
+      for (int kk = 0; kk < SKR_KR; ++kk)
+        if (kk >= n) v[kk] = 0;
+    }
+  }
+  __device__ __forceinline__ void take(const SkrP& o) {
+#pragma unroll
+    for (int kk = 0; kk < SKR_KR; ++kk) v[kk] = o.v[kk];
+  }
+};
+template <>
+struct SkrP<SKR_SCALAR> {
+  float v0[SKR_KR], v1[SKR_KR];
+  __device__ __forceinline__ void load(const SkinnyArgs& a, int kb, int ke, int32_t o0, int32_t o1,
+                                       const float*, const float*, int32_t ko_lane, bool) {
 #pragma unroll
     for (int kk = 0; kk < SKR_KR; ++kk) {
       const int32_t ko = __shfl_sync(0xffffffffu, ko_lane, kk);
-      p[kk] = f32x2(s0 ? __ldg(s0 + ko) : 0.0f, s1 ? __ldg(s1 + ko) : 0.0f);
+      const bool in = kb + kk < ke;
+      v0[kk] = in && o0 != SK_NONE ? __ldg(a.P + o0 + ko) : 0.0f;
+      v1[kk] = in && o1 != SK_NONE ? __ldg(a.P + o1 + ko) : 0.0f;
     }
   }
-  if (n < SKR_KR) {
+  __device__ __forceinline__ void take(const SkrP& o) {
 #pragma unroll
-    for (int kk = 0; kk < SKR_KR; ++kk)
-      if (kk >= n) p[kk] = 0;
+    for (int kk = 0; kk < SKR_KR; ++kk) {
+      v0[kk] = o.v0[kk];
+      v1[kk] = o.v1[kk];
+    }
   }
-}
+};
 
-// A thread's sums of 2 positions x ROWS rows as pairs (fma.rn.f32x2): v[i][s] =
-// (row 2 i of position s, row 2 i + 1 of position 1 - s).
-template <int ROWS>
+// A thread's sums of 2 positions x ROWS rows. Pairs: v[i][s] = (row 2 i of
+// position s, row 2 i + 1 of position 1 - s).
+template <int ROWS, int FORM>
 struct SkrAcc {
   uint64_t v[ROWS / 2][2];
   __device__ __forceinline__ void clear() {
@@ -953,12 +995,46 @@ struct SkrAcc {
   __device__ __forceinline__ float get(int h, int r) const {
     return r % 2 == 0 ? f32x2_lo(v[r / 2][h]) : f32x2_hi(v[r / 2][1 - h]);
   }
+  // k = kk of the step: q = ROWS values of Q
+  __device__ __forceinline__ void fma_k(const float* q, const SkrP<FORM>& p, int kk) {
+    const uint64_t w = f32x2_swap(p.v[kk]);
+#pragma unroll
+    for (int r = 0; r < ROWS; r += 4) {
+      const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(q + r);
+      v[r / 2][0] = fma_x2(t.x, p.v[kk], v[r / 2][0]);
+      v[r / 2][1] = fma_x2(t.x, w, v[r / 2][1]);
+      v[r / 2 + 1][0] = fma_x2(t.y, p.v[kk], v[r / 2 + 1][0]);
+      v[r / 2 + 1][1] = fma_x2(t.y, w, v[r / 2 + 1][1]);
+    }
+  }
+};
+template <int ROWS>
+struct SkrAcc<ROWS, SKR_SCALAR> {
+  float v[2][ROWS];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) v[0][r] = v[1][r] = 0.0f;
+  }
+  __device__ __forceinline__ float get(int h, int r) const { return v[h][r]; }
+  __device__ __forceinline__ void fma_k(const float* q, const SkrP<SKR_SCALAR>& p, int kk) {
+    float qv[ROWS];
+#pragma unroll
+    for (int r = 0; r < ROWS; r += 4) {
+      const float4 t = *reinterpret_cast<const float4*>(q + r);
+      qv[r] = t.x; qv[r + 1] = t.y; qv[r + 2] = t.z; qv[r + 3] = t.w;
+    }
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      v[0][r] = fmaf(qv[r], p.v0[kk], v[0][r]);
+      v[1][r] = fmaf(qv[r], p.v1[kk], v[1][r]);
+    }
+  }
 };
 
 // The end of a job: raw sums to its k slice, or the rows to C (staged in os).
-template <int ROWS>
+template <int ROWS, int FORM>
 __device__ __forceinline__ void skinny_reg_finish(const SkinnyArgs& a, const SkJob& j,
-                                                  const SkrAcc<ROWS>& acc, float* os,
+                                                  const SkrAcc<ROWS, FORM>& acc, float* os,
                                                   const int32_t* cw, const int32_t* cs) {
   const int tid = threadIdx.x;
   if (a.partial) {  // layout of the 16-row (RS = 4) tile path; rows >= ROWS not written
@@ -1008,7 +1084,7 @@ __device__ __forceinline__ void skinny_reg_finish(const SkinnyArgs& a, const SkJ
 
 // One job of the register path with ROWS computed rows (16, or 8 for a
 // narrow side of at most 8: half the FMAs and Q copies).
-template <int ROWS, bool KW>
+template <int ROWS, int FORM>
 __device__ __forceinline__ void skinny_reg_job(const SkinnyArgs& a, const SkJob& job, float* Qs,
                                                float* os, const int32_t* pw, const int32_t* cw,
                                                const int32_t* cs) {
@@ -1016,24 +1092,24 @@ __device__ __forceinline__ void skinny_reg_job(const SkinnyArgs& a, const SkJob&
   const int32_t po0 = pw[tid], po1 = pw[tid + SKR_THREADS];
   const int kbeg = job.c0 * SK_KC;
   const int kend = job.c1 * SK_KC < a.K ? job.c1 * SK_KC : a.K;
-  SkrAcc<ROWS> acc;
+  SkrAcc<ROWS, FORM> acc;
   acc.clear();
-  const bool quads = KW && a.p_vec;
-  uint64_t pc[SKR_KR];
+  const bool quads = FORM == SKR_QUADS && a.p_vec;
+  SkrP<FORM> pc;
   const float* s0 = po0 != SK_NONE ? a.P + po0 : nullptr;
   const float* s1 = po1 != SK_NONE ? a.P + po1 : nullptr;
   skinny_reg_q<ROWS>(a, kbeg, kend, Qs);
-  skinny_reg_p<KW>(kbeg, kend, s0, s1, pc, skinny_reg_ko(a, kbeg, kend), quads);
+  pc.load(a, kbeg, kend, po0, po1, s0, s1, skinny_reg_ko(a, kbeg, kend), quads);
   int32_t ko_next = skinny_reg_ko(a, kbeg + SKR_KR, kend);  // the next step's
   int st = 0;
 #pragma unroll 1
   for (int kb = kbeg; kb < kend; kb += SKR_KR) {
     const int nb = kb + SKR_KR;
-    uint64_t pn[SKR_KR];
+    SkrP<FORM> pn;
     if (nb < kend) {
       __syncthreads();  // stage st ^ 1 was read by the previous step
       skinny_reg_q<ROWS>(a, nb, kend, Qs + (st ^ 1) * SKR_KR * SKR_ROWS);
-      skinny_reg_p<KW>(nb, kend, s0, s1, pn, ko_next, quads);
+      pn.load(a, nb, kend, po0, po1, s0, s1, ko_next, quads);
       ko_next = skinny_reg_ko(a, nb + SKR_KR, kend);
       cp_async_wait<1>();
     } else {
@@ -1042,27 +1118,14 @@ __device__ __forceinline__ void skinny_reg_job(const SkinnyArgs& a, const SkJob&
     __syncthreads();  // Q of this step landed
     const float* q = Qs + st * SKR_KR * SKR_ROWS;
 #pragma unroll
-    for (int kk = 0; kk < SKR_KR; ++kk) {
-      const uint64_t w = f32x2_swap(pc[kk]);
-#pragma unroll
-      for (int r = 0; r < ROWS; r += 4) {
-        const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(q + kk * ROWS + r);
-        acc.v[r / 2][0] = fma_x2(t.x, pc[kk], acc.v[r / 2][0]);
-        acc.v[r / 2][1] = fma_x2(t.x, w, acc.v[r / 2][1]);
-        acc.v[r / 2 + 1][0] = fma_x2(t.y, pc[kk], acc.v[r / 2 + 1][0]);
-        acc.v[r / 2 + 1][1] = fma_x2(t.y, w, acc.v[r / 2 + 1][1]);
-      }
-    }
-    if (nb < kend) {
-#pragma unroll
-      for (int kk = 0; kk < SKR_KR; ++kk) pc[kk] = pn[kk];
-    }
+    for (int kk = 0; kk < SKR_KR; ++kk) acc.fma_k(q + kk * ROWS, pc, kk);
+    if (nb < kend) pc.take(pn);
     st ^= 1;
   }
-  skinny_reg_finish<ROWS>(a, job, acc, os, cw, cs);
+  skinny_reg_finish<ROWS, FORM>(a, job, acc, os, cw, cs);
 }
 
-template <int ROWS, bool KW, typename Resolve>
+template <int ROWS, int FORM, typename Resolve>
 __device__ __forceinline__ void skinny_reg_loop(int j0, int jstep, int njobs, Resolve&& resolve,
                                                 uint8_t* smem) {
   float* Qs = reinterpret_cast<float*>(smem);  // [2][KR][ROWS], stages SKR_ROWS rows apart
@@ -1078,24 +1141,23 @@ __device__ __forceinline__ void skinny_reg_loop(int j0, int jstep, int njobs, Re
     __syncthreads();  // the previous job's stores are done with os, pw, cw, cs
     skinny_reg_begin(a, job.b, pw, cw, cs);
     __syncthreads();
-    skinny_reg_job<ROWS, KW>(a, job, Qs, os, pw, cw, cs);
+    skinny_reg_job<ROWS, FORM>(a, job, Qs, os, pw, cw, cs);
   }
 }
 
 // ROWS = 16, or 8 for a narrow side of at most 8 (one kernel per row count:
 // both in one kernel would need more registers than four CTAs per SM leave)
-// KW: items with quads of k (SK_P_K).
-template <int ROWS, bool KW>
+template <int ROWS, int FORM>
 __global__ void __launch_bounds__(SKR_THREADS, SKR_CTAS_PER_SM)
     skinny_reg_kernel(const __grid_constant__ SkinnyArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
   grid_dep_wait();
   auto resolve = [&](int J) { return SkRef{&a, J}; };
-  skinny_reg_loop<ROWS, KW>(blockIdx.x, gridDim.x, a.njobs, resolve, smem);
+  skinny_reg_loop<ROWS, FORM>(blockIdx.x, gridDim.x, a.njobs, resolve, smem);
   bulk_wait_all();  // bulk C copies complete before the CTA exits
 }
 
-template <int ROWS, bool KW>
+template <int ROWS, int FORM>
 __global__ void __launch_bounds__(SKR_THREADS, SKR_CTAS_PER_SM)
     skinny_reg_group_kernel(const SkinnyItem* items, const int64_t* begin, int n, int njobs) {
   extern __shared__ __align__(16) uint8_t smem[];
@@ -1103,7 +1165,7 @@ __global__ void __launch_bounds__(SKR_THREADS, SKR_CTAS_PER_SM)
     const SkinnyItem& it = items[find_segment(begin, n, J)];
     return SkRef{&it.args, (int)(J - it.begin)};
   };
-  skinny_reg_loop<ROWS, KW>(blockIdx.x, gridDim.x, njobs, resolve, smem);
+  skinny_reg_loop<ROWS, FORM>(blockIdx.x, gridDim.x, njobs, resolve, smem);
   bulk_wait_all();
 }
 

@@ -1565,18 +1565,12 @@ static cudaError_t set_attrs() {
                            (int)SKT_SMEM_BYTES));
   chk(cudaFuncSetAttribute(skinny_tc_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)SKT_SMEM_BYTES));
-  chk(cudaFuncSetAttribute(skinny_reg_kernel<8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)SKR_SMEM_BYTES));
-  chk(cudaFuncSetAttribute(skinny_reg_kernel<8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)SKR_SMEM_BYTES));
-  chk(cudaFuncSetAttribute(skinny_reg_kernel<16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)SKR_SMEM_BYTES));
-  chk(cudaFuncSetAttribute(skinny_reg_kernel<16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)SKR_SMEM_BYTES));
-  chk(cudaFuncSetAttribute(skinny_reg_group_kernel<16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)SKR_SMEM_BYTES));
-  chk(cudaFuncSetAttribute(skinny_reg_group_kernel<16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)SKR_SMEM_BYTES));
+  for (auto kernel : {skinny_reg_kernel<8, SKR_SCALAR>, skinny_reg_kernel<8, SKR_PAIRS>,
+                      skinny_reg_kernel<8, SKR_QUADS>, skinny_reg_kernel<16, SKR_SCALAR>,
+                      skinny_reg_kernel<16, SKR_PAIRS>, skinny_reg_kernel<16, SKR_QUADS>})
+    chk(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SKR_SMEM_BYTES));
+  for (auto kernel : {skinny_reg_group_kernel<16, SKR_PAIRS>, skinny_reg_group_kernel<16, SKR_QUADS>})
+    chk(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SKR_SMEM_BYTES));
   chk(cudaFuncSetAttribute(skinny_reduce_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)SK_SMEM_BYTES));
   chk(cudaFuncSetAttribute(gett_tc2_kernel<TC_BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2275,6 +2269,14 @@ static bool reg_quads(const tccg_plan* p) {
   return p->sk_reg && p->sk.p_walk == SK_P_K && p->sk_p_vec;
 }
 
+// The register path's jobs are few enough for its scalar form (SkrForm): one per
+// SM, or one wave of short ones (at most 4 chunks of K each: the loads' wait is
+// most of their time; 391 jobs of 3240 k are faster by pairs).
+static bool reg_one_wave(const tccg_plan* p) {
+  return p->sk.njobs <= p->num_sms ||
+         (p->sk.chunks_per_split <= 4 && p->sk.njobs <= (int64_t)SKR_CTAS_PER_SM * p->num_sms);
+}
+
 static int run_skinny(const tccg_plan* p, const void* GA, const void* GB, float* C, float alpha,
                       float beta, char* w, cudaStream_t s) {
   if (p->sk_tc) return run_skinny_tc(p, GA, GB, C, alpha, beta, w, s);
@@ -2283,10 +2285,14 @@ static int run_skinny(const tccg_plan* p, const void* GA, const void* GB, float*
   if (p->sk_reg) {
     const int64_t grid = std::min<int64_t>(a.njobs, (int64_t)SKR_CTAS_PER_SM * p->num_sms);
     // 8 computed rows for a narrow side of at most 8, else 16
-    const bool kw = reg_quads(p);
+    const bool kw = reg_quads(p), one_wave = reg_one_wave(p);
     launch_after(false, p,
-                 a.S <= 8 ? (kw ? skinny_reg_kernel<8, true> : skinny_reg_kernel<8, false>)
-                          : (kw ? skinny_reg_kernel<16, true> : skinny_reg_kernel<16, false>),
+                 a.S <= 8 ? (kw         ? skinny_reg_kernel<8, SKR_QUADS>
+                             : one_wave ? skinny_reg_kernel<8, SKR_SCALAR>
+                                        : skinny_reg_kernel<8, SKR_PAIRS>)
+                          : (kw         ? skinny_reg_kernel<16, SKR_QUADS>
+                             : one_wave ? skinny_reg_kernel<16, SKR_SCALAR>
+                                        : skinny_reg_kernel<16, SKR_PAIRS>),
                  dim3((unsigned)grid), dim3(SKR_THREADS), SKR_SMEM_BYTES, s, a);
   } else {
     const int64_t grid = std::min<int64_t>(a.njobs, (int64_t)SK_CTAS_PER_SM * p->num_sms);
@@ -3250,7 +3256,7 @@ static int run_wave(const tccg_group* g, const tccg_group::Wave& wv, cudaStream_
         // item alone
         const unsigned grid =
             (unsigned)std::min<int64_t>(wv.sk_jobs[cls], (int64_t)SKR_CTAS_PER_SM * g->num_sms);
-        auto kernel = cls == 3 ? skinny_reg_group_kernel<16, true> : skinny_reg_group_kernel<16, false>;
+        auto kernel = cls == 3 ? skinny_reg_group_kernel<16, SKR_QUADS> : skinny_reg_group_kernel<16, SKR_PAIRS>;
         kernel<<<grid, SKR_THREADS, SKR_SMEM_BYTES, s_sk>>>(
             g->d_sk + wv.sk0[cls], g->b_sk + wv.sk0[cls], wv.nsk[cls], (int)wv.sk_jobs[cls]);
       } else {
