@@ -690,9 +690,13 @@ static bool skinny_geometry(tccg_plan* p, std::vector<int>& ym, int* xmode, bool
   p->sk_p_vec = a.p_walk == SK_P_X && a.px == 1 && k4;
   // P's stride-one index contracted: quads of k as 16-byte loads (the run
   // checks P's alignment); on the register path only for 8 chunks and more
-  // (S = 9, K = 168: 811 us with them off, 830 on)
+  // (S = 9, K = 168: 811 us with them off, 830 on) and where positions are 12
+  // elements apart or more: nearer ones share the lines that single loads touch
+  // (K = 576 in runs of 8, W = 374400, S = 14: 433 us single, 501 by quads; K =
+  // 864 in runs of 12, W = 18720, S = 8: 42.5 / 37.2; 1152 of 16: 72 / 48)
   if (a.p_walk == SK_P_K)
-    p->sk_p_vec = (sn ? p->ks_a : p->ks_b) && p->K % 4 == 0 && (tc || a.nchunks >= 8);
+    p->sk_p_vec = (sn ? p->ks_a : p->ks_b) && p->K % 4 == 0 &&
+                  (tc || (a.nchunks >= 8 && min_abs_stride(nw, wext, wp) >= 12));
   build_offsets(nsm, sext, sc, t);
   auto affine = [&](int64_t st) {
     for (size_t i = 0; i < t.size(); ++i)
