@@ -305,32 +305,54 @@ static double simt_time(const tccg_plan* p) {
   return std::max(2.0 * simt_work * K / 35e12, (cb + simt_passes * op) / 4.5e12);
 }
 
-// FP32 as six bf16 products on the tensor cores (TC_F32X6). Its normwise error
-// against FP64 on N(0, 1) values is below FFMA's at every K measured (K = 64:
-// 0.7e-7 against 1.4e-7, 256: 1.2e-7 / 2.9e-7, 1024: 1.3e-7 / 5.7e-7, 4096:
-// 1.6e-7 / 1.15e-6; the same order for uniform and for wide-ranged values),
-// so time decides: tiles of 128 x 160 (the MMAs of one column of tiles only as
-// wide as N) at 0.72 us per 32 k and round of the persistent grid (half rounds
-// where the tail split applies), the pack's 4 + 6 and the loads' 6 bytes per
+// FP32 as six bf16 products on the tensor cores (TC_F32X6), where its error is no
+// larger than that of the FFMA form (f32_split_chunk) and the time model finds
+// it faster: tiles of 128 x 160 (the MMAs of one column of tiles only as wide
+// as N) at 0.72 us per 32 k and round of the persistent grid (half rounds
+// where the tail split applies; chunks of 3, 2 and 1 k-blocks 1.06, 1.12 and
+// 1.33 times that), the pack's 4 + 6 and the loads' 6 bytes per
 // element at 4.5 TB/s, the k-split's partial sums and 20 us of launches,
 // against FFMA at 45 TFLOP/s on padded tiles with its own operand passes and 8
-// us. 2048 x 2080 x K, us: K = 128 31.8 against 35.6 (both near the launch
-// floor; the rule keeps FFMA), 256: 38 / 59, 512: 54 / 106, 4096: 228 / 773.
+// us. 2048 x 2080 x K, us: K = 256 40 against 56, 512 54 / 106, 4096 228 / 773.
 // Plans for groups (tail_split < 0) share their launches: 5 us. With a
 // k-split the model is less sure of both sides: by 1.25x at least. A tuning that
 // names a CUDA-core form (variant < 0, direct, shortk, simt_tile, an explicit
-// k-split) keeps the CUDA cores; variant > 0 asks for this path.
-static constexpr int64_t F32X6_MIN_K = 128;  // an accumulation chunk
+// k-split) keeps the CUDA cores; variant > 0 asks for this path, whatever K.
 static constexpr int64_t F32X6_MIN_KB = 8;   // k-blocks of a k-split slice
 static constexpr int F32X6_BM = TcCfgT<TC_F32X6>::BM, F32X6_BN = TcCfgT<TC_F32X6>::BN;
+
+// k slices of the CUDA-core tile kernel with tile shape `shape` (at least 8
+// k-tiles each, min_blocks CTAs per SM); returns the k-tiles per slice.
+static int64_t simt_ksplit(const tccg_plan* p, int shape, int32_t* splits) {
+  int BM, BN, BK;
+  simt_dims(p->prec == TCCG_PREC_FP64, shape, &BM, &BN, &BK);
+  const int min_blocks = shape == SIMT_SQUARE ? SimtCfg<float>::MIN_BLOCKS
+                                              : SimtCfg<float, SIMT_NARROW_N>::MIN_BLOCKS;
+  return choose_ksplit(p->tune.ksplit, cdiv(p->M, BM) * cdiv(p->N, BN), cdiv(p->K, BK),
+                       min_blocks * (int64_t)p->num_sms, 8, splits);
+}
+
+// The accumulation chunk of an FP32 plan on the tensor cores, in k-blocks: the
+// tuning's (at most 4: 6400 k in one gave an error of 6e-6), or by the FFMA
+// form's chains; 0 = FFMA.
+static int f32x6_chunk(const tccg_plan* p) {
+  if (p->tune.variant > 0) return std::min(p->tune.variant, 4);
+  const int shape = choose_simt_shape(p, nullptr);
+  int32_t splits = 1;
+  int BM, BN, BK;
+  simt_dims(false, shape, &BM, &BN, &BK);
+  const int64_t chain = std::min<int64_t>(p->K, simt_ksplit(p, shape, &splits) * BK);
+  return f32_split_chunk(chain, splits);
+}
+
 static bool choose_f32x6(const tccg_plan* p) {
   const tccg_tuning& t = p->tune;
   if (p->prec != TCCG_PREC_FP32 || p->dtype != TCCG_F32 || t.method != TCCG_METHOD_GETT || t.pair ||
       t.variant < 0 || t.ksplit > 1 || t.direct > 0 || t.shortk > 0 || t.simt_tile != 0)
     return false;
   if (!f32_split_fits(p->M, p->N, p->K)) return false;
-  if (t.variant > 0) return true;
-  if (p->K < F32X6_MIN_K) return false;
+  const int chunk = f32x6_chunk(p);
+  if (t.variant > 0 || chunk == 0) return chunk > 0;
   const int64_t tiles = cdiv(p->M, F32X6_BM) * cdiv(p->N, F32X6_BN), kb = cdiv(p->K, 32);
   int32_t split = 1;
   const int64_t per =
@@ -338,16 +360,17 @@ static bool choose_f32x6(const tccg_plan* p) {
   const double rounds =
       split > 1 ? 1.0 : std::max(1.0, 0.5 * (double)cdiv(2 * tiles, p->num_sms));
   const double width =
-      p->N >= F32X6_BN ? 1.0 : std::max(0.4, (double)round_up(p->N, 32) / F32X6_BN);
+      (p->N >= F32X6_BN ? 1.0 : std::max(0.4, (double)round_up(p->N, 32) / F32X6_BN)) *
+      (chunk >= 4 ? 1.0 : chunk >= 3 ? 1.06 : chunk >= 2 ? 1.12 : 1.33);
   const double M = (double)p->M, N = (double)p->N, K = (double)p->K;
   double t_tc = rounds * (double)per * 0.72e-6 * width + (M + N) * K * 16.0 / 4.5e12 +
                 (t.tail_split < 0 ? 5e-6 : 20e-6);
   if (split > 1) t_tc += 8.0 * split * M * N / 3e12 + 3e-6;
   double work = 0;
   const int shape = choose_simt_shape(p, &work);
-  const double t_ffma = 2.0 * work * K / 45e12 +
-                        (direct_eligible(p, shape) ? 4.0 : 12.0) * (M + N) * K / 4.5e12 +
-                        (t.tail_split < 0 ? 2e-6 : 8e-6);
+  double t_ffma = 2.0 * work * K / 45e12 +
+                  (direct_eligible(p, shape) ? 4.0 : 12.0) * (M + N) * K / 4.5e12 +
+                  (t.tail_split < 0 ? 2e-6 : 8e-6);
   return (split > 1 || 2 * tiles < p->num_sms ? 1.25 : 1.0) * t_tc < t_ffma;
 }
 
@@ -1257,17 +1280,13 @@ static int plan_layout(tccg_plan* p) {
     simt_dims(dbl, p->simt_shape, &BM, &BN, &BK);
     p->simt_bm = BM;
     p->simt_bn = BN;
-    const int min_blocks = p->simt_shape == SIMT_SQUARE ? SimtCfg<float>::MIN_BLOCKS
-                                                        : SimtCfg<float, SIMT_NARROW_N>::MIN_BLOCKS;
     const size_t es = dbl ? 8 : 4;
     p->Mp = round_up(p->M, BM);
     p->Np = round_up(p->N, BN);
     p->Kp = round_up(p->K, BK);
     p->ktiles = (int32_t)(p->Kp / BK);
     const int64_t tiles = (p->Mp / BM) * (p->Np / BN);
-    // min_blocks CTAs per SM; a slice is at least 8 k-tiles
-    p->ktiles_per_split = (int32_t)choose_ksplit(p->tune.ksplit, tiles, p->ktiles,
-                                                 min_blocks * (int64_t)p->num_sms, 8, &p->ksplit);
+    p->ktiles_per_split = (int32_t)simt_ksplit(p, p->simt_shape, &p->ksplit);
     p->direct = choose_direct(p);
     choose_gather_k(p);
     p->shortk = choose_shortk(p, tiles);
@@ -1304,10 +1323,8 @@ static int plan_layout(tccg_plan* p) {
       p->num_kb = (int32_t)cdiv(p->K, 64);
     }
     // BF16X3 accumulates 512 k per TMEM accumulator (tuning.variant overrides,
-    // in k-blocks of 32), FP32 at most 128 (its error bound needs short
-    // chunks: 6400 k in one gave 6e-6); BF16 one chunk per tile
-    p->chunk_kb = x3 || x6 ? (p->tune.variant > 0 ? p->tune.variant : x6 ? 4 : 16) : p->num_kb;
-    if (x6) p->chunk_kb = std::min(p->chunk_kb, 4);
+    // in k-blocks of 32), FP32 at most 128 (f32x6_chunk); BF16 one chunk per tile
+    p->chunk_kb = x6 ? f32x6_chunk(p) : x3 ? (p->tune.variant > 0 ? p->tune.variant : 16) : p->num_kb;
     if (p->chunk_kb < 1) p->chunk_kb = 1;
     const bool pair = p->tune.pair != 0;
     int stages = 0;

@@ -12,6 +12,7 @@ from tccg_b200 import build
 WRAP = """
 #include "f32_split_rule.h"
 extern "C" int fits(long long m, long long n, long long k) { return tccg::f32_split_fits(m, n, k); }
+extern "C" int chunk(long long chain, long long splits) { return tccg::f32_split_chunk(chain, splits); }
 """
 
 
@@ -27,6 +28,7 @@ def rule(tmp_path_factory):
     subprocess.run([gxx, "-std=c++17", "-shared", "-fPIC", "-I" + build.CSRC, src, "-o", out], check=True)
     lib = ctypes.CDLL(out)
     lib.fits.argtypes = [ctypes.c_longlong] * 3
+    lib.chunk.argtypes = [ctypes.c_longlong] * 2
     return lib
 
 
@@ -42,3 +44,13 @@ def test_last_packed_column_is_a_tma_coordinate(rule, k):
 
 def test_rows(rule):
     assert rule.fits((1 << 30) - 1, 8, 64) and not rule.fits(1 << 30, 8, 64) and not rule.fits(8, 1 << 30, 64)
+
+
+def test_chunk_follows_the_chain(rule):
+    """No split below a chain of 256 adds; a chunk's truncations (2 per k-block)
+    at most a 48th of the chain's roundings plus 3 up to the longest chunk."""
+    assert rule.chunk(255, 1) == 0 and rule.chunk(256, 1) == 1
+    assert rule.chunk(128, 2) == 1 and rule.chunk(400, 28) == 1 and rule.chunk(2 * 768, 2) == 3
+    chunks = [rule.chunk(c, 1) for c in range(0, 5000)]
+    assert chunks == sorted(chunks) and max(chunks) == 4
+    assert all(2 * k <= c / 48 + 3 for c, k in enumerate(chunks))
