@@ -314,6 +314,9 @@ static double simt_time(const tccg_plan* p) {
 // element at 4.5 TB/s, the k-split's partial sums and 20 us of launches,
 // against FFMA at 45 TFLOP/s on padded tiles with its own operand passes and 8
 // us. 2048 x 2080 x K, us: K = 256 40 against 56, 512 54 / 106, 4096 228 / 773.
+// Where C goes out in short runs (crun) the tcgen05 epilogue is the slower one:
+// 152 x 42240 x 260 in runs of 8 beta = 1 303 us against 210 (beta = 0 156 / 160);
+// 900 x 1599 x 266 of 18 68 / 48; 1024 x 2048 x 1024 of 8 90 / 126.
 // Plans for groups (tail_split < 0) share their launches: 5 us. With a
 // k-split the model is less sure of both sides: by 1.25x at least. A tuning that
 // names a CUDA-core form (variant < 0, direct, shortk, simt_tile, an explicit
@@ -371,6 +374,10 @@ static bool choose_f32x6(const tccg_plan* p) {
   double t_ffma = 2.0 * work * K / 45e12 +
                   (direct_eligible(p, shape) ? 4.0 : 12.0) * (M + N) * K / 4.5e12 +
                   (t.tail_split < 0 ? 2e-6 : 8e-6);
+  if (p->crun > 0) {  // C in short runs, read too (beta may be 1): us per MB of C
+    t_tc += 6e-12 * 4.0 * M * N;
+    t_ffma += 2e-12 * 4.0 * M * N;
+  }
   return (split > 1 || 2 * tiles < p->num_sms ? 1.25 : 1.0) * t_tc < t_ffma;
 }
 
