@@ -711,32 +711,45 @@ __global__ void __launch_bounds__(256, SimtCfg<T, S>::MIN_BLOCKS) simt_gett_kern
 
 // FP32 contractions that run as products of the operands' three-way bf16
 // splits (TC_F32X6) but whose values the splits do not represent: the tile
-// kernel on operands packed by the tensor-core kernel (f32_fallback_pack; in a
-// group: on the caller's tensors). Launched behind the tensor-core kernel;
-// its CTAs read the range words and leave at once in the ordinary case, so
-// the grid is one persistent wave, not one CTA per tile.
+// kernel on operands packed by the tensor-core kernel (f32_fallback_pack),
+// with the k slices of the FFMA plan. Launched behind the tensor-core kernel;
+// in the ordinary case the CTAs read the range words and leave at once.
 struct F32FallbackItem {
-  SimtArgs<float> args;  // no k-split
+  SimtArgs<float> args;
   const uint32_t* range;
   int32_t K, tiles_m;
-  int64_t tiles;
+  int64_t tiles, jobs;  // tiles x k slices
 };
 
-template <int LOAD>
-__device__ __forceinline__ void f32_fallback(const F32FallbackItem& it) {
-  if (f32_split_exact(it.range, it.K)) return;
-  for (int64_t t = blockIdx.x; t < it.tiles; t += gridDim.x)
-    simt_gett_tile<float, LOAD>(it.args, (int)(t % it.tiles_m), (int)(t / it.tiles_m), 0);
+__device__ __forceinline__ void f32_fallback_job(const F32FallbackItem& it, int64_t j) {
+  const int64_t t = j % it.tiles;
+  simt_gett_tile<float, SIMT_PACKED>(it.args, (int)(t % it.tiles_m), (int)(t / it.tiles_m),
+                                     (int)(j / it.tiles));
 }
 
-__global__ void __launch_bounds__(256, 2) f32_fallback_kernel(const F32FallbackItem it) {
+// One CTA per job: 1024 CTAs that leave cost 1 us; the same tiles by 296
+// persistent CTAs take 15 % longer (they all store at the same time, and the
+// loop spills). With one infinity, us, the FFMA plan / this path: 4096 x 4096 x
+// 1024 673 / 716, 13824 x 13824 x 1024 7300 / 7235, 512 x 700 x 3000 70 / 101,
+// 12648 x 85 x 4418 516 / 789 (three passes over the operands).
+__global__ void __launch_bounds__(256, 2)
+    f32_fallback_kernel(const __grid_constant__ F32FallbackItem it) {
   grid_dep_wait();  // range words of the packing pass; C written by nobody before this
-  f32_fallback<SIMT_PACKED>(it);
+  if (!f32_split_exact(it.range, it.K)) f32_fallback_job(it, blockIdx.x);
 }
 
+// Grouped: a persistent wave; the jobs of the items that need it, one item's
+// after another's, go round the grid.
 __global__ void __launch_bounds__(256, 2)
     f32_fallback_group_kernel(const F32FallbackItem* items, int n_items) {
-  for (int i = 0; i < n_items; ++i) f32_fallback<SIMT_DIRECT>(items[i]);
+  const int64_t g = gridDim.x;
+  int64_t first = 0;  // the CTA that takes the item's first job
+  for (int i = 0; i < n_items; ++i) {
+    const F32FallbackItem& it = items[i];
+    if (f32_split_exact(it.range, it.K)) continue;
+    for (int64_t j = (blockIdx.x + g - first) % g; j < it.jobs; j += g) f32_fallback_job(it, j);
+    first = (first + it.jobs) % g;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1084,9 +1097,11 @@ __global__ void __launch_bounds__(256) simt_reduce_kernel(const T* __restrict__ 
                                                           int64_t M, int64_t N, T* C,
                                                           const int64_t* c_m_off,
                                                           const int64_t* c_n_off, T alpha,
-                                                          T beta, const uint32_t* range, int K) {
+                                                          T beta, const uint32_t* range, int K,
+                                                          bool fallback) {
   grid_dep_wait();  // partial sums written by the GETT kernel before
-  if (range && !f32_split_exact(range, K)) return;  // computed by f32_fallback_kernel
+  // an FP32 plan on the tensor cores: its slices, or the fallback's
+  if (range && f32_split_exact(range, K) == fallback) return;
   const int64_t m = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (m >= M) return;
   const int64_t cmo = c_m_off[m];
@@ -1117,6 +1132,7 @@ struct ReduceJob {
   int32_t ncols;  // columns per CTA: fewer when there are many slices
   int32_t K;
   const uint32_t* range;  // FP32 on the tensor cores: the item's range words, or null
+  int32_t fallback;       // its fallback's slices, not the split products'
 };
 
 template <typename T>
@@ -1124,7 +1140,7 @@ __global__ void __launch_bounds__(256) reduce_group_kernel(const ReduceJob<T>* j
                                                            const int64_t* begin, int n_jobs) {
   const int64_t t = blockIdx.x;
   const ReduceJob<T> j = jobs[find_segment(begin, n_jobs, t)];  // fields loaded up front
-  if (j.range && !f32_split_exact(j.range, j.K)) return;  // computed by f32_fallback_group_kernel
+  if (j.range && f32_split_exact(j.range, j.K) == (j.fallback != 0)) return;
   const int64_t local = t - j.begin;
   const int64_t m = (local % j.mblocks) * 256 + threadIdx.x;
   if (m >= j.M) return;

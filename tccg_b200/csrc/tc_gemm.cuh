@@ -188,10 +188,11 @@ struct TcArgs {
   // C by the first N mode: stores go through shared memory in runs of e0 m
   // by 32 / e0 columns, which are consecutive addresses of C
   int32_t crun;
-  // TC_F32X6: the operands' range words (AbsRange, GA's two then GB's); where
-  // the fallback takes packed operands (not in groups), their place
+  // TC_F32X6: the operands' range words (AbsRange, GA's two then GB's); the
+  // place of the fallback's packed operands and whether they are read along k
   const uint32_t* range;
   float* fb_pack[2];
+  int32_t fb_kfast[2];
   // C's element offsets all fit 31 bits: the epilogue passes column offsets
   // around as 32-bit values
   int32_t c32;
@@ -1136,36 +1137,70 @@ __global__ void __launch_bounds__(TcCfgT<MODE, LOAD, BNV>::NUM_THREADS, 1)
   gett_tc_body<MODE, LOAD, BNV, false>(&tmA, &tmB, &a, g, a.status);
 }
 
+// Operands of the FFMA fallback, packed as PACK_MN does (rows padded to 128, k
+// to 16, zeros) in the memory of the split ones, which nobody reads then: by
+// the tensor-core kernel, which has nothing else to do, so that the ordinary
+// case pays no launch. A warp per 32 rows x 32 k, read along the operand's fast
+// index, turned through the warp's 4 KB of shared memory where that is k.
+// sm: (threads / 32) x 32 x 33 floats, free of other use.
+static __device__ __noinline__ void f32_fallback_pack(const TcArgs& a, int threads, float* sm) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float* t = sm + warp * (32 * 33);
+  const int64_t step = (int64_t)gridDim.x * (threads / 32);
+#pragma unroll 1
+  for (int o = 0; o < 2; ++o) {
+    const int64_t R = o ? a.N : a.M, Rp = (R + 127) / 128 * 128, K = a.K, Kp = (K + 15) / 16 * 16;
+    const int64_t kt = (Kp + 31) / 32, tiles = Rp / 32 * kt;
+    const int64_t* const row = a.grow[o];
+    const int64_t* const col = a.gk[o];
+    const float* const src = a.gsrc[o];
+    float* const dst = a.fb_pack[o];
+    const bool kfast = a.fb_kfast[o] != 0;
+#pragma unroll 1
+    for (int64_t i = (int64_t)blockIdx.x * (threads / 32) + warp; i < tiles; i += step) {
+      const int64_t r0 = i / kt * 32, k0 = i % kt * 32;
+      // this lane's row and k; offset 0 and no load where they lie outside
+      const bool rok = r0 + lane < R, kok = k0 + lane < K;
+      const int64_t ro = rok ? __ldg(row + r0 + lane) : 0, ko = kok ? __ldg(col + k0 + lane) : 0;
+      float v[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        const int64_t off = (kfast ? ko : ro) + __shfl_sync(0xffffffffu, kfast ? ro : ko, j);
+        const bool in = kfast ? kok && r0 + j < R : rok && k0 + j < K;
+        v[j] = in ? __ldg(src + off) : 0.0f;
+      }
+      if (kfast) {
+        __syncwarp();  // the tile before was read
+#pragma unroll
+        for (int j = 0; j < 32; ++j) t[j * 33 + lane] = v[j];
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = t[lane * 33 + j];
+      }
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        if (k0 + j < Kp) dst[(k0 + j) * Rp + r0 + lane] = v[j];
+    }
+  }
+}
+
+// After the tensor-core body of an FP32 kernel: packs for the fallback if this
+// contraction needs it. All threads; the body's shared memory is free.
+template <int MODE, int LOAD, int BNV>
+__device__ __forceinline__ void f32_fallback_prepare(const TcArgs& a) {
+  using Cfg = TcCfgT<MODE, LOAD, BNV>;
+  static_assert(Cfg::NUM_THREADS / 32 * 32 * 33 * 4 <= Cfg::SMEM_BYTES, "transposition tiles fit");
+  extern __shared__ uint8_t smem_raw[];
+  if (!f32_split_exact(a.range, a.K))
+    f32_fallback_pack(a, Cfg::NUM_THREADS, reinterpret_cast<float*>(smem_raw));
+}
+
 template <int MODE, int LOAD = TC_LOAD_TMA, int BNV = 0>
 __global__ void __launch_bounds__(TcCfgT<MODE, LOAD, BNV>::NUM_THREADS, 1)
     gett_tc_group_kernel(const TcGroup g, int32_t* status) {
   gett_tc_body<MODE, LOAD, BNV, true>(nullptr, nullptr, nullptr, g, status);
-}
-
-// Operands of the FFMA fallback, packed as PACK_MN does (rows padded to 128, k
-// to 16, zeros) in the memory of the split ones, which nobody reads then: by
-// the tensor-core kernel, which has nothing else to do, so that the ordinary
-// case pays no launch. 4096 x 4096 x 1024 with one element of 1e-37: 0.97 ms;
-// 1.39 with the fallback reading the caller's tensors element by element. (The
-// FFMA plan, with its 16-byte packs and k slices, 0.66; split products 0.21.)
-static __device__ __noinline__ void f32_fallback_pack(const TcArgs& a, int threads) {
-  constexpr int U = 4;
-#pragma unroll 1
-  for (int o = 0; o < 2; ++o) {
-    const int64_t R = o ? a.N : a.M, Rp = (R + 127) / 128 * 128, Kp = ((int64_t)a.K + 15) / 16 * 16;
-    const int64_t step = (int64_t)gridDim.x * threads, total = Rp * Kp;
-    for (int64_t i0 = (int64_t)blockIdx.x * threads + threadIdx.x; i0 < total; i0 += U * step) {
-      float v[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int64_t i = i0 + u * step, k = i / Rp, r = i - k * Rp;
-        v[u] = i < total && k < a.K && r < R ? __ldg(a.gsrc[o] + a.grow[o][r] + a.gk[o][k]) : 0.0f;
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (i0 + u * step < total) a.fb_pack[o][i0 + u * step] = v[u];
-    }
-  }
+  if constexpr (MODE == TC_F32X6)
+    for (int i = 0; i < g.n_items; ++i) f32_fallback_prepare<MODE, LOAD, BNV>(g.items[i].args);
 }
 
 // FP32 results (TC_F32X6): the hi | mid parts through tmA / tmB, the lo parts
@@ -1180,7 +1215,7 @@ __global__ void __launch_bounds__(TcCfgT<MODE, LOAD, BNV>::NUM_THREADS, 1)
   TcGroup g{nullptr, nullptr, 0, 0};
   gett_tc_body<MODE, LOAD, BNV, false>(&tmA, &tmB, &a, g, a.status, &tmAl, &tmBl);
   grid_dep_wait();  // the range words: not every warp has waited
-  if (!f32_split_exact(a.range, a.K)) f32_fallback_pack(a, TcCfgT<MODE, LOAD, BNV>::NUM_THREADS);
+  f32_fallback_prepare<MODE, LOAD, BNV>(a);
 }
 
 // Tail split: C = alpha * (slice 0 + slice 1 + ...) + beta * C over the tail

@@ -137,7 +137,10 @@ struct tccg_plan {
   int32_t* t_sk = nullptr;
   size_t sk_tab[6] = {};
   // workspace layout
-  size_t off_fb = 0;  // FP32 on the tensor cores: the fallback's B (its A at off_a)
+  // FP32 on the tensor cores, the fallback: its k slices (those of the FFMA
+  // plan), its packed B and partial sums (its packed A at off_a)
+  int32_t fb_ksplit = 1, fb_ktiles = 0;
+  size_t off_fb = 0, off_fb_part = 0;
   size_t off_a = 0, off_b = 0, off_part = 0, off_cprime = 0, off_tail = 0, ws_bytes = 0;
   char describe[512] = "";
 };
@@ -1225,9 +1228,20 @@ extern "C" int tccg_plan_create(const tccg_desc* desc, int32_t dtype, int32_t pr
   return TCCG_OK;
 }
 
-// Elements of one operand packed for the FP32 fallback (f32_fallback_pack).
-static int64_t f32_fallback_elems(int64_t rows, int64_t K) {
-  return round_up(rows, SimtCfg<float>::BM) * round_up(K, SimtCfg<float>::BK);
+// The FP32 fallback: its k slices -- those of the FFMA plan that would run without
+// the split; one where the tuning asks for the split -- and its part of the
+// workspace, over the split operands, which nobody reads then.
+static size_t f32_fallback_layout(tccg_plan* p) {
+  p->fb_ktiles = (int32_t)cdiv(p->K, SimtCfg<float>::BK);
+  p->fb_ksplit = 1;
+  if (p->tune.variant <= 0)
+    p->fb_ktiles = (int32_t)simt_ksplit(p, choose_simt_shape(p, nullptr), &p->fb_ksplit);
+  const int64_t Mp = round_up(p->M, SimtCfg<float>::BM), Np = round_up(p->N, SimtCfg<float>::BN);
+  const int64_t Kp = round_up(p->K, SimtCfg<float>::BK);
+  p->off_fb = align_up(p->off_a + (size_t)(Mp * Kp) * 4, 256);
+  p->off_fb_part = align_up(p->off_fb + (size_t)(Np * Kp) * 4, 256);
+  const size_t slices = p->fb_ksplit > 1 ? (size_t)p->fb_ksplit * Mp * Np * 4 : 0;
+  return align_up(p->off_fb_part + slices, 256);
 }
 
 static int plan_layout(tccg_plan* p) {
@@ -1399,17 +1413,15 @@ static int plan_layout(tccg_plan* p) {
       p->grid = 2 * (int32_t)std::min<int64_t>(tiles, clusters);
     } else
       p->grid = (int32_t)std::min<int64_t>(tiles, ctas);
-    p->off_a = 0;
-    if (!p->gather) {  // packed operands
-      ws = align_up((size_t)(p->M * p->Kc) * 2, 256);
-      p->off_b = ws;
-      ws = align_up(ws + (size_t)(p->N * p->Kc) * 2, 256);
-    }
-    if (x6) {  // the operands' range words, past the fallback's packed operands too
-      p->off_fb = align_up((size_t)f32_fallback_elems(p->M, p->K) * 4, 256);
-      ws = std::max(ws, align_up(p->off_fb + (size_t)f32_fallback_elems(p->N, p->K) * 4, 256));
+    if (x6) {  // the operands' range words; the fallback's part is laid over the rest
       p->off_range = ws;
       ws += 256;
+    }
+    p->off_a = ws;
+    if (!p->gather) {  // packed operands
+      ws = align_up(ws + (size_t)(p->M * p->Kc) * 2, 256);
+      p->off_b = ws;
+      ws = align_up(ws + (size_t)(p->N * p->Kc) * 2, 256);
     }
     if (p->ksplit > 1) {  // FP32 slices [split][N][M]
       p->off_part = ws;
@@ -1419,6 +1431,7 @@ static int plan_layout(tccg_plan* p) {
       p->off_tail = ws;
       ws = align_up(ws + (size_t)p->tail_split * (size_t)(mn - p->full_tiles) * p->bn * 128 * 4, 256);
     }
+    if (x6) ws = std::max(ws, f32_fallback_layout(p));
     static const char* gr[] = {"rows", "k", "kquad"};
     if (p->gather)
       snprintf(p->describe, sizeof(p->describe),
@@ -2016,7 +2029,7 @@ static int run_simt(const tccg_plan* p, const void* GA, const void* GB, T* Cout,
     dim3 g2((unsigned)cdiv(p->M, 256), (unsigned)std::min<int64_t>(p->N, 65535));
     mark(2, 0, s);
     launch_after(true, p, simt_reduce_kernel<T>, g2, dim3(256), 0, s, a.partial, (int)p->ksplit,
-                 p->Mp, p->Np, p->M, p->N, Cout, c_m, c_n, alpha, beta, (const uint32_t*)nullptr, 0);
+                 p->Mp, p->Np, p->M, p->N, Cout, c_m, c_n, alpha, beta, (const uint32_t*)nullptr, 0, false);
     mark(2, 1, s);
     rc = launch_check("simt_reduce");
   }
@@ -2080,29 +2093,45 @@ static int encode_f32x6(const tccg_plan* p, void* Ap, void* Bp, CUtensorMap* tmA
 }
 
 // The CUDA-core form of an FP32 plan on the tensor cores, for values its
-// operand splits do not represent.
-static F32FallbackItem f32_fallback_item(const tccg_plan* p, const void* GA, const void* GB,
-                                         float* C, const uint32_t* range, float alpha, float beta) {
+// operand splits do not represent, on the operands packed by f32_fallback_pack.
+static F32FallbackItem f32_fallback_item(const tccg_plan* p, char* ws, float* C,
+                                         const uint32_t* range, float alpha, float beta) {
   F32FallbackItem it{};
   SimtArgs<float>& a = it.args;
   a.M = p->M;
   a.N = p->N;
-  a.ktiles = a.ktiles_per_split = (int32_t)cdiv(p->K, SimtCfg<float>::BK);
+  a.K = p->K;
+  a.Mp = round_up(p->M, SimtCfg<float>::BM);
+  a.Np = round_up(p->N, SimtCfg<float>::BN);
+  a.Ap = reinterpret_cast<const float*>(ws + p->off_a);
+  a.Bp = reinterpret_cast<const float*>(ws + p->off_fb);
+  a.ktiles = (int32_t)cdiv(p->K, SimtCfg<float>::BK);
+  a.ktiles_per_split = p->fb_ktiles;
+  a.partial = p->fb_ksplit > 1 ? reinterpret_cast<float*>(ws + p->off_fb_part) : nullptr;
   a.C = C;
   a.c_m_off = p->t_c_m;
   a.c_n_off = p->t_c_n;
   a.alpha = alpha;
   a.beta = beta;
-  set_direct(a, p, GA, GB);
-  a.direct = 1;
   a.status = p->d_status;
   a.crun = p->crun;
   a.c_vec = c_vectors(p, C, false);
   it.range = range;
   it.K = (int32_t)p->K;
-  it.tiles_m = (int32_t)cdiv(p->M, SimtCfg<float>::BM);
-  it.tiles = (int64_t)it.tiles_m * cdiv(p->N, SimtCfg<float>::BN);
+  it.tiles_m = (int32_t)(a.Mp / SimtCfg<float>::BM);
+  it.tiles = (int64_t)it.tiles_m * (a.Np / SimtCfg<float>::BN);
+  it.jobs = it.tiles * p->fb_ksplit;
   return it;
+}
+
+// The source tensors and destinations of f32_fallback_pack.
+static void set_gather(TcArgs& a, const tccg_plan* p, const void* GA, const void* GB);
+static void set_fallback_pack(TcArgs& a, const tccg_plan* p, const void* GA, const void* GB, char* ws) {
+  set_gather(a, p, GA, GB);
+  a.fb_pack[0] = reinterpret_cast<float*>(ws + p->off_a);
+  a.fb_pack[1] = reinterpret_cast<float*>(ws + p->off_fb);
+  a.fb_kfast[0] = p->read_k_fast_a;
+  a.fb_kfast[1] = p->read_k_fast_b;
 }
 
 // Gather loader: the kernel reads GA and GB through the plan's offset tables.
@@ -2139,7 +2168,7 @@ static int tc_reduce(const tccg_plan* p, const TcArgs& a, float* Cout, const int
   mark(2, 0, s);
   launch_after(true, p, simt_reduce_kernel<float>, g2, dim3(256), 0, s, (const float*)a.partial,
                (int)p->ksplit, (int64_t)p->M, (int64_t)p->N, (int64_t)p->M, (int64_t)p->N, Cout, c_m,
-               c_n, alpha, beta, a.range, (int)p->K);
+               c_n, alpha, beta, a.range, (int)p->K, false);
   mark(2, 1, s);
   return launch_check("tc_reduce");
 }
@@ -2184,9 +2213,7 @@ static int run_tc(const tccg_plan* p, const void* GA, const void* GB, float* Cou
       rc = launch_pack<float, __nv_bfloat16, PACK_K_BF16>(pa, s, &packed);
     if (rc) return rc;
     if (x6) {
-      set_gather(a, p, GA, GB);
-      a.fb_pack[0] = static_cast<float*>(Ap);
-      a.fb_pack[1] = reinterpret_cast<float*>(ws + p->off_fb);
+      set_fallback_pack(a, p, GA, GB, ws);
       rc = encode_f32x6(p, Ap, Bp, &tmA, &tmB, &tmAl, &tmBl);
     } else {
       rc = encode_kmajor(&tmA, Ap, p->M, p->Kc, 128);
@@ -2218,14 +2245,14 @@ static int run_tc(const tccg_plan* p, const void* GA, const void* GB, float* Cou
   if (rc) return rc;
   rc = tc_reduce(p, a, Cout, c_m, c_n, alpha, beta, s);
   if (rc || !x6) return rc;
-  F32FallbackItem it = f32_fallback_item(p, GA, GB, Cout, a.range, alpha, beta);
-  it.args.direct = 0;
-  it.args.Ap = a.fb_pack[0];
-  it.args.Bp = a.fb_pack[1];
-  it.args.Mp = round_up(p->M, SimtCfg<float>::BM);
-  it.args.Np = round_up(p->N, SimtCfg<float>::BN);
-  launch_after(true, p, f32_fallback_kernel, dim3((unsigned)std::min<int64_t>(it.tiles, 2 * p->num_sms)),
+  const F32FallbackItem it = f32_fallback_item(p, ws, Cout, a.range, alpha, beta);
+  launch_after(true, p, f32_fallback_kernel, dim3((unsigned)it.jobs),
                dim3(256), simt_smem_bytes<float>(), s, it);
+  if (it.args.partial)
+    launch_after(true, p, simt_reduce_kernel<float>,
+                 dim3((unsigned)cdiv(p->M, 256), (unsigned)std::min<int64_t>(p->N, 65535)), dim3(256), 0, s,
+                 (const float*)it.args.partial, (int)p->fb_ksplit, it.args.Mp, it.args.Np, (int64_t)p->M,
+                 (int64_t)p->N, Cout, c_m, c_n, alpha, beta, a.range, (int)p->K, true);
   return launch_check("f32_fallback");
 }
 
@@ -2794,8 +2821,9 @@ extern "C" int tccg_group_create(const tccg_plan* const* plans, int32_t count, t
     e = cudaMalloc((void**)&g->d_sktc, sizeof(SkinnyTcItem) * g->n_sktc);
   if (e == cudaSuccess && g->n_sk + g->n_sktc)
     e = cudaMalloc((void**)&g->d_skr, sizeof(SkinnyItem) * (g->n_sk + g->n_sktc));
-  if (e == cudaSuccess) e = cudaMalloc(&g->d_reduce, sizeof(ReduceJob<double>) * count);
-  const size_t nbegin = 2 * (size_t)g->n_simt + n_tcj + g->n_simt + g->n_tc + count + g->n_sk +
+  const int32_t n_red = count + g->n_x6;  // FP32 items on the tensor cores: the fallback's too
+  if (e == cudaSuccess) e = cudaMalloc(&g->d_reduce, sizeof(ReduceJob<double>) * n_red);
+  const size_t nbegin = 2 * (size_t)g->n_simt + n_tcj + g->n_simt + g->n_tc + n_red + g->n_sk +
                         (g->n_sk + g->n_sktc) + g->n_sktc;
   if (e == cudaSuccess) e = cudaMalloc((void**)&g->d_begin, sizeof(int64_t) * nbegin);
   if (e == cudaSuccess) {
@@ -2804,7 +2832,7 @@ extern "C" int tccg_group_create(const tccg_plan* const* plans, int32_t count, t
     g->b_simt_items = g->b_tc_jobs + n_tcj;
     g->b_tc_items = g->b_simt_items + g->n_simt;
     g->b_reduce = g->b_tc_items + g->n_tc;
-    g->b_sk = g->b_reduce + count;
+    g->b_sk = g->b_reduce + n_red;
     g->b_skr = g->b_sk + g->n_sk;
     g->b_sktc = g->b_skr + g->n_sk + g->n_sktc;
   }
@@ -2869,6 +2897,7 @@ static ReduceJob<T> reduce_job_for(const T* partial, int32_t splits, int64_t Mp,
   j.begin = begin;
   j.splits = splits;
   j.range = nullptr;
+  j.fallback = 0;
   j.K = (int32_t)std::min<int64_t>(p->K, INT32_MAX);
   j.mblocks = (int32_t)cdiv(p->M, 256);
   // about 256 loads per thread: many slices -> few columns per CTA
@@ -3010,8 +3039,17 @@ static int bind_tc(tccg_group* g, tccg_group::Wave& wv, const void* const* A, co
           it.args.range = range;
           jobs[jobs.size() - 2].op.range = range;
           jobs[jobs.size() - 1].op.range = range + 2;
-          fallback.push_back(f32_fallback_item(p, GA, GB, static_cast<float*>(C[i]), range,
-                                               (float)alpha[i], (float)beta[i]));
+          set_fallback_pack(it.args, p, GA, GB, w);
+          fallback.push_back(f32_fallback_item(p, w, static_cast<float*>(C[i]), range, (float)alpha[i],
+                                               (float)beta[i]));
+          if (p->fb_ksplit > 1) {
+            const SimtArgs<float>& fa = fallback.back().args;
+            red.push_back(reduce_job_for<float>(fa.partial, p->fb_ksplit, fa.Mp, fa.Np, p, C[i], alpha[i],
+                                                beta[i], rctas));
+            red.back().range = range;
+            red.back().fallback = 1;
+            rctas += reduce_ctas(red.back());
+          }
           rc = encode_f32x6(p, w + p->off_a, w + p->off_b, &it.tmA, &it.tmB, &it.tmAl, &it.tmBl);
         } else {
           rc = encode_kmajor(&it.tmA, w + p->off_a, p->M, p->Kc, 128);
