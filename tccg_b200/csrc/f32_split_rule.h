@@ -29,6 +29,7 @@ inline bool f32_split_fits(int64_t M, int64_t N, int64_t K) {
 //   lognormal(1)  17 | 16 8.2 5.7   24 | 16 8.3 6.3    28 | 16 8.4 6.7   39 | 16 8.1 5.7   54 | 16 8.2 5.7
 //   lognormal(2)  18 | 44 21  12    24 | 45 22  13     30 | 46 23  13    42 | 47 23  13    60 | 48 24  14
 //   e^-20u        16 | 46 25  14    26 | 44 24  14     34 | 44 24  15    60 | 43 23  14    107| 42 23  14
+//   e^-58u                         8.3| 17 11  8.1    9.9| 17 11  8.7    14 | 16 10 7.8     21 | 15 9.9 7.7
 //   normal        2.8| 1.7 1.0 .85  2.7| .9 .6 .6      2.6| .7 .5 .5     2.6| .5 .4 .3     2.6| .3 .3 .2
 // Below 256 FFMA stays: 14 against 16 is no distance. 4096 x 4096 x 1024 takes
 // 210 us by chunks of 4, 231 of 2, 263 of 1 (FFMA 658).
@@ -40,7 +41,7 @@ inline bool f32_split_fits(int64_t M, int64_t N, int64_t K) {
 // e^-20u 13 | 23 14.
 inline int f32_split_chunk(int64_t chain, int64_t splits) {
   const int64_t c = chain / splits;
-  return c >= 1536 ? 4 : c >= 768 ? 3 : c >= 384 ? 2 : c >= 256 || splits > 1 ? 1 : 0;
+  return c >= 1536 ? 4 : c >= 768 ? 3 : c >= 512 ? 2 : c >= 256 || splits > 1 ? 1 : 0;
 }
 
 }  // namespace tccg

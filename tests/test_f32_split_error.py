@@ -17,6 +17,7 @@ DRAW = {
     "lognormal1": lambda n, u: n.exp(),
     "lognormal2": lambda n, u: (2 * n).exp(),
     "log_uniform": lambda n, u: (-20 * u).exp(),
+    "many_magnitudes": lambda n, u: (-55 * u).exp(),
 }
 
 
@@ -42,7 +43,7 @@ def _errors(m, n, k, draw, **tuned):
 
 
 # K at the edges of the chunk rule; few tiles (k slices on both sides)
-@pytest.mark.parametrize("m,n,k,chunk", [(2048, 2080, 256, 1), (2048, 2080, 383, 1), (2048, 2080, 384, 2),
+@pytest.mark.parametrize("m,n,k,chunk", [(2048, 2080, 256, 1), (2048, 2080, 511, 1), (2048, 2080, 512, 2),
                                          (2048, 2080, 767, 2), (2048, 2080, 768, 3), (2048, 2080, 1535, 3),
                                          (2048, 2080, 1536, 4), (12648, 85, 4418, 3)])
 @pytest.mark.parametrize("draw", sorted(DRAW))
