@@ -319,8 +319,8 @@ __device__ __forceinline__ void split_bf16x2(float x0, float x1, uint32_t& hi, u
 // ---- three-way split of FP32 ---------------------------------------------------
 // x = hi + mid + lo exactly: hi = bf16_rn(x), mid = bf16_rn(x - hi), lo =
 // x - hi - mid (|x - hi| <= 2^-8 |x| and |x - hi - mid| <= 2^-17 |x|, so at
-// most 7 of x's 24 significant bits are left for lo). Exact for every x that
-// f32_split_exact() accepts.
+// most 7 of x's 24 significant bits are left for lo). Exact for every (scaled)
+// x that f32_split_exact() accepts.
 __device__ __forceinline__ void split3_bf16x2(float x0, float x1, uint32_t& hi, uint32_t& mid,
                                               uint32_t& lo) {
   const __nv_bfloat162 h = __floats2bfloat162_rn(x0, x1);
@@ -354,19 +354,34 @@ struct AbsRange {
   }
 };
 
-// Whether FP32 products of two operands with ranges w[0..1] and w[2..3] over
-// K terms may run as products of their three-way splits: every value finite
-// and below 2^127 (the split's rounding cannot overflow), no sum of products
-// near overflow, nonzero values at least 2^-100 (every part of the split is a
-// normal bf16 or exact) and nonzero products at least 2^-100 (the dropped and
-// the smallest kept terms stay clear of FP32's subnormals).
-__device__ __forceinline__ bool f32_split_exact(const uint32_t* w, int K) {
-  const uint4 r = *reinterpret_cast<const uint4*>(w);
+// A contraction over K terms of operands with the range words w[0..1] and
+// w[2..3] (null: not such a contraction), each multiplied by 2^shift before its
+// split. With F32_SPLIT_SHIFT (2^-149, FP32's smallest step, becomes 2^-126) the
+// parts of every value, subnormals too, are normal bf16 numbers or zero, so the
+// split of any finite value is exact; products, scaled by 2^46, leave FP32's
+// range only below 2^-172, where FP32 multiply-adds round them off as well.
+// Only large values are left outside.
+constexpr int F32_SPLIT_SHIFT = 23;
+struct SplitRange {
+  const uint32_t* w;
+  int32_t K, shift;
+};
+
+// Whether its FP32 products may run as products of three-way splits: every
+// value finite and, scaled, below 2^127 (the split's rounding cannot overflow),
+// and no sum of scaled products near overflow: |a| |b| K below 2^78 at
+// F32_SPLIT_SHIFT. With a smaller shift also: nonzero values at least 2^-100 (every
+// part of the split is a normal bf16 or exact) and nonzero products at least
+// 2^-100 (the dropped and the smallest kept terms stay clear of FP32's
+// subnormals).
+__device__ __forceinline__ bool f32_split_exact(const SplitRange& s) {
+  const uint4 r = *reinterpret_cast<const uint4*>(s.w);
   const int ea = (int)(~r.x >> 23), eb = (int)(~r.z >> 23);  // biased exponents
-  if (ea >= 254 || eb >= 254) return false;
+  if (ea + s.shift >= 254 || eb + s.shift >= 254) return false;
   if (r.y == 0xffffffffu || r.w == 0xffffffffu) return true;  // an operand of zeros
-  const int logk = 32 - __clz(K);
-  if (ea - 127 + eb - 127 + 2 + logk >= 126) return false;
+  const int logk = 32 - __clz(s.K);
+  if (ea - 127 + eb - 127 + 2 * s.shift + 2 + logk >= 126) return false;
+  if (s.shift >= F32_SPLIT_SHIFT) return true;
   const int ma = (int)((r.y + 1u) >> 23) - 127, mb = (int)((r.w + 1u) >> 23) - 127;
   return ma >= -100 && mb >= -100 && ma + mb >= -100;
 }

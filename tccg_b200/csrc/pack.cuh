@@ -20,7 +20,8 @@ enum PackLayout : int {
   PACK_K_BF16X3 = 2,  // dst[r * ld + (k/32)*64 + k%32] = hi, +32 = lo (bf16)
   PACK_MN_BF16 = 3,   // as PACK_MN, each value rounded to bf16 (BF16 semantics on CUDA cores)
   PACK_K_F32X6 = 4,   // dst[r * ld + (k/32)*96 + k%32] = hi, +32 = mid, +64 = lo (bf16): the
-                      // exact three-way split of FP32, with the operand's magnitude range
+                      // exact three-way split of FP32 times a power of two, with the
+                      // operand's magnitude range
 };
 __host__ __device__ constexpr bool pack_k_major(int layout) {
   return layout == PACK_K_BF16 || layout == PACK_K_BF16X3 || layout == PACK_K_F32X6;
@@ -62,8 +63,9 @@ struct PackOperand {
   // tile grid of this operand: tiles along k and in total (set by the host)
   int64_t ktiles, tiles;
   // PACK_K_F32X6: the operand's two range words (AbsRange), 0xffffffff before
-  // the pass
+  // the pass, and the power of two that its values are split times
   uint32_t* range;
+  float scale;
 };
 
 // The values a thread packs, for PACK_K_F32X6's range words (else nothing).
@@ -75,6 +77,7 @@ struct PackRange {
 template <>
 struct PackRange<PACK_K_F32X6> {
   AbsRange r;
+  float scale;
   __device__ __forceinline__ void add(const float (&x)[4]) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) r.add(x[j]);
@@ -114,8 +117,9 @@ __device__ __forceinline__ void store_k4(__nv_bfloat16* base, int64_t k, int64_t
   if constexpr (LAYOUT == PACK_K_F32X6) {  // kcover is a multiple of 32
     __nv_bfloat16* row = base + (k / 32) * 96;  // 64-byte aligned: ld % 96 == 0
     uint2 uh, um, ul;
-    split3_bf16x2(x[0], x[1], uh.x, um.x, ul.x);
-    split3_bf16x2(x[2], x[3], uh.y, um.y, ul.y);
+    const float c = rng.scale;
+    split3_bf16x2(c * x[0], c * x[1], uh.x, um.x, ul.x);
+    split3_bf16x2(c * x[2], c * x[3], uh.y, um.y, ul.y);
     *reinterpret_cast<uint2*>(row + k % 32) = uh;
     *reinterpret_cast<uint2*>(row + 32 + k % 32) = um;
     *reinterpret_cast<uint2*>(row + 64 + k % 32) = ul;
@@ -559,6 +563,7 @@ __device__ __forceinline__ void pack_tiles(const PackOperand& o, int64_t kt, int
 template <typename Tin, typename Tout, int LAYOUT, int READ>
 __device__ __forceinline__ void pack_any(const PackOperand& o, int64_t kt, int64_t rt) {
   PackRange<LAYOUT> rng;
+  if constexpr (LAYOUT == PACK_K_F32X6) rng.scale = o.scale;
   pack_tiles<Tin, Tout, LAYOUT, READ>(o, kt, rt, rng);
   if constexpr (LAYOUT == PACK_K_F32X6) __syncwarp();
   rng.flush(o.range);

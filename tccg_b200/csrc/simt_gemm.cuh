@@ -716,8 +716,8 @@ __global__ void __launch_bounds__(256, SimtCfg<T, S>::MIN_BLOCKS) simt_gett_kern
 // in the ordinary case the CTAs read the range words and leave at once.
 struct F32FallbackItem {
   SimtArgs<float> args;
-  const uint32_t* range;
-  int32_t K, tiles_m;
+  SplitRange split;
+  int32_t tiles_m;
   int64_t tiles, jobs;  // tiles x k slices
 };
 
@@ -735,7 +735,7 @@ __device__ __forceinline__ void f32_fallback_job(const F32FallbackItem& it, int6
 __global__ void __launch_bounds__(256, 2)
     f32_fallback_kernel(const __grid_constant__ F32FallbackItem it) {
   grid_dep_wait();  // range words of the packing pass; C written by nobody before this
-  if (!f32_split_exact(it.range, it.K)) f32_fallback_job(it, blockIdx.x);
+  if (!f32_split_exact(it.split)) f32_fallback_job(it, blockIdx.x);
 }
 
 // Grouped: a persistent wave; the jobs of the items that need it, one item's
@@ -746,7 +746,7 @@ __global__ void __launch_bounds__(256, 2)
   int64_t first = 0;  // the CTA that takes the item's first job
   for (int i = 0; i < n_items; ++i) {
     const F32FallbackItem& it = items[i];
-    if (f32_split_exact(it.range, it.K)) continue;
+    if (f32_split_exact(it.split)) continue;
     for (int64_t j = (blockIdx.x + g - first) % g; j < it.jobs; j += g) f32_fallback_job(it, j);
     first = (first + it.jobs) % g;
   }
@@ -1097,11 +1097,11 @@ __global__ void __launch_bounds__(256) simt_reduce_kernel(const T* __restrict__ 
                                                           int64_t M, int64_t N, T* C,
                                                           const int64_t* c_m_off,
                                                           const int64_t* c_n_off, T alpha,
-                                                          T beta, const uint32_t* range, int K,
+                                                          T beta, SplitRange split,
                                                           bool fallback) {
   grid_dep_wait();  // partial sums written by the GETT kernel before
   // an FP32 plan on the tensor cores: its slices, or the fallback's
-  if (range && f32_split_exact(range, K) == fallback) return;
+  if (split.w && f32_split_exact(split) == fallback) return;
   const int64_t m = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (m >= M) return;
   const int64_t cmo = c_m_off[m];
@@ -1130,9 +1130,8 @@ struct ReduceJob {
   int64_t begin;
   int32_t splits, mblocks;
   int32_t ncols;  // columns per CTA: fewer when there are many slices
-  int32_t K;
-  const uint32_t* range;  // FP32 on the tensor cores: the item's range words, or null
-  int32_t fallback;       // its fallback's slices, not the split products'
+  int32_t fallback;  // FP32 on the tensor cores: the fallback's slices, not the split products'
+  SplitRange split;  // FP32 on the tensor cores: the item's ranges
 };
 
 template <typename T>
@@ -1140,7 +1139,7 @@ __global__ void __launch_bounds__(256) reduce_group_kernel(const ReduceJob<T>* j
                                                            const int64_t* begin, int n_jobs) {
   const int64_t t = blockIdx.x;
   const ReduceJob<T> j = jobs[find_segment(begin, n_jobs, t)];  // fields loaded up front
-  if (j.range && f32_split_exact(j.range, j.K) == (j.fallback != 0)) return;
+  if (j.split.w && f32_split_exact(j.split) == (j.fallback != 0)) return;
   const int64_t local = t - j.begin;
   const int64_t m = (local % j.mblocks) * 256 + threadIdx.x;
   if (m >= j.M) return;

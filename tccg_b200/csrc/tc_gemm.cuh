@@ -55,7 +55,7 @@ namespace tccg {
 //   Tile: 128 x 160 -- three accumulators of 160 columns in 480 of the 512
 //   TMEM columns, and four 54 KB stages beside the epilogue staging.
 //   Values that the split does not represent (infinity, NaN, magnitudes near
-//   either end of the range): the packing pass keeps the operands' ranges,
+//   the largest; SplitRange): the packing pass keeps the operands' ranges,
 //   every role skips the tiles of such a contraction (f32_split_exact), and a
 //   CUDA-core launch behind computes it from the caller's tensors.
 enum TcMode : int { TC_BF16 = 0, TC_BF16X3 = 1, TC_F32X6 = 2 };
@@ -188,9 +188,11 @@ struct TcArgs {
   // C by the first N mode: stores go through shared memory in runs of e0 m
   // by 32 / e0 columns, which are consecutive addresses of C
   int32_t crun;
-  // TC_F32X6: the operands' range words (AbsRange, GA's two then GB's); the
-  // place of the fallback's packed operands and whether they are read along k
-  const uint32_t* range;
+  // TC_F32X6: the operands' ranges and scale, and 2^(-2 shift), which the sums
+  // are multiplied by; the place of the fallback's packed operands and whether
+  // they are read along k
+  SplitRange split;
+  float descale;
   float* fb_pack[2];
   int32_t fb_kfast[2];
   // C's element offsets all fit 31 bits: the epilogue passes column offsets
@@ -739,7 +741,7 @@ __device__ __forceinline__ void gett_tc_body(const CUtensorMap* tmA, const CUten
     bool ok = true;
     for (int tile = cta; tile < num_tiles && ok; tile += gridDim.x) {
       const TileRef t = resolve_tile<GROUPED>(tile, tmA, tmB, a1, g, tmAl, tmBl);
-      if (X6 && !f32_split_exact(t.a->range, t.a->K)) continue;
+      if (X6 && !f32_split_exact(t.a->split)) continue;
       for (int kb = t.kb_begin; kb < t.kb_end; ++kb) {
         if (!mbar_wait(&empty[stage], phase ^ 1, wait_ns)) {
           record_error(status, 1);
@@ -779,7 +781,7 @@ __device__ __forceinline__ void gett_tc_body(const CUtensorMap* tmA, const CUten
     uint32_t sm_phase = 0;  // X6: fills of the small products' accumulator
     for (int tile = cta; tile < num_tiles && ok; tile += gridDim.x) {
       const TileRef t = resolve_tile<GROUPED>(tile, tmA, tmB, a1, g);
-      if (X6 && !f32_split_exact(t.a->range, t.a->K)) continue;
+      if (X6 && !f32_split_exact(t.a->split)) continue;
       const int nkb = t.kb_end, K = t.a->K, ckb = t.a->chunk_kb;
       const int seg = small_chunks<Cfg::SMALL_KB>(ckb);  // X6: chunks per fill
       int seg_ch = 0;
@@ -897,7 +899,7 @@ __device__ __forceinline__ void gett_tc_body(const CUtensorMap* tmA, const CUten
     for (int tile = cta; tile < num_tiles && ok; tile += gridDim.x) {
       const TileRef t = resolve_tile<GROUPED>(tile, tmA, tmB, a1, g);
       const TcArgs& a = *t.a;
-      if (X6 && !f32_split_exact(a.range, a.K)) continue;
+      if (X6 && !f32_split_exact(a.split)) continue;
       const int64_t m = (int64_t)t.tm * Cfg::BM + q * 32 + lane;
       const bool m_ok = m < a.M;
       const int64_t cmo = m_ok ? a.c_m_off[m] : 0;
@@ -1077,6 +1079,10 @@ __device__ __forceinline__ void gett_tc_body(const CUtensorMap* tmA, const CUten
           }
         }
         if (!ok) break;
+        if constexpr (X6) {
+#pragma unroll
+          for (int j = 0; j < HC; ++j) sum[j] *= a.descale;
+        }
         if (part) {  // warp-uniform, like the branches below
           if (m_ok) {
             float* d = part + (size_t)pc0 * pld;
@@ -1191,7 +1197,7 @@ __device__ __forceinline__ void f32_fallback_prepare(const TcArgs& a) {
   using Cfg = TcCfgT<MODE, LOAD, BNV>;
   static_assert(Cfg::NUM_THREADS / 32 * 32 * 33 * 4 <= Cfg::SMEM_BYTES, "transposition tiles fit");
   extern __shared__ uint8_t smem_raw[];
-  if (!f32_split_exact(a.range, a.K))
+  if (!f32_split_exact(a.split))
     f32_fallback_pack(a, Cfg::NUM_THREADS, reinterpret_cast<float*>(smem_raw));
 }
 
@@ -1225,7 +1231,7 @@ template <int MODE, int LOAD = TC_LOAD_TMA, int BNV = 0>
 __global__ void __launch_bounds__(256) tc_tail_reduce_kernel(const TcArgs a) {
   using Cfg = TcCfgT<MODE, LOAD, BNV>;
   grid_dep_wait();  // partial sums written by the GETT kernel before
-  if (MODE == TC_F32X6 && !f32_split_exact(a.range, a.K)) return;
+  if (MODE == TC_F32X6 && !f32_split_exact(a.split)) return;
   const int tail = a.tiles_m * a.tiles_n - a.full_tiles;
   const int tl = blockIdx.x;
   const int e = blockIdx.y * 256 + threadIdx.x;

@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <cmath>
 #include <cstdarg>
 #include <cstdlib>
 #include <cstdio>
@@ -1798,6 +1799,7 @@ static PackOperand pack_op(const void* src, const int64_t* roff, const int64_t* 
   o.kstream = o.rquad = 0;
   o.ktiles = o.tiles = 0;
   o.range = nullptr;
+  o.scale = 1.0f;
   return o;
 }
 
@@ -2029,7 +2031,7 @@ static int run_simt(const tccg_plan* p, const void* GA, const void* GB, T* Cout,
     dim3 g2((unsigned)cdiv(p->M, 256), (unsigned)std::min<int64_t>(p->N, 65535));
     mark(2, 0, s);
     launch_after(true, p, simt_reduce_kernel<T>, g2, dim3(256), 0, s, a.partial, (int)p->ksplit,
-                 p->Mp, p->Np, p->M, p->N, Cout, c_m, c_n, alpha, beta, (const uint32_t*)nullptr, 0, false);
+                 p->Mp, p->Np, p->M, p->N, Cout, c_m, c_n, alpha, beta, SplitRange{}, false);
     mark(2, 1, s);
     rc = launch_check("simt_reduce");
   }
@@ -2049,6 +2051,19 @@ static bool sm_order_enabled() {
 
 // Arguments of the tcgen05 kernels common to both loaders (k-split partial
 // sums and tail slices in the workspace `ws`).
+// The range words and scale of an FP32 plan on the tensor cores (else none). A
+// tuning that asks for the split runs it on the values as they are: its narrower
+// window, with the CUDA cores outside it, is what it asks for.
+static SplitRange split_range(const tccg_plan* p, uint32_t* words) {
+  if (!p->f32x6) return SplitRange{};
+  return SplitRange{words, (int32_t)p->K, p->tune.variant > 0 ? 0 : F32_SPLIT_SHIFT};
+}
+
+static void set_split(PackOperand& o, const SplitRange& s, int operand) {
+  o.range = const_cast<uint32_t*>(s.w) + 2 * operand;
+  o.scale = std::ldexp(1.0f, s.shift);
+}
+
 static TcArgs tc_args(const tccg_plan* p, float* Cout, const int64_t* c_m, const int64_t* c_n,
                       float alpha, float beta, char* ws) {
   TcArgs a{};
@@ -2076,7 +2091,8 @@ static TcArgs tc_args(const tccg_plan* p, float* Cout, const int64_t* c_m, const
   a.crun = c_m == p->t_c_m ? p->crun : 0;  // not for TTGT's contiguous C'
   a.sm_order = sm_order_enabled() ? 1 : 0;
   a.c32 = c_m == p->t_c_m ? p->c32 : p->M * p->N <= INT32_MAX;
-  a.range = p->f32x6 ? reinterpret_cast<uint32_t*>(ws + p->off_range) : nullptr;
+  a.split = split_range(p, reinterpret_cast<uint32_t*>(ws + p->off_range));
+  a.descale = std::ldexp(1.0f, -2 * a.split.shift);
   return a;
 }
 
@@ -2095,7 +2111,7 @@ static int encode_f32x6(const tccg_plan* p, void* Ap, void* Bp, CUtensorMap* tmA
 // The CUDA-core form of an FP32 plan on the tensor cores, for values its
 // operand splits do not represent, on the operands packed by f32_fallback_pack.
 static F32FallbackItem f32_fallback_item(const tccg_plan* p, char* ws, float* C,
-                                         const uint32_t* range, float alpha, float beta) {
+                                         const SplitRange& split, float alpha, float beta) {
   F32FallbackItem it{};
   SimtArgs<float>& a = it.args;
   a.M = p->M;
@@ -2116,8 +2132,7 @@ static F32FallbackItem f32_fallback_item(const tccg_plan* p, char* ws, float* C,
   a.status = p->d_status;
   a.crun = p->crun;
   a.c_vec = c_vectors(p, C, false);
-  it.range = range;
-  it.K = (int32_t)p->K;
+  it.split = split;
   it.tiles_m = (int32_t)(a.Mp / SimtCfg<float>::BM);
   it.tiles = (int64_t)it.tiles_m * (a.Np / SimtCfg<float>::BN);
   it.jobs = it.tiles * p->fb_ksplit;
@@ -2168,7 +2183,7 @@ static int tc_reduce(const tccg_plan* p, const TcArgs& a, float* Cout, const int
   mark(2, 0, s);
   launch_after(true, p, simt_reduce_kernel<float>, g2, dim3(256), 0, s, (const float*)a.partial,
                (int)p->ksplit, (int64_t)p->M, (int64_t)p->N, (int64_t)p->M, (int64_t)p->N, Cout, c_m,
-               c_n, alpha, beta, a.range, (int)p->K, false);
+               c_n, alpha, beta, a.split, false);
   mark(2, 1, s);
   return launch_check("tc_reduce");
 }
@@ -2202,8 +2217,8 @@ static int run_tc(const tccg_plan* p, const void* GA, const void* GB, float* Cou
     if (x6) {
       uint32_t* range = reinterpret_cast<uint32_t*>(ws + p->off_range);
       CUDA_TRY(cudaMemsetAsync(range, 0xff, 4 * sizeof(uint32_t), s));
-      pa.op[0].range = range;
-      pa.op[1].range = range + 2;
+      set_split(pa.op[0], a.split, 0);
+      set_split(pa.op[1], a.split, 1);
       rc = launch_pack<float, __nv_bfloat16, PACK_K_F32X6>(pa, s, &packed);
     } else if (x3)
       rc = launch_pack<float, __nv_bfloat16, PACK_K_BF16X3>(pa, s, &packed);
@@ -2245,14 +2260,14 @@ static int run_tc(const tccg_plan* p, const void* GA, const void* GB, float* Cou
   if (rc) return rc;
   rc = tc_reduce(p, a, Cout, c_m, c_n, alpha, beta, s);
   if (rc || !x6) return rc;
-  const F32FallbackItem it = f32_fallback_item(p, ws, Cout, a.range, alpha, beta);
+  const F32FallbackItem it = f32_fallback_item(p, ws, Cout, a.split, alpha, beta);
   launch_after(true, p, f32_fallback_kernel, dim3((unsigned)it.jobs),
                dim3(256), simt_smem_bytes<float>(), s, it);
   if (it.args.partial)
     launch_after(true, p, simt_reduce_kernel<float>,
                  dim3((unsigned)cdiv(p->M, 256), (unsigned)std::min<int64_t>(p->N, 65535)), dim3(256), 0, s,
                  (const float*)it.args.partial, (int)p->fb_ksplit, it.args.Mp, it.args.Np, (int64_t)p->M,
-                 (int64_t)p->N, Cout, c_m, c_n, alpha, beta, a.range, (int)p->K, true);
+                 (int64_t)p->N, Cout, c_m, c_n, alpha, beta, a.split, true);
   return launch_check("f32_fallback");
 }
 
@@ -2896,9 +2911,8 @@ static ReduceJob<T> reduce_job_for(const T* partial, int32_t splits, int64_t Mp,
   j.beta = (T)beta;
   j.begin = begin;
   j.splits = splits;
-  j.range = nullptr;
+  j.split = SplitRange{};
   j.fallback = 0;
-  j.K = (int32_t)std::min<int64_t>(p->K, INT32_MAX);
   j.mblocks = (int32_t)cdiv(p->M, 256);
   // about 256 loads per thread: many slices -> few columns per CTA
   j.ncols = (int32_t)std::max<int64_t>(1, std::min<int64_t>(64, 256 / splits));
@@ -3035,18 +3049,18 @@ static int bind_tc(tccg_group* g, tccg_group::Wave& wv, const void* const* A, co
                       pack_k_tile<PACK_K_BF16>(), true);
         int rc;
         if (p->f32x6) {
-          uint32_t* range = g->d_range + 4 * fallback.size();
-          it.args.range = range;
-          jobs[jobs.size() - 2].op.range = range;
-          jobs[jobs.size() - 1].op.range = range + 2;
+          const SplitRange split = split_range(p, g->d_range + 4 * fallback.size());
+          it.args.split = split;
+          set_split(jobs[jobs.size() - 2].op, split, 0);
+          set_split(jobs[jobs.size() - 1].op, split, 1);
           set_fallback_pack(it.args, p, GA, GB, w);
-          fallback.push_back(f32_fallback_item(p, w, static_cast<float*>(C[i]), range, (float)alpha[i],
+          fallback.push_back(f32_fallback_item(p, w, static_cast<float*>(C[i]), split, (float)alpha[i],
                                                (float)beta[i]));
           if (p->fb_ksplit > 1) {
             const SimtArgs<float>& fa = fallback.back().args;
             red.push_back(reduce_job_for<float>(fa.partial, p->fb_ksplit, fa.Mp, fa.Np, p, C[i], alpha[i],
                                                 beta[i], rctas));
-            red.back().range = range;
+            red.back().split = split;
             red.back().fallback = 1;
             rctas += reduce_ctas(red.back());
           }
@@ -3063,7 +3077,7 @@ static int bind_tc(tccg_group* g, tccg_group::Wave& wv, const void* const* A, co
       if (p->ksplit > 1) {
         red.push_back(reduce_job_for<float>(it.args.partial, p->ksplit, p->M, p->N, p, C[i],
                                             alpha[i], beta[i], rctas));
-        red.back().range = it.args.range;
+        red.back().split = it.args.split;
         rctas += reduce_ctas(red.back());
       }
     }
