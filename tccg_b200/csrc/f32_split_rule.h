@@ -17,6 +17,15 @@ inline bool f32_split_fits(int64_t M, int64_t N, int64_t K) {
   return M < lim && N < lim && K < lim && 3 * f32_split_k(K) <= INT32_MAX;
 }
 
+// Whether an automatic plan may take the split's workspace: 6 bytes per operand
+// element, where the FFMA forms need 4 or none, so a call that fills the GPU could
+// fit with those only. Operands, C and workspace together stay within half of
+// the 180 GB.
+inline bool f32_split_memory(int64_t M, int64_t N, int64_t K) {
+  const double k = (double)f32_split_k(K);
+  return 10.0 * ((double)M + (double)N) * k + 4.0 * (double)M * (double)N <= 90e9;
+}
+
 // k-blocks of 32 per accumulation chunk of an automatic plan, 0 = FFMA, by the
 // chains of FP32 adds of the FFMA form: `splits` k slices of `chain` each. Tensor
 // memory truncates each of a chunk's 2 sums per k-block, so the split's error

@@ -360,6 +360,7 @@ static bool choose_f32x6(const tccg_plan* p) {
   if (!f32_split_fits(p->M, p->N, p->K)) return false;
   const int chunk = f32x6_chunk(p);
   if (t.variant > 0 || chunk == 0) return chunk > 0;
+  if (!f32_split_memory(p->M, p->N, p->K)) return false;
   const int64_t tiles = cdiv(p->M, F32X6_BM) * cdiv(p->N, F32X6_BN), kb = cdiv(p->K, 32);
   int32_t split = 1;
   const int64_t per =

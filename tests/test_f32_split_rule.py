@@ -12,6 +12,7 @@ from tccg_b200 import build
 WRAP = """
 #include "f32_split_rule.h"
 extern "C" int fits(long long m, long long n, long long k) { return tccg::f32_split_fits(m, n, k); }
+extern "C" int memory(long long m, long long n, long long k) { return tccg::f32_split_memory(m, n, k); }
 extern "C" int chunk(long long chain, long long splits) { return tccg::f32_split_chunk(chain, splits); }
 """
 
@@ -28,6 +29,7 @@ def rule(tmp_path_factory):
     subprocess.run([gxx, "-std=c++17", "-shared", "-fPIC", "-I" + build.CSRC, src, "-o", out], check=True)
     lib = ctypes.CDLL(out)
     lib.fits.argtypes = [ctypes.c_longlong] * 3
+    lib.memory.argtypes = [ctypes.c_longlong] * 3
     lib.chunk.argtypes = [ctypes.c_longlong] * 2
     return lib
 
@@ -54,3 +56,10 @@ def test_chunk_follows_the_chain(rule):
     chunks = [rule.chunk(c, 1) for c in range(0, 5000)]
     assert chunks == sorted(chunks) and max(chunks) == 4
     assert all(2 * k <= c / 48 + 3 for c, k in enumerate(chunks))
+
+
+@pytest.mark.parametrize("m,n,k,fits", [(4096, 4096, 1024, 1), (32768, 32768, 65536, 1), (65536, 65536, 65536, 0),
+                                        (100_000_000, 256, 256, 0), (8, 8, 500_000_000, 1)])
+def test_footprint(rule, m, n, k, fits):
+    assert rule.memory(m, n, k) == fits
+    assert fits == (10 * (m + n) * -(-k // 32) * 32 + 4 * m * n <= 90e9)
