@@ -1936,10 +1936,16 @@ static void set_direct(SimtArgs<T>& a, const tccg_plan* p, const void* GA, const
   a.b_k_off = p->t_b_k;
 }
 
-// Whether the CUDA-core epilogue may move 4 m of C per thread (SimtArgs::c_vec):
-// C in the plan's layout, or TTGT's contiguous C' (tt).
+// Whether the CUDA-core epilogue moves 4 m of C per thread (SimtArgs::c_vec): C in
+// the plan's layout, or TTGT's contiguous C' (tt). FP64 moves single elements,
+// lanes along m, but for C read (beta) in 10 and more tiles per SM: 2940 x 2244 x 17
+// beta = 0 28.4 us by quads, 25.0 by elements, beta = 1 33.2 / 29.4; 112 x 8544 x
+// 1 9.8 / 8.7; 9216 x 2000 x 33 84.9 / 83.1 and 96.8 / 100.1.
 template <typename T>
-static int32_t c_vectors(const tccg_plan* p, const T* C, bool tt) {
+static int32_t c_vectors(const tccg_plan* p, const T* C, bool tt, T beta) {
+  if (sizeof(T) == 8 &&
+      (beta == T(0) || (p->Mp / p->simt_bm) * (p->Np / p->simt_bn) < 10 * (int64_t)p->num_sms))
+    return 0;
   return (tt ? p->M % 4 == 0 : p->c_quads) && reinterpret_cast<uintptr_t>(C) % (4 * sizeof(T)) == 0;
 }
 
@@ -2005,7 +2011,7 @@ static int run_simt(const tccg_plan* p, const void* GA, const void* GB, T* Cout,
   set_direct(a, p, GA, GB);
   a.status = p->d_status;
   a.crun = c_m == p->t_c_m ? p->crun : 0;  // not for TTGT's contiguous C'
-  a.c_vec = c_vectors(p, Cout, c_m != p->t_c_m);
+  a.c_vec = c_vectors(p, Cout, c_m != p->t_c_m, beta);
   a.ldc = c_ldc;
   dim3 grid((unsigned)(p->Mp / p->simt_bm), (unsigned)(p->Np / p->simt_bn), (unsigned)p->ksplit);
   if (grid.y > 65535u || grid.z > 65535u) return fail(TCCG_ERR_UNSUPPORTED, "grid too large");
@@ -2132,7 +2138,7 @@ static F32FallbackItem f32_fallback_item(const tccg_plan* p, char* ws, float* C,
   a.beta = beta;
   a.status = p->d_status;
   a.crun = p->crun;
-  a.c_vec = c_vectors(p, C, false);
+  a.c_vec = c_vectors(p, C, false, beta);
   it.split = split;
   it.tiles_m = (int32_t)(a.Mp / SimtCfg<float>::BM);
   it.tiles = (int64_t)it.tiles_m * (a.Np / SimtCfg<float>::BN);
@@ -2890,7 +2896,7 @@ static SimtArgs<T> simt_args_for(const tccg_plan* p, char* w, const void* GA, co
   set_direct(a, p, GA, GB);
   a.status = p->d_status;
   a.crun = p->crun;
-  a.c_vec = c_vectors(p, a.C, false);
+  a.c_vec = c_vectors(p, a.C, false, a.beta);
   return a;
 }
 

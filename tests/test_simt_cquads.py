@@ -44,3 +44,28 @@ def test_quads(cuda, name, beta, precision, tol):
         torch.cuda.synchronize()
         assert p.status() == 0
         assert error_metrics(dC.cpu().numpy(), ref)["normwise"] <= tol
+
+
+@pytest.mark.parametrize("beta", [0.0, 0.75])
+def test_fp64_many_tiles(cuda, beta):
+    """FP64 with 10 and more tiles per SM: quads where C is read and aligned,
+    elements on a C off the alignment; the same bits."""
+    import torch
+    m, n, k = 2052, 6000, 30
+    con = make_contraction("mn", "mk", "kn", dict(m=m, n=n, k=k), 1.25, beta)
+    p = Plan(con, "fp64", tuning=Tuning(shortk=-1))
+    assert "simt_gett" in p.describe() and "cquads=1" in p.describe()
+    g = torch.Generator(device="cuda").manual_seed(1)
+    draw = lambda s: torch.randn(s, generator=g, device="cuda", dtype=torch.float64)
+    A, B, C = draw(m * k), draw(k * n), draw(m * n)
+    outs = []
+    for offset in (0, 1):
+        buf = torch.empty(m * n + 4, dtype=torch.float64, device="cuda")
+        out = buf[offset:offset + m * n]
+        out.copy_(C)
+        p.run(A, B, out)
+        outs.append(out)
+    torch.cuda.synchronize()
+    assert p.status() == 0 and torch.equal(outs[0], outs[1])
+    ref = 1.25 * (B.view(n, k) @ A.view(k, m)) + beta * C.view(n, m)
+    assert ((outs[0].view(n, m) - ref).norm() / ref.norm()).item() <= 1e-13
