@@ -2354,8 +2354,11 @@ static bool reg_quads(const tccg_plan* p) {
 
 // The register path's jobs are few enough for its scalar form (SkrForm): one per
 // SM, or one wave of short ones (at most 4 chunks of K each: the loads' wait is
-// most of their time; 391 jobs of 3240 k are faster by pairs).
+// most of their time; 391 jobs of 3240 k are faster by pairs). With up to 8 rows
+// and a walk along positions pairs are faster there too: W = 4176, S = 1, K = 208
+// 14.9 us scalar, 12.7 by pairs; 5207, 6, 300: 16.8 / 14.9; 40134, 2, 119: 12.6 / 10.8.
 static bool reg_one_wave(const tccg_plan* p) {
+  if (p->sk.S <= 8 && p->sk.p_walk != SK_P_K) return false;
   return p->sk.njobs <= p->num_sms ||
          (p->sk.chunks_per_split <= 4 && p->sk.njobs <= (int64_t)SKR_CTAS_PER_SM * p->num_sms);
 }
