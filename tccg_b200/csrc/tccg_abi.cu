@@ -391,16 +391,16 @@ static bool choose_simt(const tccg_plan* p) {
   if (p->prec == TCCG_PREC_FP64) return true;
   if (p->tune.pair || p->tune.variant > 0 || p->tune.load > 0) return false;
   if (p->tune.variant < 0) return true;
-  // K <= 24 on a 2-D C: the short-K kernel, which streams C in and out in
+  // K <= 28 on a 2-D C: the short-K kernel, which streams C in and out in
   // blocks; a plan does not know its calls' beta. BF16, us there / on the tensor
   // cores: 9216^2 x 8 beta = 0 74 / 102, beta = 1 110 / 239; x 24 115 / 102, 135 /
-  // 241; x 32 136 / 102, 149 / 239; 6930 x 8585 (columns off 16 bytes) x 16 78 /
-  // 79, 107 / 196; x 24 105 / 81, 123 / 199; x 32 121 / 80, 140 / 197; 2304^2 x
-  // 24 16.7 / 18.7, 16.9 / 21.1. So up to 24 it costs beta = 0 at most 1.3x and
-  // gives beta = 1 1.6x and more; past that the model decides. Not in groups
+  // 241; x 28 122 / 99, 140 / 235; x 32 134 / 99, 147 / 234; 6930 x 8585 (columns off
+  // 16 bytes) x 16 78 / 79, 107 / 196; x 28 111 / 76, 130 / 192; 2304^2 x 28 14.6 /
+  // 15.4, 15.5 / 19.0. So up to 28 it costs beta = 0 at most 1.45x and gives
+  // beta = 1 1.2x to 2x; past that the model decides. Not in groups
   // (tail_split < 0), which have no short-K kernel: 8 x 2304^2 x 24 105 us by
   // their tile kernel, 76 on the tensor cores.
-  constexpr int64_t SHORT_K = 24;
+  constexpr int64_t SHORT_K = 28;
   if (p->tune.load == 0 && p->tune.tile_n == 0 && p->K <= SHORT_K && p->tune.tail_split >= 0 &&
       p->tune.shortk >= 0 && p->tune.ksplit <= 1 && p->tune.method == TCCG_METHOD_GETT &&
       p->c_ldc > 0 && p->M >= 128 && p->N >= 128 &&

@@ -1,5 +1,5 @@
 """Which kernel the BF16 precisions take for a short K on a 2-D C: the CUDA
-cores' short-K kernel up to K = 24 in plans of their own; past that, and in
+cores' short-K kernel up to K = 28 in plans of their own; past that, and in
 groups (whose CUDA-core lane has no short-K kernel), what the time model says."""
 import pytest
 
@@ -16,8 +16,8 @@ def _con(k, m=4949, n=2080):
 
 @pytest.mark.parametrize("precision", ["bf16", "bf16x3"])
 def test_choice(cuda, precision):
-    assert "simt_shortk" in Plan(_con(24), precision).describe()
-    assert "gett_tc" in Plan(_con(31), precision).describe()
+    assert "simt_shortk" in Plan(_con(28), precision).describe()
+    assert "gett_tc" in Plan(_con(29), precision).describe()
     grp = Group([_con(24), _con(32)], precision)
     for p in grp.plans:
         assert "gett_tc" in p.describe()
