@@ -8,15 +8,18 @@
 // products run on the tensor cores:
 //
 //   warps 0-7   (256 threads): copy P's chunks of 32 k from the caller's
-//               tensor into a ring of FP32 staging slots. 16-byte cp.async
-//               where four positions are consecutive and aligned; else 32
-//               loads per thread into registers, in flight while the slot
-//               frees up, then shared-memory stores: 4-byte cp.async moves at
-//               most 2.7 TB/s over 148 SMs whatever its pattern (13 cycles a
-//               warp instruction), the loads 5.1. Slots are [k][position],
-//               or [position][k] where P's stride-one index is contracted
-//               (pitch 33; 36 where rows of 4 k are aligned and move as
-//               16-byte loads): conflict-free for copies and conversion;
+//               tensor into FP32 staging slots, two groups of four warps with
+//               one slot each, taking the chunks in turn. Walks along
+//               positions by cp.async, 16 bytes where four positions are
+//               consecutive and aligned, else 4, into [k][position]. Where P's
+//               stride-one index is contracted through registers, 32 loads per
+//               thread in flight while the slot frees up, then shared-memory
+//               stores into [position][k]: 4-byte cp.async moves at most 2.7
+//               TB/s over 148 SMs whatever its pattern (13 cycles a warp
+//               instruction), the loads 5.1. Rows of 33 elements, or, where
+//               quads of k are aligned and move as 16-byte loads, of 32 with
+//               their 16-byte chunks permuted by position: conflict-free for
+//               copies and conversion;
 //   warps 8-15  (256 threads, thread = box position = TMEM lane of its
 //               half): per chunk, split the position's 32 staged values into
 //               bf16 hi / lo and write them to its TMEM lane of the chunk's A
@@ -42,9 +45,9 @@
 // issuing a chunk's copies, its Q load and its conversion in turn, a chunk
 // took 1.7-2.8 us against the 0.7 us of its HBM bytes.
 //
-// One CTA per SM (201 KB of shared memory: four 36 KB staging slots, two
-// 8 KB Q stages, the 33 KB epilogue staging and the offset tables; 25
-// warps); TMEM 512 columns (accumulators, running sums, A stages). Every
+// One CTA per SM (121 KB of shared memory: two 33 KB staging slots, two
+// 8 KB Q stages, the 33 KB epilogue staging and the offset tables, which
+// leaves the loads in flight their L1; 25 warps); TMEM 512 columns (accumulators, running sums, A stages). Every
 // wait is bounded (TCCG_DEVICE_WAIT_NS): a wait that runs out records a
 // status code and the CTA winds down.
 #pragma once
@@ -64,7 +67,7 @@ constexpr int SKT_EPI_THREADS = SK_BW;  // one position each: TMEM lane of its h
 constexpr int SKT_THREADS = SKT_COPY_THREADS + SKT_CONV_THREADS + 32 + SKT_EPI_THREADS;  // 800
 constexpr int SKT_SMAX = 64;   // rows per pass (a narrow side above 64 runs passes of 64)
 constexpr int SKT_HALF = 128;  // MMA rows: positions per half box
-constexpr int SKT_SLOTS = 2;   // FP32 staging ring
+constexpr int SKT_SLOTS = 2;   // FP32 staging slots, one per copy group
 constexpr int SKT_STAGES = 2;  // MMA operand stages (P in TMEM, Q in shared memory)
 constexpr size_t SKT_B_STAGE = (size_t)SKT_SMAX * 128;  // up to 64 Q rows x 128 B
 // staging slot layouts: [k][position], pitch SK_LDP; [position][k], pitch

@@ -461,7 +461,7 @@ static void choose_gather_k(tccg_plan* p) {
 
 // The short-K kernel moves its C block by TMA when C is a 2-D matrix
 // C[m + ldc n] with a 16-byte column stride and at least one full tile in
-// each direction (else by cp.async through the offset tables).
+// each direction.
 static bool shortk_tma(const tccg_plan* p, int64_t ldc) {
   const bool dbl = p->prec == TCCG_PREC_FP64;
   const int64_t es = dbl ? 8 : 4;
@@ -473,10 +473,12 @@ static bool shortk_tma(const tccg_plan* p, int64_t ldc) {
 
 // The short-K kernel that prefetches its C block under the FMA phase:
 // packed operands, the whole K in one panel, no k-split. Automatically where
-// C is a 2-D matrix (moved by TMA, or with lanes along m where its columns
-// are not 16-byte aligned; for other layouts it measured no faster than the
-// tile kernel) of at least two tiles per SM and one tile in each direction.
-// TTGT writes the contiguous C' (ldc = M).
+// C is a 2-D matrix of at least two tiles per SM and one tile in each direction:
+// moved by TMA, or where its columns are not 16-byte aligned by one bulk copy
+// per column (FP32) or element by element (FP64: 4097 x 4099 x 4 beta = 0 39.7 us
+// against 45.8 in the tile kernel, beta = 1 64 / 74; 6930 x 8585 x 16 132 / 164 and
+// 163 / 242; no size measured is slower). For other layouts it measured no
+// faster than the tile kernel. TTGT writes the contiguous C' (ldc = M).
 static bool choose_shortk(const tccg_plan* p, int64_t tiles) {
   if (p->direct || p->ksplit > 1 || p->tune.shortk < 0 || p->simt_shape != SIMT_SQUARE) return false;
   const int kp = p->prec == TCCG_PREC_FP64 ? SimtShortKCfg<double>::KP : SimtShortKCfg<float>::KP;
@@ -837,9 +839,9 @@ static bool choose_skinny(const tccg_plan* p) {
   const SkinnyArgs& a = p->sk;
   const int64_t W = (int64_t)a.ex * a.ey;
   if (p->K <= SK_KC && ((a.S <= 48 && W >= 65536) || W >= (int64_t(1) << 20))) return true;
-  // FP32 precision (the CUDA-core tiles its only other choice): a narrow side
-  // of at most 48 and at least 4096 positions, any K -- on the 59 such items
-  // 2.6 ms less in sum than the CUDA-core tiles (21 % of their time)
+  // FP32 precision: a narrow side of at most 48 and at least 4096 positions,
+  // any K -- on the 59 such items 2.6 ms less in sum than the CUDA-core tiles
+  // (21 % of their time). The tensor cores' six products are not weighed here.
   if (p->prec == TCCG_PREC_FP32 && a.S <= 48 && W >= 4096) return true;
   // split-BF16x3, a narrow side of at most 16 (the register path), K > 32
   // and at least 48 blocks: on the 8 such items 1.36 ms in sum where the
