@@ -60,9 +60,14 @@ extern "C" {
 #define TCCG_BF16 2
 
 /* arithmetic of the contraction */
-#define TCCG_PREC_FP32 0   /* FP32: FFMA on the CUDA cores, or (K >= 128, where a model finds it faster)
-                              six bf16 products of the exact three-way operand split on tcgen05,
-                              no less accurate; operands outside the split's range run on FFMA */
+#define TCCG_PREC_FP32 0   /* FP32: FFMA on the CUDA cores, or (chains of K >= 256, where a model
+                              finds it faster) six bf16 products of the exact three-way operand
+                              split on tcgen05. The split's error is no larger on normal,
+                              one-signed, exponential and lognormal operands (RMS relative to
+                              |A| |B|); under k slices, operands over many decades may lose up to
+                              1.3x (both near 1e-7). Infinities, NaN and operands with
+                              |a| |b| K past about 2^78 run on FFMA. The split's plans take a
+                              workspace of 6 bytes per operand element (tccg_plan_workspace) */
 #define TCCG_PREC_FP64 1   /* FP64 multiply-adds (mma.sync f64; DFMA for short K); k-split partial
                               sums and alpha/beta in FP64 */
 #define TCCG_PREC_BF16 2   /* BF16 products on tcgen05 tensor cores, FP32 accumulation in TMEM */
@@ -103,8 +108,9 @@ typedef struct tccg_tuning {
   int32_t variant;     /* BF16/BF16X3 kernel family: 0 = chosen by a bandwidth/compute model,
                           > 0 = tensor cores (BF16X3: k-blocks of 32 per TMEM accumulation
                           chunk, default 16), < 0 = CUDA cores (operands rounded to bf16 for
-                          BF16, FP32 FFMA). FP32: > 0 = the tensor-core split (k-blocks per
-                          chunk, at most 4), < 0 = CUDA cores */
+                          BF16, FP32 FFMA). FP32: > 0 = the tensor-core split whatever K
+                          (k-blocks per chunk, at most 4; operands unscaled: values
+                          below 2^-100 run on FFMA too), < 0 = CUDA cores */
   int32_t ksplit;      /* k-split factor: 0 = automatic (split K over CTAs when the C tiles
                           cannot fill the GPU), 1 = none, > 1 = that many slices
                           (the CTA-pair kernel never splits) */
@@ -117,8 +123,8 @@ typedef struct tccg_tuning {
                           operand loads stay coalesced), 1 = always, -1 = never (GETT only) */
   int32_t shortk;      /* CUDA-core kernels, K <= 32 (FP64: 16): the kernel that prefetches each
                           tile's C block under its FMA phase. 0 = automatic (C a 2-D matrix,
-                          moved by TMA or one bulk copy per column, at least two tiles per
-                          SM), 1 = always, -1 = never */
+                          moved by TMA, one bulk copy per column (FP32) or by elements
+                          (FP64), at least two tiles per SM), 1 = always, -1 = never */
   int32_t simt_tile;   /* CUDA-core tile shape, FP32 accumulation: 0 = the least padded work
                           (narrow tiles counted at 1.6x), 1 = 128x128, 2 = 128x32 (small N),
                           3 = 32x128 (small M); FP64 always 128x64 */
