@@ -742,6 +742,9 @@ __global__ void __launch_bounds__(256, 2)
 // after another's, go round the grid.
 __global__ void __launch_bounds__(256, 2)
     f32_fallback_group_kernel(const F32FallbackItem* items, int n_items) {
+  bool any = false;
+  for (int i = threadIdx.x; i < n_items; i += blockDim.x) any |= !f32_split_exact(items[i].split);
+  if (!__syncthreads_or(any)) return;
   const int64_t g = gridDim.x;
   int64_t first = 0;  // the CTA that takes the item's first job
   for (int i = 0; i < n_items; ++i) {

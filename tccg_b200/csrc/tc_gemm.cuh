@@ -1205,8 +1205,14 @@ template <int MODE, int LOAD = TC_LOAD_TMA, int BNV = 0>
 __global__ void __launch_bounds__(TcCfgT<MODE, LOAD, BNV>::NUM_THREADS, 1)
     gett_tc_group_kernel(const TcGroup g, int32_t* status) {
   gett_tc_body<MODE, LOAD, BNV, true>(nullptr, nullptr, nullptr, g, status);
-  if constexpr (MODE == TC_F32X6)
-    for (int i = 0; i < g.n_items; ++i) f32_fallback_prepare<MODE, LOAD, BNV>(g.items[i].args);
+  if constexpr (MODE == TC_F32X6) {
+    // the items' ranges read side by side: one after another they would cost
+    // every CTA two dependent loads per item
+    bool any = false;
+    for (int i = threadIdx.x; i < g.n_items; i += blockDim.x) any |= !f32_split_exact(g.items[i].args.split);
+    if (__syncthreads_or(any))
+      for (int i = 0; i < g.n_items; ++i) f32_fallback_prepare<MODE, LOAD, BNV>(g.items[i].args);
+  }
 }
 
 // FP32 results (TC_F32X6): the hi | mid parts through tmA / tmB, the lo parts
