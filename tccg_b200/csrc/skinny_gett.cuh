@@ -904,9 +904,9 @@ __device__ __forceinline__ int32_t skinny_reg_ko(const SkinnyArgs& a, int kb, in
 }
 
 // How a register-path job multiplies and loads P:
-//   SKR_SCALAR  single values (FFMA). For one wave of jobs: a CTA then has its
-//               SM nearly to itself and waits for its own loads, which the
-//               compiler sets earlier in this form (W = 22749, S = 14, K = 152:
+//   SKR_SCALAR  single values (FFMA). For jobs that wait for their own loads, as in
+//               one wave, where a CTA has its SM nearly to itself: the
+//               compiler sets the loads earlier in this form (W = 22749, S = 14, K = 152:
 //               22.6 us against 25.2 by pairs; 5060, 9, 334: 31 / 34; 151360, 4,
 //               23: 9.2 / 9.9).
 //   SKR_PAIRS   FP32 pairs (fma.rn.f32x2). With several CTAs on an SM the issue

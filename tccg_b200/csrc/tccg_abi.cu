@@ -2354,15 +2354,22 @@ static bool reg_quads(const tccg_plan* p) {
   return p->sk_reg && p->sk.p_walk == SK_P_K && p->sk_p_vec;
 }
 
-// The register path's jobs are few enough for its scalar form (SkrForm): one per
-// SM, or one wave of short ones (at most 4 chunks of K each: the loads' wait is
-// most of their time; 391 jobs of 3240 k are faster by pairs). With up to 8 rows
-// and a walk along positions pairs are faster there too: W = 4176, S = 1, K = 208
-// 14.9 us scalar, 12.7 by pairs; 5207, 6, 300: 16.8 / 14.9; 40134, 2, 119: 12.6 / 10.8.
-static bool reg_one_wave(const tccg_plan* p) {
-  if (p->sk.S <= 8 && p->sk.p_walk != SK_P_K) return false;
-  return p->sk.njobs <= p->num_sms ||
-         (p->sk.chunks_per_split <= 4 && p->sk.njobs <= (int64_t)SKR_CTAS_PER_SM * p->num_sms);
+// Whether a plan on the register path runs its scalar form (SkrForm); us, scalar /
+// pairs:
+//   a walk along k with K in one chunk, where a job is little more than its
+//   loads: W of 16128 boxes, S = 13, K = 20 419 / 520, 1112, 8, 20 24 / 28, 22464,
+//   15, 24 724 / 830;
+//   one wave of jobs, which wait for their own loads: one per SM, or short ones (at
+//   most 4 chunks of K each; long ones go either way: 504 jobs, S = 14, K = 6660
+//   449 / 520, 391, 13, 3240 474 / 442, 313, 12, 333 96 / 84).
+// Up to 8 rows on a walk along positions pairs are faster there too: W = 4176, S
+// = 1, K = 208 14.9 / 12.7; 5207, 6, 300 16.8 / 14.9; 40134, 2, 119 12.6 / 10.8.
+static bool reg_scalar(const tccg_plan* p) {
+  const SkinnyArgs& a = p->sk;
+  if (a.p_walk == SK_P_K && a.nchunks == 1) return true;
+  if (a.S <= 8 && a.p_walk != SK_P_K) return false;
+  if (a.njobs <= p->num_sms) return true;
+  return a.njobs <= (int64_t)SKR_CTAS_PER_SM * p->num_sms && a.chunks_per_split <= 4;
 }
 
 static int run_skinny(const tccg_plan* p, const void* GA, const void* GB, float* C, float alpha,
@@ -2373,13 +2380,13 @@ static int run_skinny(const tccg_plan* p, const void* GA, const void* GB, float*
   if (p->sk_reg) {
     const int64_t grid = std::min<int64_t>(a.njobs, (int64_t)SKR_CTAS_PER_SM * p->num_sms);
     // 8 computed rows for a narrow side of at most 8, else 16
-    const bool kw = reg_quads(p), one_wave = reg_one_wave(p);
+    const bool kw = reg_quads(p), scalar = reg_scalar(p);
     launch_after(false, p,
                  a.S <= 8 ? (kw         ? skinny_reg_kernel<8, SKR_QUADS>
-                             : one_wave ? skinny_reg_kernel<8, SKR_SCALAR>
+                             : scalar   ? skinny_reg_kernel<8, SKR_SCALAR>
                                         : skinny_reg_kernel<8, SKR_PAIRS>)
                           : (kw         ? skinny_reg_kernel<16, SKR_QUADS>
-                             : one_wave ? skinny_reg_kernel<16, SKR_SCALAR>
+                             : scalar   ? skinny_reg_kernel<16, SKR_SCALAR>
                                         : skinny_reg_kernel<16, SKR_PAIRS>),
                  dim3((unsigned)grid), dim3(SKR_THREADS), SKR_SMEM_BYTES, s, a);
   } else {

@@ -16,12 +16,13 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("ksplit", [1, 2])
 @pytest.mark.parametrize("m,n,k", [(300, 3, 1), (5001, 8, 23), (5001, 9, 32), (5001, 16, 33), (39000, 7, 17),
                                    (40000, 12, 33), (155000, 4, 30)])
-def test_forms_agree(cuda, m, n, k, ksplit):
+@pytest.mark.parametrize("la", ["mk", "km"])
+def test_forms_agree(cuda, la, m, n, k, ksplit):
     import torch
     from tccg_b200.grouped import Group
     sizes = dict(m=m, n=n, k=k)
-    con = make_contraction("mn", "mk", "kn", sizes, 1.25, -0.5)
-    ln = LoopNest("mn", "mk", "kn", sizes)
+    con = make_contraction("mn", la, "kn", sizes, 1.25, -0.5)
+    ln = LoopNest("mn", la, "kn", sizes)
     A, B, C = (seeded_normal(s, 71 + i).astype(np.float32)
                for i, s in enumerate((ln.size_a, ln.size_b, ln.size_c)))
     dA, dB, dC = (torch.from_numpy(x).cuda() for x in (A, B, C))
